@@ -81,11 +81,10 @@ int pfsoft_cuda_dsoft_noalloc(const double* d_grid, int B, double* d_coeffs, voi
 
 /* ---- Batches of transforms, uneven bandwidths ------------------------------------------------
  * No counterpart in the reference (which transforms one grid per call). A plan groups `count`
- * transforms by bandwidth; each execution runs batched FFT passes per bandwidth and ONE
- * persistent DWT launch over every (bandwidth, order class, transform block) item, longest
- * first, in which one on-chip Wigner recurrence serves up to `transforms_per_cta` transforms
- * (0 = default: 4 for B <= 64, 2 above). Bandwidths up to 128 share the fused FP64 launch;
- * larger ones use the per-transform FP64 DWT (or the split launch, below). The sequence is captured once into a CUDA graph and replayed
+ * transforms by bandwidth; each execution runs, per bandwidth, batched FFT passes and one DWT
+ * launch over every (order class, transform), longest classes first (or the split launch, below).
+ * `transforms_per_cta` (0, 1, 2 or 4) is checked and reported back (0: 4 for B <= 64, 2 above) and
+ * has no other effect. The sequence is captured once into a CUDA graph and replayed
  * (PFSOFT_BATCH_NO_GRAPH disables the graph). The plan owns one spectrum workspace per
  * transform (pfsoft_batch_workspace_bytes). Pointer tables are host arrays of `count` device
  * pointers in the caller's order; every buffer has the single-transform layouts above. Stream
@@ -275,8 +274,8 @@ int pfsoft_shard_unpack(pfsoft_shard_plan* plan, int direction, const double* d_
  * device milliseconds and launch count (and resets them). Returns the number of stages;
  * pfsoft_profile_stage_name(i) names stage i. */
 long long pfsoft_launch_count(void);
-/* Tuning knob used by the autotuner: direction 0 = DSOFT, 1 = IDSOFT; case_split 1 = each warp
- * applies all eight symmetry cases, 2 = warp pairs split them, 0 = library default. */
+/* Tuning knob of earlier DWT kernels: direction 0 = DSOFT, 1 = IDSOFT; case_split 0, 1 or 2. The
+ * values are checked; the present kernels have one form for all symmetry cases. */
 int pfsoft_tune_dwt_case_split(int direction, int case_split);
 /* Tuning knob: on != 0 runs the two FFT passes of a direction in one persistent launch, layer
  * chunk by layer chunk, so that the second pass reads the first pass's output from L2; 0 (the

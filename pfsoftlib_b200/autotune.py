@@ -3,8 +3,8 @@
 For a multiset of bandwidths it times candidate schedules on the device with CUDA events and
 caches the winners in a JSON table keyed by GPU name and the sorted bandwidth counts:
 
-  tune_batch  transforms per CTA of the fused FP64 DWT launch (1, 2, 4), i.e. how many
-              transforms share one on-chip Wigner recurrence;
+  tune_batch  the `transforms_per_cta` argument of a batch plan (1, 2, 4; the present DWT kernels
+              take one transform per CTA whatever it is);
   tune_plan   per bandwidth: the FFT stage as one fused launch or two passes
               (pfsoft_tune_fft_fused), and the DWT of a PFSOFT_BATCH_SPLIT plan on the
               split-precision kernel or the FP64 kernels (pfsoft_tune_split_bandwidth); the

@@ -5,9 +5,8 @@
     plan.dsoft(grid_tensors, coeff_tensors)
     plan.close()
 
-A plan groups its transforms by bandwidth, runs the FFT passes batched per bandwidth and one
-persistent DWT launch over every (bandwidth, order class, transform block) item, and replays the
-whole sequence from a CUDA graph. Create it once per bandwidth mix (it builds tables, work lists
+A plan groups its transforms by bandwidth, runs the FFT passes and one DWT launch over every (order
+class, transform) per bandwidth, and replays the whole sequence from a CUDA graph. Create it once per bandwidth mix (it builds tables, work lists
 and the graph) and reuse it with any buffers. ``split=True`` runs the DWT of bandwidths 16..128
 (multiples of 16) on the tensor cores in split precision (relative error about 1e-13 against the
 FP64 path). Calls are ordered on torch's current stream unless ``stream`` is given.

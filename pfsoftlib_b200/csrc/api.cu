@@ -326,42 +326,62 @@ size_t grid_elems(int B)
     return N * N * N;
 }
 
-// Tables for bandwidth B on the current device; built on first use.
-int get_tables(int B, cudaStream_t stream, BandTables* out)
+// Tables for bandwidth B on the current device; built on first use (the split-precision DWT's own
+// ones when `split` is first asked for).
+int get_tables(int B, cudaStream_t stream, BandTables* out, bool split = false)
 {
     int dev = 0;
     PF_CUDA(cudaGetDevice(&dev));
     DeviceState* st = device_state(dev);
     std::lock_guard<std::mutex> lk(st->mu);
     auto it = st->tables.find(B);
-    if (it != st->tables.end()) {
+    const bool have = it != st->tables.end();
+    if (have && (!split || it->second.rc_cf)) {
         *out = it->second;
         return PFSOFT_OK;
     }
-    void* mem = nullptr;
-    cudaError_t e = cudaMalloc(&mem, tables_bytes(B));
-    if (e != cudaSuccess) return fail(PFSOFT_ENOMEM, std::string("table allocation: ") + cudaGetErrorString(e));
     BandTables t;
-    {
-        StageScope sc(ST_TABLES, stream);
-        e = tables_build(B, mem, &t, stream);
+    if (have) t = it->second;
+    // one block: allocate, fill on the stream, wait
+    auto build = [&](size_t bytes, auto fill) -> int {
+        void* mem = nullptr;
+        cudaError_t e = cudaMalloc(&mem, bytes);
+        if (e != cudaSuccess) return fail(PFSOFT_ENOMEM, std::string("table allocation: ") + cudaGetErrorString(e));
+        {
+            StageScope sc(ST_TABLES, stream);
+            e = fill(mem);
+        }
+        if (e == cudaSuccess) e = cudaStreamSynchronize(stream);
+        if (e != cudaSuccess) {
+            cudaFree(mem);
+            return cuda_fail(e, "tables_build");
+        }
+        return PFSOFT_OK;
+    };
+    if (!have) {
+        int rc = build(tables_bytes(B), [&](void* mem) { return tables_build(B, mem, &t, stream); });
+        if (rc) return rc;
+        if (fft_needs_bluestein(2 * B)) {
+            // lengths with a large prime factor: the FFT's Bluestein table, computed on the host
+            std::vector<double2> h(fft_bluestein_elems(2 * B));
+            fft_bluestein_fill(2 * B, h.data());
+            void* bt = nullptr;
+            cudaError_t e = cudaMalloc(&bt, h.size() * sizeof(double2));
+            if (e == cudaSuccess) e = cudaMemcpy(bt, h.data(), h.size() * sizeof(double2), cudaMemcpyHostToDevice);
+            if (e != cudaSuccess) {
+                cudaFree(bt);
+                cudaFree(t.block);
+                return cuda_fail(e, "tables_build");
+            }
+            t.bluestein = static_cast<double2*>(bt);
+        }
+        st->tables[B] = t;
     }
-    if (e == cudaSuccess) e = cudaStreamSynchronize(stream);
-    if (e == cudaSuccess && fft_needs_bluestein(2 * B)) {
-        // lengths with a large prime factor: the FFT's Bluestein table, computed on the host
-        std::vector<double2> h(fft_bluestein_elems(2 * B));
-        fft_bluestein_fill(2 * B, h.data());
-        void* bt = nullptr;
-        e = cudaMalloc(&bt, h.size() * sizeof(double2));
-        if (e == cudaSuccess) e = cudaMemcpy(bt, h.data(), h.size() * sizeof(double2), cudaMemcpyHostToDevice);
-        if (e == cudaSuccess) t.bluestein = static_cast<double2*>(bt);
-        else if (bt) cudaFree(bt);
+    if (split) {
+        int rc = build(split_tables_bytes(B), [&](void* mem) { return split_tables_build(B, mem, &t, stream); });
+        if (rc) return rc;
+        st->tables[B] = t;
     }
-    if (e != cudaSuccess) {
-        cudaFree(mem);
-        return cuda_fail(e, "tables_build");
-    }
-    st->tables[B] = t;
     *out = t;
     return PFSOFT_OK;
 }
@@ -370,7 +390,7 @@ int get_tables(int B, cudaStream_t stream, BandTables* out)
 
 namespace pfsoft_dev {
 void set_last_error(const char* msg) { g_last_error = msg; }
-int tables_for(int B, cudaStream_t s, BandTables* out);
+int tables_for(int B, cudaStream_t s, BandTables* out, bool split);
 }  // namespace pfsoft_dev
 
 namespace {
@@ -459,7 +479,7 @@ int run_dsoft(const double* d_grid, int B, double* d_coeffs, void* ws, cudaStrea
     DwtArgs a = dwt_args(t);
     {
         StageScope sc(ST_DWT_FWD, s);
-        PF_CUDA(dwt_forward_launch(X, reinterpret_cast<double2*>(d_coeffs), a, 0, s));
+        PF_CUDA(dwt_forward_launch(X, reinterpret_cast<double2*>(d_coeffs), a, 1, s));
     }
     return PFSOFT_OK;
 }
@@ -477,7 +497,7 @@ int run_idsoft(const double* d_coeffs, int B, double* d_grid, void* ws, cudaStre
     a.zero_nyquist = 1;   // the Nyquist bins, which no order class writes, zeroed in the DWT's tail
     {
         StageScope sc(ST_DWT_INV, s);
-        PF_CUDA(dwt_inverse_launch(reinterpret_cast<const double2*>(d_coeffs), X, a, 0, s));
+        PF_CUDA(dwt_inverse_launch(reinterpret_cast<const double2*>(d_coeffs), X, a, 1, s));
     }
     // I2: inverse DFT over alpha, in place on X
     FftPassArgs i2 = pass_args(N, N, t, FftStrides{1, n2, n}, FftStrides{1, n2, n}, 1.0);
@@ -588,7 +608,7 @@ __global__ void wigner_matrix_kernel(int B, int M, int Mp, const double* w, cons
 
 namespace pfsoft_dev {
 // Cached tables of a bandwidth on the current device (used by the batch plans).
-int tables_for(int B, cudaStream_t s, BandTables* out) { return get_tables(B, s, out); }
+int tables_for(int B, cudaStream_t s, BandTables* out, bool split) { return get_tables(B, s, out, split); }
 }  // namespace pfsoft_dev
 
 extern "C" {
@@ -849,10 +869,10 @@ int pfsoft_tune_fft_fused(int B, int on)
     return PFSOFT_OK;
 }
 
+// The FP64 DWT has one form for all eight cases; the value is checked and otherwise without effect.
 int pfsoft_tune_dwt_case_split(int direction, int case_split)
 {
     if (direction < 0 || direction > 1 || case_split < 0 || case_split > 2) return fail(PFSOFT_EINVAL, "bad tuning value");
-    dwt_set_case_split(direction, case_split);
     return PFSOFT_OK;
 }
 

@@ -3,10 +3,9 @@
 // A batch plan groups its transforms by bandwidth. One forward execution is
 //   per group:  F1 (gamma DFT -> beta-innermost spectrum), F2 (alpha DFT)   [one launch each,
 //               gridDim.z = transforms of the group]
-//   all groups: one persistent DWT launch over every (group, order class, transform block)
-//               item, longest first (dwt_batch.cu)
-// and the inverse runs the mirror image. FP64 groups above B = 128 run the per-transform DWT
-// kernels; with PFSOFT_BATCH_SPLIT every group up to B = 256 shares one split-precision launch.
+//               then one DWT launch over every (order class, transform) of the group (dwt.cu)
+// and the inverse runs the mirror image. With PFSOFT_BATCH_SPLIT every group up to B = 256 shares
+// one split-precision DWT launch.
 // The whole sequence is captured once into a CUDA graph; the device tables of grid and
 // coefficient pointers that the kernels read are refreshed before each replay, so one graph
 // serves any buffers.
@@ -28,12 +27,10 @@
 using namespace pfsoft_dev;
 
 namespace pfsoft_dev {
-int tables_for(int B, cudaStream_t s, BandTables* out);   // api.cu: cached tables of a bandwidth
+int tables_for(int B, cudaStream_t s, BandTables* out, bool split = false);   // api.cu: cached tables of a bandwidth
 }
 
 namespace {
-
-constexpr int kBatchMaxFused = 128;   // largest bandwidth of the fused DWT launch (N <= 256)
 
 // Autotuner's split-precision choice per bandwidth (0 default = split where supported, 1 split,
 // -1 FP64), read when a PFSOFT_BATCH_SPLIT plan is created.
@@ -121,80 +118,41 @@ cudaError_t zero_nyquist_launch(double2** ws, int B, int T, cudaStream_t s)
     return cudaGetLastError();
 }
 
-// Per-transform DWT launches of a group (bandwidths above the fused launch); X / coeffs are host
-// arrays of the device pointers.
-cudaError_t dwt_per_transform(int dir, const BandTables& t, int T, double2* const* X, double2* const* coeffs,
-                              cudaStream_t s)
+// The FP64 DWT of a group's T transforms in one launch; ws / coefs are device pointer tables.
+// The inverse also zeroes the Nyquist bins.
+cudaError_t group_dwt_launch(int dir, const BandTables& t, int T, double2** ws, double2** coefs, cudaStream_t s)
 {
-    const DwtArgs a = dwt_args_for(t);
-    for (int i = 0; i < T; ++i) {
-        cudaError_t e = dir == 0 ? dwt_forward_launch(X[i], coeffs[i], a, 0, s) : dwt_inverse_launch(coeffs[i], X[i], a, 0, s);
-        if (e != cudaSuccess) return e;
-    }
-    return cudaSuccess;
+    DwtArgs a = dwt_args_for(t);
+    a.Xs = ws;
+    a.coefs = coefs;
+    a.zero_nyquist = dir;
+    return dir == 0 ? dwt_forward_launch(nullptr, nullptr, a, T, s) : dwt_inverse_launch(nullptr, nullptr, a, T, s);
 }
 
-// One same-bandwidth group of T transforms in direction dir (0 forward, 1 inverse) on stream s.
-// d_grids / d_coefs / d_ws are device tables of T pointers; d_group describes the group for the
-// fused DWT and d_items lists its items (group_items); *d_counter is reset here. Bandwidths
-// above the fused launch use the per-transform kernels with the host copies h_coef / h_ws.
-int launch_group(int dir, const BandTables& t, int T, double2** d_grids, double2** d_ws, const DwtGroup* d_group,
-                 const DwtItem* d_items, int n_items, int* d_counter, int tpc, double2* const* h_coef,
-                 double2* const* h_ws, cudaStream_t s)
+// Both FFT passes of a group: one fused launch when the plan allows (its counters at double2 offset
+// sync_off of each workspace), else the two passes.
+cudaError_t group_fft_launch(int dir, const BandTables& t, int T, double2** grids, double2** ws, long long sync_off,
+                             cudaStream_t s)
 {
     const int sign = dir == 0 ? -1 : +1;
-    auto pass = [&](bool first) {
-        return fft_pass_launch(nullptr, nullptr, group_pass_args(dir, first, t, d_grids, d_ws), t.N, sign, s, T);
-    };
-    // both passes of the direction: one fused launch (counters past each spectrum) or two
-    auto passes = [&]() -> cudaError_t {
-        const FftPassArgs a = group_pass_args(dir, true, t, d_grids, d_ws), b = group_pass_args(dir, false, t, d_grids, d_ws);
-        if (fft_fused_enabled(t.N) && fft_fused_chunk(a, b))
-            return fft_fused_launch(sign, a, b, t.N, t.N, T, nullptr, nullptr, nullptr, nullptr, nullptr,
-                                    (long long)t.N * t.N * t.N, s);
-        cudaError_t e = pass(true);
-        return e == cudaSuccess ? pass(false) : e;
-    };
-    auto dwt = [&]() -> cudaError_t {
-        if (t.B > kBatchMaxFused) return dwt_per_transform(dir, t, T, h_ws, h_coef, s);
-        cudaError_t e = cudaMemsetAsync(d_counter, 0, sizeof(int), s);
-        if (e != cudaSuccess) return e;
-        return dwt_batch_launch(dir, d_group, d_items, n_items, d_counter, tpc, t.N <= 64 ? 64 : (t.N <= 128 ? 128 : 256), s);
-    };
-    cudaError_t e;
-    if (dir == 0) {
-        e = passes();
-        if (e == cudaSuccess) e = dwt();
-    } else {
-        e = zero_nyquist_launch(d_ws, t.B, T, s);
-        if (e == cudaSuccess) e = dwt();
-        if (e == cudaSuccess) e = passes();
-    }
-    if (e != cudaSuccess) return fail(PFSOFT_ECUDA, std::string("group launch: ") + cudaGetErrorString(e));
-    return PFSOFT_OK;
+    const FftPassArgs a = group_pass_args(dir, true, t, grids, ws), b = group_pass_args(dir, false, t, grids, ws);
+    if (fft_fused_enabled(t.N) && fft_fused_chunk(a, b))
+        return fft_fused_launch(sign, a, b, t.N, t.N, T, nullptr, nullptr, nullptr, nullptr, nullptr, sync_off, s);
+    cudaError_t e = fft_pass_launch(nullptr, nullptr, a, t.N, sign, s, T);
+    return e == cudaSuccess ? fft_pass_launch(nullptr, nullptr, b, t.N, sign, s, T) : e;
 }
 
-// Fused-DWT work items of one group of T transforms at bandwidth B, longest first.
-void group_items(int B, int T, int tpc, std::vector<DwtItem>& out)
+// One same-bandwidth group of T transforms in direction dir (0 forward, 1 inverse) on stream s;
+// d_grids / d_coefs / d_ws are device tables of T pointers.
+int launch_group(int dir, const BandTables& t, int T, double2** d_grids, double2** d_coefs, double2** d_ws, cudaStream_t s)
 {
-    std::vector<std::pair<double, DwtItem> > v;
-    for (int c = 0; c < num_classes(B); ++c) {
-        int M, Mp;
-        class_orders(c, M, Mp);
-        for (int t0 = 0; t0 < T; t0 += tpc) {
-            DwtItem it;
-            it.group = 0;
-            it.cls = c;
-            it.t0 = t0;
-            it.nt = std::min(tpc, T - t0);
-            v.push_back(std::make_pair((double)(B - M) * it.nt + 64.0, it));
-        }
-    }
-    std::stable_sort(v.begin(), v.end(), [](const std::pair<double, DwtItem>& a, const std::pair<double, DwtItem>& b) {
-        return a.first > b.first;
-    });
-    out.clear();
-    for (auto& p : v) out.push_back(p.second);
+    const long long sync_off = (long long)t.N * t.N * t.N;
+    cudaError_t e = dir == 0 ? group_fft_launch(dir, t, T, d_grids, d_ws, sync_off, s)
+                             : group_dwt_launch(dir, t, T, d_ws, d_coefs, s);
+    if (e == cudaSuccess)
+        e = dir == 0 ? group_dwt_launch(dir, t, T, d_ws, d_coefs, s) : group_fft_launch(dir, t, T, d_grids, d_ws, sync_off, s);
+    if (e != cudaSuccess) return fail(PFSOFT_ECUDA, std::string("group launch: ") + cudaGetErrorString(e));
+    return PFSOFT_OK;
 }
 
 }  // namespace pfsoft_dev
@@ -209,17 +167,12 @@ struct pfsoft_batch {
     };
     int count = 0;
     int tpc = 1;
-    int nmax = 0;
     bool use_graph = true;
     std::vector<Group> groups;
     // device: pointer tables [3][count] (grid, coeffs, workspace) in group order
     double2** d_ptr = nullptr;
     double2** h_ptr = nullptr;   // pinned staging of the same
-    DwtGroup* d_groups_fwd = nullptr;
-    DwtGroup* d_groups_inv = nullptr;
-    DwtItem* d_items = nullptr;
-    int n_items = 0;
-    int* d_counter = nullptr;
+    DwtGroup* d_groups = nullptr;   // the split groups
     // split-precision DWT (PFSOFT_BATCH_SPLIT): segments of the groups it takes (one per group),
     // their item counts, and the sticky status of its bounded waits
     void* d_split_fwd = nullptr;
@@ -243,64 +196,33 @@ namespace {
 // Sequence of one direction on stream s (captured into a graph, or run directly).
 int enqueue(pfsoft_batch* b, int dir, cudaStream_t s)
 {
-    const int sign = dir == 0 ? -1 : +1;
-    auto fft_group = [&](const pfsoft_batch::Group& g, bool first_pass) -> cudaError_t {
-        FftPassArgs a = group_pass_args(dir, first_pass, g.tables, b->grid_ptrs() + g.ptr_base, b->ws_ptrs() + g.ptr_base);
-        return fft_pass_launch(nullptr, nullptr, a, g.N, sign, s, (int)g.members.size());
-    };
-    // both passes of a group: one fused launch when the plan allows, else the two passes
-    auto fft_both = [&](const pfsoft_batch::Group& g) -> cudaError_t {
-        const FftPassArgs a = group_pass_args(dir, true, g.tables, b->grid_ptrs() + g.ptr_base, b->ws_ptrs() + g.ptr_base);
-        const FftPassArgs c = group_pass_args(dir, false, g.tables, b->grid_ptrs() + g.ptr_base, b->ws_ptrs() + g.ptr_base);
-        if (fft_fused_enabled(g.N) && fft_fused_chunk(a, c))
-            return fft_fused_launch(sign, a, c, g.N, g.N, (int)g.members.size(), nullptr, nullptr, nullptr, nullptr, nullptr,
-                                    (long long)g.N * g.N * g.N + (g.split ? (long long)dwt_split_aux_elems(g.B) : 0), s);
-        cudaError_t e = fft_group(g, true);
-        return e == cudaSuccess ? fft_group(g, false) : e;
-    };
-    auto dwt_large = [&](const pfsoft_batch::Group& g) -> cudaError_t {
-        const size_t c = (size_t)b->count;
-        return dwt_per_transform(dir, g.tables, (int)g.members.size(), b->h_ptr + 2 * c + g.ptr_base,
-                                 b->h_ptr + c + g.ptr_base, s);
+    typedef pfsoft_batch::Group Group;
+    auto T = [](const Group& g) { return (int)g.members.size(); };
+    auto fft = [&](const Group& g) {
+        const long long sync_off = (long long)g.N * g.N * g.N + (g.split ? (long long)dwt_split_aux_elems(g.B) : 0);
+        return group_fft_launch(dir, g.tables, T(g), b->grid_ptrs() + g.ptr_base, b->ws_ptrs() + g.ptr_base, sync_off, s);
     };
     cudaError_t e = cudaSuccess;
-    if (dir == 0) {
+    if (dir == 0)
         for (const auto& g : b->groups)
-            if (e == cudaSuccess) e = fft_both(g);
-        if (e == cudaSuccess && b->n_items > 0) {
-            e = cudaMemsetAsync(b->d_counter, 0, sizeof(int), s);
-            if (e == cudaSuccess) e = dwt_batch_launch(0, b->d_groups_fwd, b->d_items, b->n_items, b->d_counter, b->tpc, b->nmax, s);
-        }
-        for (const auto& g : b->groups)
-            if (e == cudaSuccess && g.split)
-                e = dwt_split_scales(0, g.B, (int)g.members.size(), b->ws_ptrs() + g.ptr_base, b->coef_ptrs() + g.ptr_base, g.tables.w, s);
-        if (e == cudaSuccess && b->n_split_fwd > 0) {
-            e = cudaMemsetAsync(b->d_split, 0, sizeof(int), s);
-            if (e == cudaSuccess)
-                e = dwt_split_launch(0, b->d_groups_fwd, b->d_split_fwd, b->n_split_seg, b->n_split_fwd, b->d_split + 1, s);
-        }
-        for (const auto& g : b->groups)
-            if (e == cudaSuccess && g.B > kBatchMaxFused && !g.split) e = dwt_large(g);
-    } else {
-        for (const auto& g : b->groups)
-            if (e == cudaSuccess) e = zero_nyquist_launch(b->ws_ptrs() + g.ptr_base, g.B, (int)g.members.size(), s);
-        if (e == cudaSuccess && b->n_items > 0) {
-            e = cudaMemsetAsync(b->d_counter, 0, sizeof(int), s);
-            if (e == cudaSuccess) e = dwt_batch_launch(1, b->d_groups_inv, b->d_items, b->n_items, b->d_counter, b->tpc, b->nmax, s);
-        }
-        for (const auto& g : b->groups)
-            if (e == cudaSuccess && g.split)
-                e = dwt_split_scales(1, g.B, (int)g.members.size(), b->ws_ptrs() + g.ptr_base, b->coef_ptrs() + g.ptr_base, g.tables.w, s);
-        if (e == cudaSuccess && b->n_split_inv > 0) {
-            e = cudaMemsetAsync(b->d_split, 0, sizeof(int), s);
-            if (e == cudaSuccess)
-                e = dwt_split_launch(1, b->d_groups_inv, b->d_split_inv, b->n_split_seg, b->n_split_inv, b->d_split + 1, s);
-        }
-        for (const auto& g : b->groups)
-            if (e == cudaSuccess && g.B > kBatchMaxFused && !g.split) e = dwt_large(g);
-        for (const auto& g : b->groups)
-            if (e == cudaSuccess) e = fft_both(g);
+            if (e == cudaSuccess) e = fft(g);
+    for (const auto& g : b->groups) {
+        double2** ws = b->ws_ptrs() + g.ptr_base;
+        double2** coefs = b->coef_ptrs() + g.ptr_base;
+        if (e == cudaSuccess && !g.split) e = group_dwt_launch(dir, g.tables, T(g), ws, coefs, s);
+        if (e == cudaSuccess && g.split && dir == 1) e = zero_nyquist_launch(ws, g.B, T(g), s);
+        if (e == cudaSuccess && g.split) e = dwt_split_scales(dir, g.B, T(g), ws, coefs, g.tables.w, s);
     }
+    const int n_split = dir == 0 ? b->n_split_fwd : b->n_split_inv;
+    if (e == cudaSuccess && n_split > 0) {
+        e = cudaMemsetAsync(b->d_split, 0, sizeof(int), s);
+        if (e == cudaSuccess)
+            e = dwt_split_launch(dir, b->d_groups, dir == 0 ? b->d_split_fwd : b->d_split_inv, b->n_split_seg, n_split,
+                                 b->d_split + 1, s);
+    }
+    if (dir == 1)
+        for (const auto& g : b->groups)
+            if (e == cudaSuccess) e = fft(g);
     if (e != cudaSuccess) return fail(PFSOFT_ECUDA, std::string("batch launch: ") + cudaGetErrorString(e));
     return PFSOFT_OK;
 }
@@ -312,10 +234,7 @@ void free_batch(pfsoft_batch* b)
     if (b->uploaded) cudaEventDestroy(b->uploaded);
     cudaFree(b->d_ptr);
     cudaFreeHost(b->h_ptr);
-    cudaFree(b->d_groups_fwd);
-    cudaFree(b->d_groups_inv);
-    cudaFree(b->d_items);
-    cudaFree(b->d_counter);
+    cudaFree(b->d_groups);
     cudaFree(b->d_split_fwd);
     cudaFree(b->d_split_inv);
     cudaFree(b->d_split);
@@ -357,61 +276,27 @@ int pfsoft_batch_create(const int* bandwidths, int count, int transforms_per_cta
             ws_total += ((((size_t)g.N * g.N * g.N + (g.split ? dwt_split_aux_elems(g.B) : 0)) * sizeof(double2) + kFftSyncBytes
                           + 255) & ~(size_t)255);   // each workspace 256-byte aligned
         }
-        int rc = tables_for(g.B, nullptr, &g.tables);
+        int rc = tables_for(g.B, nullptr, &g.tables, g.split);
         if (rc) {
             free_batch(b);
             return rc;
         }
-        if (g.B <= kBatchMaxFused && !g.split) b->nmax = std::max(b->nmax, g.N);
         b->groups.push_back(g);
     }
-    b->tpc = transforms_per_cta ? transforms_per_cta : dwt_batch_transforms_per_cta(std::max(b->nmax, 2));
-    // work items, longest first: (B - M) degrees x N columns of beta x transforms
-    std::vector<DwtItem> items;
-    std::vector<double> cost;
-    std::vector<DwtGroup> dg_f, dg_i;
-    int gi_fused = 0;
-    std::vector<int> fused_index(b->groups.size(), -1);
+    // reported as asked for (0: 4 up to B = 64, 2 above); the DWT kernels take one transform per CTA
+    b->tpc = transforms_per_cta ? transforms_per_cta : (std::min(by_b.rbegin()->first, 128) <= 64 ? 4 : 2);
     std::vector<int> split_group, split_B, split_T;   // the split groups: index in d_groups, B, T
-    for (size_t gi = 0; gi < b->groups.size(); ++gi) {
-        const auto& g = b->groups[gi];
-        if (g.B > kBatchMaxFused && !g.split) continue;
-        fused_index[gi] = gi_fused++;
-        const int T = (int)g.members.size();
-        if (g.split) {
-            split_group.push_back(fused_index[gi]);
-            split_B.push_back(g.B);
-            split_T.push_back(T);
-            continue;
-        }
-        for (int c = 0; c < num_classes(g.B); ++c) {
-            int M, Mp;
-            class_orders(c, M, Mp);
-            for (int t0 = 0; t0 < T; t0 += b->tpc) {
-                DwtItem it;
-                it.group = fused_index[gi];
-                it.cls = c;
-                it.t0 = t0;
-                it.nt = std::min(b->tpc, T - t0);
-                items.push_back(it);
-                cost.push_back((double)(g.B - M) * g.N * it.nt + 64.0 * g.N);
-            }
-        }
+    for (const auto& g : b->groups) {
+        if (!g.split) continue;
+        split_group.push_back((int)split_group.size());
+        split_B.push_back(g.B);
+        split_T.push_back((int)g.members.size());
     }
     std::vector<unsigned char> split_f, split_i;   // forward / inverse segments
     const int n_split_f = dwt_split_segments(0, split_group, split_B, split_T, split_f);
     const int n_split_i = dwt_split_segments(1, split_group, split_B, split_T, split_i);
-    std::vector<int> order(items.size());
-    for (size_t i = 0; i < order.size(); ++i) order[i] = (int)i;
-    std::stable_sort(order.begin(), order.end(), [&](int x, int y) { return cost[x] > cost[y]; });
-    std::vector<DwtItem> sorted(items.size());
-    for (size_t i = 0; i < order.size(); ++i) sorted[i] = items[order[i]];
-    b->n_items = (int)sorted.size();
-
     cudaError_t e = cudaMalloc(&b->d_ptr, 3 * (size_t)count * sizeof(double2*));
     if (e == cudaSuccess) e = cudaHostAlloc(&b->h_ptr, 3 * (size_t)count * sizeof(double2*), cudaHostAllocDefault);
-    if (e == cudaSuccess) e = cudaMalloc(&b->d_counter, sizeof(int));
-    if (e == cudaSuccess && !sorted.empty()) e = cudaMalloc(&b->d_items, sorted.size() * sizeof(DwtItem));
     if (e == cudaSuccess) e = cudaMalloc(&b->ws, ws_total);
     if (e == cudaSuccess) e = cudaEventCreateWithFlags(&b->uploaded, cudaEventDisableTiming);
     if (e == cudaSuccess) e = cudaMalloc(&b->d_split, 2 * sizeof(int));
@@ -448,10 +333,10 @@ int pfsoft_batch_create(const int* bandwidths, int count, int transforms_per_cta
         free_batch(b);
         return fail(PFSOFT_ECUDA, std::string("batch setup: ") + cudaGetErrorString(e));
     }
-    // group descriptors for the fused DWT (pointer tables inside the device array)
-    for (size_t gi = 0; gi < b->groups.size(); ++gi) {
-        const auto& g = b->groups[gi];
-        if (fused_index[gi] < 0) continue;
+    // group descriptors of the split-precision DWT (pointer tables inside the device array)
+    std::vector<DwtGroup> dg;
+    for (const auto& g : b->groups) {
+        if (!g.split) continue;
         DwtGroup d;
         d.B = g.B;
         d.N = g.N;
@@ -465,16 +350,11 @@ int pfsoft_batch_create(const int* bandwidths, int count, int transforms_per_cta
         d.rc_f1 = g.tables.rc_f1;
         d.X = b->ws_ptrs() + g.ptr_base;
         d.coeffs = b->coef_ptrs() + g.ptr_base;
-        dg_f.push_back(d);
-        dg_i.push_back(d);
+        dg.push_back(d);
     }
-    if (!dg_f.empty()) {
-        e = cudaMalloc(&b->d_groups_fwd, dg_f.size() * sizeof(DwtGroup));
-        if (e == cudaSuccess) e = cudaMalloc(&b->d_groups_inv, dg_i.size() * sizeof(DwtGroup));
-        if (e == cudaSuccess) e = cudaMemcpy(b->d_groups_fwd, dg_f.data(), dg_f.size() * sizeof(DwtGroup), cudaMemcpyHostToDevice);
-        if (e == cudaSuccess) e = cudaMemcpy(b->d_groups_inv, dg_i.data(), dg_i.size() * sizeof(DwtGroup), cudaMemcpyHostToDevice);
-        if (e == cudaSuccess && !sorted.empty())
-            e = cudaMemcpy(b->d_items, sorted.data(), sorted.size() * sizeof(DwtItem), cudaMemcpyHostToDevice);
+    if (!dg.empty()) {
+        e = cudaMalloc(&b->d_groups, dg.size() * sizeof(DwtGroup));
+        if (e == cudaSuccess) e = cudaMemcpy(b->d_groups, dg.data(), dg.size() * sizeof(DwtGroup), cudaMemcpyHostToDevice);
     }
     if (e == cudaSuccess) e = cudaMemcpy(b->d_ptr, b->h_ptr, 3 * (size_t)count * sizeof(double2*), cudaMemcpyHostToDevice);
     if (e != cudaSuccess) {
@@ -561,14 +441,7 @@ static int batch_run(pfsoft_batch* b, int dir, const double* const* in, double* 
     e = cudaMemcpyAsync(b->d_ptr, b->h_ptr, 2 * (size_t)b->count * sizeof(double2*), cudaMemcpyHostToDevice, s);
     if (e == cudaSuccess) e = cudaEventRecord(b->uploaded, s);
     if (e != cudaSuccess) return fail(PFSOFT_ECUDA, std::string("pointer upload: ") + cudaGetErrorString(e));
-    bool large = false;
-    for (const auto& g : b->groups) large |= g.B > kBatchMaxFused && !g.split;
-    // groups above the fused limit take their per-transform pointers at enqueue time, so they
-    // are launched directly; everything else replays one captured graph
-    if (!b->use_graph || large) {
-        // the host-side pointer table must stay valid until the launches are enqueued
-        return enqueue(b, dir, s);
-    }
+    if (!b->use_graph) return enqueue(b, dir, s);
     if (!b->graph[dir]) {
         cudaStream_t cs;
         e = cudaStreamCreateWithFlags(&cs, cudaStreamNonBlocking);

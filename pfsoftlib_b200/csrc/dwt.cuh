@@ -1,4 +1,4 @@
-// Discrete Wigner transform over beta (the DWT stage of DSOFT / iDSOFT), FP64 on CUDA cores.
+// Discrete Wigner transform over beta (the DWT stage of DSOFT / iDSOFT) and its tables.
 #pragma once
 
 #include <cuda_runtime.h>
@@ -15,16 +15,24 @@ struct BandTables {
     double* sinh = nullptr;     // sin(beta_k / 2)                [N]
     double* cosh = nullptr;     // cos(beta_k / 2)                [N]
     double* w = nullptr;        // quadrature weights w_B(k)      [N]   (fn_dwt.hpp:62-83)
-    double* normf = nullptr;    // seed norm per order class      [B(B+1)/2] (fn_dwt.hpp:117-121)
     double2* twiddle = nullptr; // exp(-2 pi i t / N)             [N]
+    double2* ht = nullptr;      // {cos, sin}(pi n / (2N))        [B]
+    // the Wigner rows at beta = pi/2, ((2l+1)/2)^(1/4) P[l][n][M] (-1)^(n-M) for n > M, tiles of 8 degrees x 8 n per
+    // order M (delta_offset); zero for l < M, n > l and l >= B          [delta_entries(B)]
+    double* delta = nullptr;
+    // (2 - [n = 0]) cos(n beta_k) and sin, n = 2 m + q < B, k < B, tiles of 8 m x 8 k in the order
+    // [cos, sin][q][m / 8][k / 8], row-major, zero past either end            [trig_entries(B)]
+    double* trig = nullptr;
+    void* block = nullptr;      // single allocation holding all of the above
+    double2* bluestein = nullptr;   // N with a prime factor above 16: the FFT's Bluestein table (own allocation)
+    // only for the split-precision DWT (split_tables_build; null until a caller asks for them)
+    double* normf = nullptr;    // seed norm per order class      [B(B+1)/2] (fn_dwt.hpp:117-121)
     double2* pw_sin = nullptr;  // sin(beta_k/2)^p as {mantissa, exponent}  [2B][N], p < 2B
     double2* pw_cos = nullptr;  // cos(beta_k/2)^p as {mantissa, exponent}  [2B][N]
     // recurrence coefficients of the step l -> l+1 for every order class and degree M <= l < B,
     // class (M, M') from rc_offset(B, M, M'): {c1, f1 f2} and f1      [rc_entries(B)]
     double2* rc_cf = nullptr;
     double* rc_f1 = nullptr;
-    void* block = nullptr;      // single allocation holding all of the above
-    double2* bluestein = nullptr;   // N with a prime factor above 16: the FFT's Bluestein table (own allocation)
 };
 
 // Entries of the recurrence-coefficient table before class (M, M'): classes run M = 0, 1, ...
@@ -36,26 +44,43 @@ __host__ __device__ __forceinline__ long long rc_offset(int B, int M, int Mp)
 }
 __host__ __device__ __forceinline__ long long rc_entries(int B) { return rc_offset(B, B, 0); }
 
+// Doubles before order M's tiles in BandTables::delta: order m has tri(nb) - tri(m/8) tiles of 64 (nb = ceil(B/8)
+// blocks of degrees, block lb with lb + 1 tiles).
+__host__ __device__ __forceinline__ long long delta_offset(int B, int M)
+{
+    const long long nb = (B + 7) / 8, T = nb * (nb + 1), b = M >> 3, r = M & 7;
+    return 256 * (b * T - (b - 1) * b * (b + 1) / 3) + r * 32 * (T - b * (b + 1));
+}
+__host__ __device__ __forceinline__ long long delta_entries(int B) { return delta_offset(B, B); }
+
+__host__ __device__ __forceinline__ long long trig_entries(int B)
+{
+    const long long nb = (B + 7) / 8;
+    return 4 * ((nb + 1) / 2) * nb * 64;
+}
+
 size_t tables_bytes(int B);
 // Carve the tables out of `mem` (tables_bytes(B) bytes, 256-byte aligned) and fill them.
 cudaError_t tables_build(int B, void* mem, BandTables* t, cudaStream_t stream);
+// The split-precision DWT's own tables, after tables_build, from another block.
+size_t split_tables_bytes(int B);
+cudaError_t split_tables_build(int B, void* mem, BandTables* t, cudaStream_t stream);
 
 struct DwtArgs {
     int B, N;
-    const double* cosb;
-    const double* sinh;
-    const double* cosh;
     const double* w;
-    const double* normf;
-    const double2* pw_sin;
-    const double2* pw_cos;
-    int team_warps;   // warps cooperating on one order class (1..4)
-    const double2* rc_cf;   // recurrence coefficients (BandTables::rc_cf / rc_f1)
-    const double* rc_f1;
+    const double2* ht;
+    const double2* tw;
+    const double* delta;
+    const double* trig;
     // Optional subset of order classes (ascending, so longest first): when set, the kernels run
     // classes[0 .. n_classes-1] only and leave every other class's outputs untouched.
     const int* classes;
     int n_classes;
+    // Several transforms of one bandwidth: device tables of their spectra and coefficients
+    double2* const* Xs;
+    double2* const* coefs;
+    int T, items;   // set by the launch
     // Inverse only: also zero the Nyquist bins (row B or column B of X, which no order class
     // writes) in the kernel's tail, instead of a separate launch.
     int zero_nyquist;
@@ -64,24 +89,18 @@ struct DwtArgs {
 // Arguments of the DWT launches over every order class of a bandwidth's tables.
 DwtArgs dwt_args_for(const BandTables& t);
 
-// nblocks <= 0 launches the persistent grid (all resident CTAs).
+// T transforms (T > 1: a.Xs and a.coefs; X and coeffs are then unused).
 // Forward: X (beta-innermost spectrum, N^3) -> packed coefficients, scale pi/(2B^2).
-cudaError_t dwt_forward_launch(const double2* X, double2* coeffs, const DwtArgs& a, int nblocks,
-                               cudaStream_t stream);
+cudaError_t dwt_forward_launch(const double2* X, double2* coeffs, const DwtArgs& a, int T, cudaStream_t stream);
 // Inverse: packed coefficients -> X (all non-Nyquist beta columns), scale 2B^2/pi.
-cudaError_t dwt_inverse_launch(const double2* coeffs, double2* X, const DwtArgs& a, int nblocks,
-                               cudaStream_t stream);
+cudaError_t dwt_inverse_launch(const double2* coeffs, double2* X, const DwtArgs& a, int T, cudaStream_t stream);
 // Zero the beta columns of the Nyquist bins (row == B or col == B) of X.
 cudaError_t zero_nyquist_launch(double2* X, int B, cudaStream_t stream);
 
-// Tuning: dir 0 = forward, 1 = inverse; cs 1 = all eight cases per warp, 2 = four cases per
-// warp (warp pairs share the recurrence), 0 = default.
-void dwt_set_case_split(int dir, int cs);
-
-// ---- batched DWT over many transforms and bandwidths (dwt_batch.cu) -------------------------
+// ---- split-precision DWT over many transforms and bandwidths (dwt_split.cu) ------------------
 // A group holds T transforms of one bandwidth; X[t] is transform t's beta-innermost spectrum
 // (N^3) and coeffs[t] its packed coefficients. Forward reads X and writes coeffs, inverse the
-// other way. A work item is one order class of a group for transforms t0 .. t0+nt-1.
+// other way.
 struct DwtGroup {
     int B, N, T;
     const double* cosb;
@@ -94,18 +113,6 @@ struct DwtGroup {
     double2* const* X;
     double2* const* coeffs;
 };
-
-struct DwtItem {
-    int group, cls, t0, nt;
-};
-
-// Transforms per CTA (1, 2 or 4) and the largest beta-column count the launch supports.
-int dwt_batch_transforms_per_cta(int nmax);
-size_t dwt_batch_smem_bytes(int direction, int tpc, int nmax);
-// One persistent launch over all items; *d_counter must be 0 (the kernel hands out items from
-// it). direction 0 = forward, 1 = inverse. nmax >= every group's N, nmax <= 256.
-cudaError_t dwt_batch_launch(int direction, const DwtGroup* d_groups, const DwtItem* d_items, int n_items,
-                             int* d_counter, int tpc, int nmax, cudaStream_t stream);
 
 // Split-precision DWT on the tensor cores (dwt_split.cu) for groups whose bandwidth passes
 // dwt_split_supported. A launch covers several groups of d_groups, described by segments
@@ -131,8 +138,5 @@ void dwt_split_set_fail_ns(unsigned long long ns);
 
 // Sets the detail string returned by pfsoft_last_error() on the calling thread.
 void set_last_error(const char* msg);
-
-// Team shape for a bandwidth: warps per class so that each lane owns at most 4 beta columns.
-int dwt_team_warps(int N);
 
 }  // namespace pfsoft_dev

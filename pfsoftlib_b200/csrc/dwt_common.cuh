@@ -1,6 +1,5 @@
-// Device helpers shared by the discrete Wigner transform kernels (dwt.cu, dwt_batch.cu):
-// recurrence coefficients, table seeds, the per-column recurrence state, the FP64 MMA, class
-// scheduling order and team barriers.
+// Device helpers of the discrete Wigner transform kernels (dwt.cu, dwt_split.cu): recurrence
+// coefficients, table seeds, the FP64 MMA and the class lists.
 #pragma once
 
 #include "common.cuh"
@@ -9,8 +8,6 @@
 namespace pfsoft_dev {
 namespace dwtk {
 
-constexpr int kWarps = 4;     // warps per CTA
-constexpr int kLB = 32;       // degrees per reduction / coefficient chunk
 constexpr double kPi = 3.141592653589793;
 
 // Recurrence step degree l -> l+1 for orders (M, Mp) (fn_dwt.hpp:167-192):
@@ -49,16 +46,6 @@ __device__ __forceinline__ double seed_value(double nf_w, double2 s, double2 c, 
     return -ldexp(v, E + 600 * sc);
 }
 
-template <int TW>
-__device__ __forceinline__ void team_sync(int team)
-{
-    if (TW == 1) {
-        __syncwarp();
-    } else {
-        asm volatile("bar.sync %0, %1;" ::"r"(1 + team), "r"(32 * TW) : "memory");
-    }
-}
-
 __device__ __forceinline__ double case_sign(const PairCase& p, int l, int M)
 {
     return (p.rev && ((l - M) & 1)) ? -p.s0 : p.s0;
@@ -73,109 +60,8 @@ __device__ __forceinline__ void dmma(double& c0, double& c1, double a, double b)
         : "d"(a), "d"(b));
 }
 
-// Hint: bring [p, p + bytes) into L2 (bytes a multiple of 16, p 16-byte aligned).
-__device__ __forceinline__ void prefetch_l2(const void* p, unsigned bytes)
-{
-    asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;" ::"l"(p), "r"(bytes) : "memory");
-}
-
-// Snake (boustrophedon) order over the longest-first class list: team `my` of `T` takes
-// classes r*T + my in even rounds and r*T + T-1-my in odd rounds.
-__device__ __forceinline__ int snake_class(int r, int T, int my) { return r * T + ((r & 1) ? (T - 1 - my) : my); }
-
-// Length of the launch's class list and its i-th class (all classes in order when no subset is
-// given; a subset keeps the longest-first order the snake relies on).
-__device__ __forceinline__ int list_length(const DwtArgs& a) { return a.classes ? a.n_classes : num_classes(a.B); }
+// The i-th class of the launch (all classes in order when no subset is given).
 __device__ __forceinline__ int list_class(const DwtArgs& a, int i) { return a.classes ? __ldg(a.classes + i) : i; }
-
-template <int KT>
-struct ColumnState {
-    double cb[KT], dcur[KT], dprev[KT], keep[KT];
-    int sc[KT];
-    bool scaled;
-
-    __device__ __forceinline__ void seed(const DwtArgs& a, const int* kc, double nf, bool weighted, int M, int Mp)
-    {
-        bool any = false;
-#pragma unroll
-        for (int j = 0; j < KT; ++j) {
-            const int k = kc[j];
-            dprev[j] = 0.0;
-            sc[j] = 0;
-            dcur[j] = k < a.N ? seed_value(weighted ? nf * a.w[k] : nf, a.pw_sin[(size_t)(M - Mp) * a.N + k],
-                                           a.pw_cos[(size_t)(M + Mp) * a.N + k], sc[j])
-                              : 0.0;
-            keep[j] = sc[j] ? 0.0 : 1.0;
-            any |= sc[j] > 0;
-        }
-        scaled = __any_sync(0xffffffffu, any);
-    }
-
-    // d(l) of the lane's columns into row[lane + 32j]; a column still below 2^-300 stores 0
-    __device__ __forceinline__ void store(double* row, int lane) const
-    {
-        if (!scaled) {
-#pragma unroll
-            for (int j = 0; j < KT; ++j) row[lane + 32 * j] = dcur[j];
-        } else {
-#pragma unroll
-            for (int j = 0; j < KT; ++j) row[lane + 32 * j] = dcur[j] * keep[j];
-        }
-    }
-
-    // d(l+1) = c1 d(l-1) + d(l) (a + b cos beta), with a = f1 f2 and b = f1
-    __device__ __forceinline__ void advance(double c1, double a, double b)
-    {
-#pragma unroll
-        for (int j = 0; j < KT; ++j) {
-            const double t = fma(b, cb[j], a);
-            const double nx = fma(c1, dprev[j], dcur[j] * t);
-            dprev[j] = dcur[j];
-            dcur[j] = nx;
-        }
-        if (scaled) {
-            bool still = false;
-#pragma unroll
-            for (int j = 0; j < KT; ++j) {
-                if (sc[j] && fabs(dcur[j]) >= 0x1p300) {
-                    dcur[j] *= 0x1p-600;
-                    dprev[j] *= 0x1p-600;
-                    if (--sc[j] == 0) keep[j] = 1.0;
-                }
-                still |= sc[j] > 0;
-            }
-            scaled = __any_sync(0xffffffffu, still);
-        }
-    }
-};
-
-// Recurrence coefficients for degrees l .. l+31 of one warp: rc[i] = {c1, f1 f2, f1, -} for the
-// step l+i -> l+i+1 (one lane per degree), read from the bandwidth's table. Steps past the last
-// degree get zeros (the rows they feed are zero and never used), so the step loop has no guards.
-__device__ __forceinline__ void fill_rc4(const DwtArgs& a, double* rc, int l, int M, int Mp, int lane)
-{
-    __syncwarp();
-    const int d = l + lane;
-    double2 cf = make_double2(0.0, 0.0);
-    double f1 = 0.0;
-    if (d < a.B) {
-        const long long i = rc_offset(a.B, M, Mp) + (d - M);
-        cf = __ldg(a.rc_cf + i);
-        f1 = __ldg(a.rc_f1 + i);
-    }
-    *reinterpret_cast<double2*>(rc + 4 * lane) = cf;
-    rc[4 * lane + 2] = f1;
-    __syncwarp();
-}
-
-// One recurrence step: store d(l) into `row`, advance to d(l+1).
-template <int KT>
-__device__ __forceinline__ void gen_step(ColumnState<KT>& cs, double* row, int lane, const double* rc)
-{
-    cs.store(row, lane);
-    const double2 ca = *reinterpret_cast<const double2*>(rc);
-    cs.advance(ca.x, ca.y, rc[2]);
-}
 
 }  // namespace dwtk
 }  // namespace pfsoft_dev

@@ -22,124 +22,13 @@
 
 #include "common.cuh"
 #include "fft.cuh"
+#include "fft_core.cuh"
 
 namespace pfsoft_dev {
 
 namespace {
 
-constexpr double kSqrtHalf = 0.70710678118654752440084436210485;
-constexpr double kCosPi8 = 0.92387953251128675612818318939679;   // cos(pi/8)
-constexpr double kSinPi8 = 0.38268343236508977172845998403040;   // sin(pi/8)
-constexpr double kSin60 = 0.86602540378443864676372317075294;    // sin(pi/3)
-constexpr double kC5_1 = 0.30901699437494742410229341718282;     // cos(2pi/5)
-constexpr double kC5_2 = -0.80901699437494742410229341718282;    // cos(4pi/5)
-constexpr double kS5_1 = 0.95105651629515357211643933337938;     // sin(2pi/5)
-constexpr double kS5_2 = 0.58778525229247312916870595463907;     // sin(4pi/5)
-
-template <int SIGN>
-__device__ __forceinline__ void dft2(double2* v)
-{
-    double2 a = v[0], b = v[1];
-    v[0] = cadd(a, b);
-    v[1] = csub(a, b);
-}
-
-template <int SIGN>
-__device__ __forceinline__ void dft4(double2& v0, double2& v1, double2& v2, double2& v3)
-{
-    double2 a0 = cadd(v0, v2), a1 = csub(v0, v2);
-    double2 b0 = cadd(v1, v3), b1 = cmul_i<SIGN>(csub(v1, v3));
-    v0 = cadd(a0, b0);
-    v2 = csub(a0, b0);
-    v1 = cadd(a1, b1);
-    v3 = csub(a1, b1);
-}
-
-// w8^q = exp(SIGN*2*pi*i*q/8)
-template <int SIGN, int Q>
-__device__ __forceinline__ double2 rot8(double2 a)
-{
-    if (Q == 0) return a;
-    if (Q == 2) return cmul_i<SIGN>(a);
-    if (Q == 1) return make_double2(kSqrtHalf * (a.x - SIGN * a.y), kSqrtHalf * (a.y + SIGN * a.x));
-    // Q == 3: (-1 + SIGN i)/sqrt2
-    return make_double2(kSqrtHalf * (-a.x - SIGN * a.y), kSqrtHalf * (-a.y + SIGN * a.x));
-}
-
-template <int SIGN>
-__device__ __forceinline__ void dft8(double2* v)
-{
-    // even/odd split: E = DFT4(v0 v2 v4 v6), O = DFT4(v1 v3 v5 v7)
-    dft4<SIGN>(v[0], v[2], v[4], v[6]);
-    dft4<SIGN>(v[1], v[3], v[5], v[7]);
-    double2 o1 = rot8<SIGN, 1>(v[3]), o2 = rot8<SIGN, 2>(v[5]), o3 = rot8<SIGN, 3>(v[7]);
-    double2 e0 = v[0], e1 = v[2], e2 = v[4], e3 = v[6], o0 = v[1];
-    v[0] = cadd(e0, o0);
-    v[4] = csub(e0, o0);
-    v[1] = cadd(e1, o1);
-    v[5] = csub(e1, o1);
-    v[2] = cadd(e2, o2);
-    v[6] = csub(e2, o2);
-    v[3] = cadd(e3, o3);
-    v[7] = csub(e3, o3);
-}
-
-template <int SIGN>
-__device__ __forceinline__ void dft16(double2* v)
-{
-    double2 e[8], o[8];
-#pragma unroll
-    for (int i = 0; i < 8; ++i) {
-        e[i] = v[2 * i];
-        o[i] = v[2 * i + 1];
-    }
-    dft8<SIGN>(e);
-    dft8<SIGN>(o);
-    // w16^q = (cos(pi q/8), SIGN sin(pi q/8))
-    const double cq[8] = {1.0, kCosPi8, kSqrtHalf, kSinPi8, 0.0, -kSinPi8, -kSqrtHalf, -kCosPi8};
-    const double sq[8] = {0.0, kSinPi8, kSqrtHalf, kCosPi8, 1.0, kCosPi8, kSqrtHalf, kSinPi8};
-#pragma unroll
-    for (int q = 0; q < 8; ++q) {
-        double2 t = (q == 0) ? o[0] : make_double2(cq[q] * o[q].x - SIGN * sq[q] * o[q].y,
-                                                    cq[q] * o[q].y + SIGN * sq[q] * o[q].x);
-        v[q] = cadd(e[q], t);
-        v[q + 8] = csub(e[q], t);
-    }
-}
-
-template <int SIGN>
-__device__ __forceinline__ void dft3(double2* v)
-{
-    double2 t1 = cadd(v[1], v[2]);
-    double2 t2 = csub(v[1], v[2]);
-    double2 a = make_double2(v[0].x - 0.5 * t1.x, v[0].y - 0.5 * t1.y);
-    double2 b = cmul_i<SIGN>(cscale(t2, kSin60));
-    v[0] = cadd(v[0], t1);
-    v[1] = cadd(a, b);
-    v[2] = csub(a, b);
-}
-
-template <int SIGN>
-__device__ __forceinline__ void dft5(double2* v)
-{
-    double2 t1 = cadd(v[1], v[4]), t2 = cadd(v[2], v[3]);
-    double2 t3 = csub(v[1], v[4]), t4 = csub(v[2], v[3]);
-    double2 a1 = make_double2(v[0].x + kC5_1 * t1.x + kC5_2 * t2.x, v[0].y + kC5_1 * t1.y + kC5_2 * t2.y);
-    double2 a2 = make_double2(v[0].x + kC5_2 * t1.x + kC5_1 * t2.x, v[0].y + kC5_2 * t1.y + kC5_1 * t2.y);
-    double2 b1 = cmul_i<SIGN>(make_double2(kS5_1 * t3.x + kS5_2 * t4.x, kS5_1 * t3.y + kS5_2 * t4.y));
-    double2 b2 = cmul_i<SIGN>(make_double2(kS5_2 * t3.x - kS5_1 * t4.x, kS5_2 * t3.y - kS5_1 * t4.y));
-    v[0] = cadd(v[0], cadd(t1, t2));
-    v[1] = cadd(a1, b1);
-    v[4] = csub(a1, b1);
-    v[2] = cadd(a2, b2);
-    v[3] = csub(a2, b2);
-}
-
-__device__ __forceinline__ double2 twiddle(const double2* __restrict__ tw, int t, int sign)
-{
-    double2 w = __ldg(tw + t);
-    return sign < 0 ? w : make_double2(w.x, -w.y);
-}
+using namespace fftk;
 
 // First-stage load of a pass: the read-only path, unless the pass reads what another CTA of the
 // same launch wrote (the second pass of fft_fused_kernel), which needs coherent loads.
@@ -158,11 +47,6 @@ __device__ __forceinline__ void store_out(const FftPassArgs& a, double2* p, doub
     else
         *p = v;
 }
-
-// smem position of element i of a vector (one pad slot every 16 elements)
-__device__ __forceinline__ int spos(int i) { return i + (i >> 4); }
-
-__host__ __device__ __forceinline__ int padded_len(int n) { return n + (n >> 4) + 1; }
 
 template <int SIGN, int R>
 __device__ __forceinline__ void run_stage_fixed(const FftPassArgs& a, int s, const double2* gsrc,
@@ -203,13 +87,7 @@ __device__ __forceinline__ void run_stage_fixed(const FftPassArgs& a, int s, con
 #pragma unroll
             for (int r = 1; r < R; ++r) v[r] = cmul(v[r], twiddle(a.twiddle, r * k * step, SIGN));
         }
-        if (R == 1) {
-        } else if (R == 2) dft2<SIGN>(v);
-        else if (R == 4) dft4<SIGN>(v[0], v[1], v[2], v[3]);
-        else if (R == 8) dft8<SIGN>(v);
-        else if (R == 16) dft16<SIGN>(v);
-        else if (R == 3) dft3<SIGN>(v);
-        else if (R == 5) dft5<SIGN>(v);
+        butterfly<SIGN, R>(v);
         const int ob = (j / Ns) * Ns * R + k;
         if (last) {
             double2* p = gdst + dst_base + (long long)kk * a.dst.sv;
@@ -274,11 +152,7 @@ __device__ __forceinline__ void run_stage_inplace(const FftPassArgs& a, int s, c
 #pragma unroll
             for (int r = 1; r < R; ++r) v[p][r] = cmul(v[p][r], twiddle(a.twiddle, r * k * step, SIGN));
         }
-        if (R == 2) dft2<SIGN>(v[p]);
-        else if (R == 4) dft4<SIGN>(v[p][0], v[p][1], v[p][2], v[p][3]);
-        else if (R == 8) dft8<SIGN>(v[p]);
-        else if (R == 3) dft3<SIGN>(v[p]);
-        else if (R == 5) dft5<SIGN>(v[p]);
+        butterfly<SIGN, R>(v[p]);
         const int ob = (j[p] / Ns) * Ns * R + k;
         if (last) {
             double2* q = gdst + dst_base + (long long)kk[p] * a.dst.sv;

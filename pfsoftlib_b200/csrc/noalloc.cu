@@ -9,12 +9,12 @@
 // file-scope device array instead.
 //
 // Limit: bandwidth B <= 32 (a 64^3 complex128 spectrum, 4 MiB, plus 320 KiB reserved for the
-// tables, of which B = 32 needs about 276 KiB). Every GPU that loads the library holds this
+// tables, of which B = 32 needs about 125 KiB). Every GPU that loads the library holds this
 // array until the process exits. All calls on a device share it and it keeps the last call's
 // contents; nothing in it has to start at zero (the first FFT pass overwrites the whole spectrum
 // before anything reads it, and the tables are rebuilt whenever the bandwidth changes). Calls
 // that overlap on the GPU race on it. Once a call has been recorded into a CUDA graph on a
-// device, every later call on that device rebuilds the tables (three small kernels): a graph
+// device, every later call on that device rebuilds the tables (two small kernels and a clear): a graph
 // replay rewrites the array with its own bandwidth's tables, which the host cannot see.
 
 #include <cuda_runtime.h>
@@ -120,7 +120,7 @@ int pfsoft_cuda_dsoft_noalloc(const double* d_grid, int B, double* d_coeffs, voi
         fft_pass_launch(X, X, f2, N, -1, s) != cudaSuccess)
         return fail(PFSOFT_ECUDA, "pfsoft_cuda_dsoft_noalloc: FFT launch failed");
     const DwtArgs a = dwt_args_for(t);
-    if (dwt_forward_launch(X, reinterpret_cast<double2*>(d_coeffs), a, 0, s) != cudaSuccess)
+    if (dwt_forward_launch(X, reinterpret_cast<double2*>(d_coeffs), a, 1, s) != cudaSuccess)
         return fail(PFSOFT_ECUDA, "pfsoft_cuda_dsoft_noalloc: DWT launch failed");
     return PFSOFT_OK;
 }

@@ -3,8 +3,8 @@
 // Requests (DSOFT or iDSOFT of one caller-owned device grid / coefficient buffer) enter a FIFO
 // queue. A scheduler thread forms batches of equal direction and bandwidth (serving.hpp: the
 // arena the HBM budget is counted against, and the batch former), and launches each batch on a
-// free stream as one group: batched FFT passes (gridDim.z = transforms) and one fused DWT launch
-// (dwt_batch.cu) over the batch's (order class, transform block) items. In split mode
+// free stream as one group: batched FFT passes (gridDim.z = transforms) and one DWT launch
+// (dwt.cu) over the batch's (order class, transform) pairs. In split mode
 // (PFSOFT_SERVER_SPLIT) a batch takes requests of one direction and any bandwidths up to 256: FFT
 // passes per bandwidth group, then ONE split-precision DWT launch (dwt_split.cu) over every
 // group's items. Completion is stamped by
@@ -39,18 +39,15 @@
 using namespace pfsoft_dev;
 
 namespace pfsoft_dev {
-int tables_for(int B, cudaStream_t s, BandTables* out);   // api.cu
-int launch_group(int dir, const BandTables& t, int T, double2** d_grids, double2** d_ws, const DwtGroup* d_group,
-                 const DwtItem* d_items, int n_items, int* d_counter, int tpc, double2* const* h_coef,
-                 double2* const* h_ws, cudaStream_t s);   // batch.cu
-void group_items(int B, int T, int tpc, std::vector<DwtItem>& out);   // batch.cu
+int tables_for(int B, cudaStream_t s, BandTables* out, bool split = false);   // api.cu
+int launch_group(int dir, const BandTables& t, int T, double2** d_grids, double2** d_coefs, double2** d_ws,
+                 cudaStream_t s);   // batch.cu
 FftPassArgs group_pass_args(int dir, bool first, const BandTables& t, double2** grids, double2** ws);   // batch.cu
 cudaError_t zero_nyquist_launch(double2** ws, int B, int T, cudaStream_t s);   // batch.cu
 }  // namespace pfsoft_dev
 
 namespace {
 
-constexpr size_t kStageHeader = 128;   // DwtGroup, padded; pointer tables follow
 constexpr int kMaxBatchLimit = 256;
 constexpr int kMaxStreams = 16;
 constexpr size_t kLatencyWindow = (size_t)1 << 20;   // latency samples kept (the most recent)
@@ -72,7 +69,6 @@ struct Slot {
     cudaStream_t stream = nullptr;
     unsigned char* h_stage = nullptr;   // pinned: DwtGroup(s), [segments], then grid / coefficient / spectrum tables
     unsigned char* d_stage = nullptr;
-    int* d_counter = nullptr;
     int* h_status = nullptr;            // split mode: mapped host flag a timed-out bounded wait sets
     int* d_status = nullptr;            // its device alias
     Batch* batch = nullptr;             // the batch on the device, or null
@@ -98,15 +94,6 @@ struct Batch {
     int status = PFSOFT_OK;
 };
 
-// transforms per CTA of the fused DWT for a batch of k transforms at bandwidth B
-int tpc_for(int B, int k)
-{
-    const int N = 2 * B;
-    int t = dwt_batch_transforms_per_cta(N <= 64 ? 64 : (N <= 128 ? 128 : 256));
-    while (t > 1 && t > k) t >>= 1;
-    return t;
-}
-
 }  // namespace
 
 struct pfsoft_server {
@@ -123,8 +110,6 @@ struct pfsoft_server {
     long long next_id = 1;
     std::vector<Batch*> finished;   // done on the device, not yet reaped
     std::vector<cudaEvent_t> dead_events;   // of cancelled requests; destroyed without the mutex
-    // fused-DWT item lists per (B, k): scheduler thread only
-    std::map<std::pair<int, int>, std::pair<DwtItem*, int> > items;
     std::mutex mu;
     std::condition_variable cv;
     bool stop = false, paused = false;
@@ -157,28 +142,6 @@ void CUDART_CB on_batch_done(void* p)   // host function: no CUDA calls in here
     s->cv.notify_all();
 }
 
-// Device item list of a (B, k) batch, built on first use.
-int items_for(pfsoft_server* s, int B, int k, int tpc, const DwtItem** d_items, int* n)
-{
-    auto key = std::make_pair(B, k);
-    auto it = s->items.find(key);
-    if (it == s->items.end()) {
-        std::vector<DwtItem> v;
-        group_items(B, k, tpc, v);
-        DwtItem* d = nullptr;
-        cudaError_t e = cudaMalloc(&d, v.size() * sizeof(DwtItem));
-        if (e == cudaSuccess) e = cudaMemcpy(d, v.data(), v.size() * sizeof(DwtItem), cudaMemcpyHostToDevice);
-        if (e != cudaSuccess) {
-            cudaFree(d);
-            return fail(PFSOFT_ECUDA, std::string("server item list: ") + cudaGetErrorString(e));
-        }
-        it = s->items.emplace(key, std::make_pair(d, (int)v.size())).first;
-    }
-    *d_items = it->second.first;
-    *n = it->second.second;
-    return PFSOFT_OK;
-}
-
 // Split mode: batch b's requests grouped by bandwidth; FFT passes per group and one
 // split-precision DWT launch over all groups (scheduler thread, mutex not held). Stage layout:
 // DwtGroup[cap], segments[cap], then the grid / coefficient / spectrum pointer tables, members of
@@ -201,7 +164,7 @@ int launch_split_batch(pfsoft_server* s, Batch* b, const std::vector<Request>& i
     int pos = 0;
     for (const auto& kv : byB) {
         BandTables t;
-        const int rc = tables_for(kv.first, sl.stream, &t);
+        const int rc = tables_for(kv.first, sl.stream, &t, true);
         if (rc) return rc;
         const int g = (int)tabs.size();
         for (size_t m = 0; m < kv.second.size(); ++m) {
@@ -278,16 +241,9 @@ int launch_batch(pfsoft_server* s, Batch* b, const std::vector<Request>& io)
     BandTables t;
     int rc = tables_for(B, sl.stream, &t);
     if (rc) return rc;
-    const int tpc = tpc_for(B, k);
-    const DwtItem* d_items = nullptr;
-    int n_items = 0;
-    if (B <= 128) {
-        rc = items_for(s, B, k, tpc, &d_items, &n_items);
-        if (rc) return rc;
-    }
     const size_t cap = (size_t)s->max_batch;
-    double2** h_tab = reinterpret_cast<double2**>(sl.h_stage + kStageHeader);
-    double2** d_tab = reinterpret_cast<double2**>(sl.d_stage + kStageHeader);
+    double2** h_tab = reinterpret_cast<double2**>(sl.h_stage);
+    double2** d_tab = reinterpret_cast<double2**>(sl.d_stage);
     double2** h_grid = h_tab;
     double2** h_coef = h_tab + cap;
     double2** h_ws = h_tab + 2 * cap;
@@ -298,28 +254,13 @@ int launch_batch(pfsoft_server* s, Batch* b, const std::vector<Request>& io)
         h_coef[i] = reinterpret_cast<double2*>(const_cast<double*>(dir == 0 ? out : in));
         h_ws[i] = reinterpret_cast<double2*>(static_cast<char*>(s->arena_base) + b->plan.offset + b->plan.offs[i]);
     }
-    DwtGroup g;
-    g.B = B;
-    g.N = 2 * B;
-    g.T = k;
-    g.cosb = t.cosb;
-    g.w = t.w;
-    g.normf = t.normf;
-    g.pw_sin = t.pw_sin;
-    g.pw_cos = t.pw_cos;
-    g.rc_cf = t.rc_cf;
-    g.rc_f1 = t.rc_f1;
-    g.X = d_tab + 2 * cap;
-    g.coeffs = d_tab + cap;
-    std::memcpy(sl.h_stage, &g, sizeof(g));
     cudaError_t e = cudaSuccess;
     for (int i = 0; i < k && e == cudaSuccess; ++i)
         if (io[i].ready) e = cudaStreamWaitEvent(sl.stream, io[i].ready, 0);
-    if (e == cudaSuccess) e = cudaMemcpyAsync(sl.d_stage, sl.h_stage, kStageHeader + 3 * cap * sizeof(double2*),
+    if (e == cudaSuccess) e = cudaMemcpyAsync(sl.d_stage, sl.h_stage, 3 * cap * sizeof(double2*),
                                     cudaMemcpyHostToDevice, sl.stream);
     if (e != cudaSuccess) return fail(PFSOFT_ECUDA, std::string("server upload: ") + cudaGetErrorString(e));
-    rc = launch_group(dir, t, k, d_tab, d_tab + 2 * cap, reinterpret_cast<const DwtGroup*>(sl.d_stage), d_items,
-                      n_items, sl.d_counter, tpc, h_coef, h_ws, sl.stream);
+    rc = launch_group(dir, t, k, d_tab, d_tab + cap, d_tab + 2 * cap, sl.stream);
     if (rc) return rc;
     e = cudaLaunchHostFunc(sl.stream, on_batch_done, b);
     if (e != cudaSuccess) return fail(PFSOFT_ECUDA, std::string("server completion hook: ") + cudaGetErrorString(e));
@@ -468,13 +409,12 @@ int pfsoft_server_create_ex(size_t budget_bytes, int max_batch, int streams, int
     s->slots.resize(streams);
     const size_t tables = 3 * (size_t)max_batch * sizeof(double2*);
     const size_t stage = s->split ? (((size_t)max_batch * (sizeof(DwtGroup) + dwt_split_seg_bytes()) + 255) & ~size_t(255)) + tables
-                                  : kStageHeader + tables;
+                                  : tables;
     s->stage_bytes = stage;
     for (auto& sl : s->slots) {
         if (e == cudaSuccess) e = cudaStreamCreateWithFlags(&sl.stream, cudaStreamNonBlocking);
         if (e == cudaSuccess) e = cudaHostAlloc(reinterpret_cast<void**>(&sl.h_stage), stage, cudaHostAllocDefault);
         if (e == cudaSuccess) e = cudaMalloc(reinterpret_cast<void**>(&sl.d_stage), stage);
-        if (e == cudaSuccess) e = cudaMalloc(reinterpret_cast<void**>(&sl.d_counter), sizeof(int));
         if (e == cudaSuccess && s->split) e = cudaHostAlloc(reinterpret_cast<void**>(&sl.h_status), sizeof(int), cudaHostAllocMapped);
         if (e == cudaSuccess && s->split) {
             *sl.h_status = 0;
@@ -489,7 +429,6 @@ int pfsoft_server_create_ex(size_t budget_bytes, int max_batch, int streams, int
             if (sl.stream) cudaStreamDestroy(sl.stream);
             cudaFreeHost(sl.h_stage);
             cudaFree(sl.d_stage);
-            cudaFree(sl.d_counter);
             cudaFreeHost(sl.h_status);
         }
         if (s->table_stream) cudaStreamDestroy(s->table_stream);
@@ -517,10 +456,8 @@ int pfsoft_server_destroy(pfsoft_server* s)
         cudaStreamDestroy(sl.stream);
         cudaFreeHost(sl.h_stage);
         cudaFree(sl.d_stage);
-        cudaFree(sl.d_counter);
         cudaFreeHost(sl.h_status);
     }
-    for (auto& kv : s->items) cudaFree(kv.second.first);
     if (s->table_stream) cudaStreamDestroy(s->table_stream);
     for (cudaEvent_t ev : s->dead_events)
         if (ev) cudaEventDestroy(ev);
@@ -555,7 +492,7 @@ int pfsoft_server_submit(pfsoft_server* s, int direction, int B, const double* d
     // latency, counted from the end of this call, does not include them
     {
         BandTables t;
-        const int rc = tables_for(B, s->table_stream, &t);
+        const int rc = tables_for(B, s->table_stream, &t, s->split);
         if (rc) return rc;
     }
     cudaEvent_t ready = nullptr;

@@ -32,7 +32,7 @@ using namespace pfsoft_dev;
 using pfsoft_shard::Run;
 
 namespace pfsoft_dev {
-int tables_for(int B, cudaStream_t s, BandTables* out);   // api.cu: cached tables of a bandwidth
+int tables_for(int B, cudaStream_t s, BandTables* out, bool split = false);   // api.cu: cached tables of a bandwidth
 }
 
 namespace {
@@ -375,7 +375,7 @@ int pfsoft_shard_dwt_forward(pfsoft_shard_plan* plan, const double* d_spectrum, 
     DwtArgs a = dwt_args_for(t);
     a.classes = plan->d_classes;
     a.n_classes = n;
-    e = dwt_forward_launch(reinterpret_cast<const double2*>(d_spectrum), reinterpret_cast<double2*>(d_coeffs), a, 0, s);
+    e = dwt_forward_launch(reinterpret_cast<const double2*>(d_spectrum), reinterpret_cast<double2*>(d_coeffs), a, 1, s);
     return e == cudaSuccess ? PFSOFT_OK : cuda_fail(e, "shard DWT launch");
 }
 
@@ -394,7 +394,7 @@ int pfsoft_shard_dwt_inverse(pfsoft_shard_plan* plan, const double* d_coeffs, do
     DwtArgs a = dwt_args_for(t);
     a.classes = plan->d_classes;
     a.n_classes = n;
-    cudaError_t e = dwt_inverse_launch(reinterpret_cast<const double2*>(d_coeffs), reinterpret_cast<double2*>(d_spectrum), a, 0, s);
+    cudaError_t e = dwt_inverse_launch(reinterpret_cast<const double2*>(d_coeffs), reinterpret_cast<double2*>(d_spectrum), a, 1, s);
     return e == cudaSuccess ? PFSOFT_OK : cuda_fail(e, "shard DWT launch");
 }
 

@@ -2,15 +2,19 @@
 //
 //   cos(beta_k), sin(beta_k/2), cos(beta_k/2)  beta_k = pi(2k+1)/(4B)     fn_dwt.hpp:155-159
 //   w_B(j) = 2/B sin(pi(2j+1)/(4B)) sum_{k<B} sin((2j+1)(2k+1)pi/(4B))/(2k+1)   fn_dwt.hpp:62-83
+//   twiddle[t] = exp(-2 pi i t/N), ht[n] = {cos, sin}(pi n/(2N))
+//   delta: the Wigner rows at beta = pi/2, whose products are the rows' Fourier coefficients in beta
+// and for the split-precision DWT alone
 //   normf(M,M') = sqrt((2M+1)/2) prod_{i<M-M'} sqrt((2M-i)/(i+1))              fn_dwt.hpp:117-121
-//   twiddle[t] = exp(-2 pi i t/N)
 //   rc_cf / rc_f1: the recurrence coefficients c1, f1 f2 and f1 of every class and degree
-//       (fn_dwt.hpp:167-199), so that the DWT kernels load them instead of recomputing them
+//       (fn_dwt.hpp:167-199), so that the kernel loads them instead of recomputing them
 //   pw_sin[p][k], pw_cos[p][k] = sin(beta_k/2)^p, cos(beta_k/2)^p, p < 2B, as an exact binary
 //       exponent and a mantissa in [0.5, 1) (exponentiation by squaring, renormalised each
 //       product), so that Wigner seeds far below the FP64 range keep full relative precision
 // The sine arguments are reduced exactly in integers before sinpi/cospi, and the weight sum
 // is compensated (Neumaier), so each entry is within a few ulp of the exact value.
+
+#include <algorithm>
 
 #include "common.cuh"
 #include "dwt.cuh"
@@ -58,8 +62,8 @@ __global__ void powers_kernel(int B, const double* sinh, const double* cosh, dou
     }
 }
 
-__global__ void tables_kernel(int B, double* cosb, double* sinh, double* cosh, double* w, double* normf,
-                              double2* tw)
+__global__ void tables_kernel(int B, double* cosb, double* sinh, double* cosh, double* w,
+                              double2* tw, double2* ht)
 {
     const int N = 2 * B;
     const int tid = blockIdx.x * blockDim.x + threadIdx.x;
@@ -75,6 +79,10 @@ __global__ void tables_kernel(int B, double* cosb, double* sinh, double* cosh, d
         double ts, tc;
         sincospi(2.0 * (double)k / (double)N, &ts, &tc);
         tw[k] = make_double2(tc, -ts);
+        if (k < B) {
+            sincospi((double)k / (double)(2 * N), &ts, &tc);
+            ht[k] = make_double2(tc, ts);
+        }
         // weights are symmetric, w(N-1-k) = w(k) (fn_dwt.hpp:80-81): compute k < B, mirror
         if (k >= B) continue;
         // exact integer reduction of (2k+1)(2q+1) modulo 8B (period of sin(pi p/(4B)))
@@ -91,6 +99,13 @@ __global__ void tables_kernel(int B, double* cosb, double* sinh, double* cosh, d
         w[k] = wk;
         w[N - 1 - k] = wk;
     }
+}
+
+// Seed norms of the order classes.
+__global__ void normf_kernel(int B, double* normf)
+{
+    const int tid = blockIdx.x * blockDim.x + threadIdx.x;
+    const int nthr = gridDim.x * blockDim.x;
     const int ncls = num_classes(B);
     for (int i = tid; i < ncls; i += nthr) {
         int M, Mp;
@@ -115,49 +130,173 @@ __global__ void rc_kernel(int B, double2* rc_cf, double* rc_f1)
     }
 }
 
+// The cosines and sines of the beta sums (BandTables::trig); n (2k+1) is reduced modulo 8B, the period of
+// the angle pi n (2k+1) / (4B).
+__global__ void trig_kernel(int B, double* trig)
+{
+    const int nb = (B + 7) / 8, mb = (nb + 1) / 2;
+    const long long total = trig_entries(B);
+    for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < total; i += (long long)gridDim.x * blockDim.x) {
+        const int tile = (int)(i / 64), kt = tile % nb, mt = tile / nb % mb, q = tile / (nb * mb) & 1, sine = tile / (2 * nb * mb);
+        const int n = 2 * (8 * mt + (int)(i >> 3 & 7)) + q, k = 8 * kt + (int)(i & 7);
+        double v = 0.0;
+        if (n < B && k < B) {
+            const double x = (double)(((long long)n * (2 * k + 1)) % (8LL * B)) / (double)(4 * B);
+            v = (n == 0 ? 1.0 : 2.0) * (sine ? sinpi(x) : cospi(x));
+        }
+        trig[i] = v;
+    }
+}
+
+// ---- the rows at beta = pi/2, in double-double arithmetic (Dekker 1971, Knuth; products by FMA) ----
+struct dd {
+    double h, l;
+};
+__device__ __forceinline__ dd quick_sum(double a, double b)   // |a| >= |b|
+{
+    const double s = a + b;
+    return {s, b - (s - a)};
+}
+__device__ __forceinline__ dd dd_add(dd a, dd b)
+{
+    const double s = a.h + b.h, v = s - a.h;
+    const double e = (a.h - (s - v)) + (b.h - v);
+    return quick_sum(s, e + a.l + b.l);
+}
+__device__ __forceinline__ dd dd_mul(dd a, dd b)
+{
+    const double p = a.h * b.h;
+    return quick_sum(p, fma(a.h, b.h, -p) + (a.h * b.l + a.l * b.h));
+}
+__device__ __forceinline__ dd dd_scale(dd a, double b)
+{
+    const double p = a.h * b;
+    return quick_sum(p, fma(a.h, b, -p) + a.l * b);
+}
+__device__ __forceinline__ dd dd_div(dd a, dd b)
+{
+    const double q = a.h / b.h;
+    const dd r = dd_add(a, dd_scale(b, -q));
+    return quick_sum(q, (r.h + r.l) / b.h);
+}
+__device__ __forceinline__ dd dd_sqrt(dd a)
+{
+    if (a.h == 0.0) return {0.0, 0.0};
+    const double r = sqrt(a.h);
+    return quick_sum(r, (fma(-r, r, a.h) + a.l) / (2.0 * r));
+}
+
+// P[l][a][b] for one pair a >= b per thread, l = a .. B-1, and its mirror image: the recurrence of
+// fn_dwt.hpp:167-199 at cos beta = 0 without its normalisation,
+//   P(l+1) = -((2l+1) a b P(l) + (l+1) sqrt(q(l)) P(l-1)) / (l sqrt(q(l+1))),  q(l) = (l^2-a^2)(l^2-b^2),
+// from P(a) = sqrt(binomial(2a, a-b)) 2^-a. Double-double keeps the products of two entries within
+// two ulp over any number of steps. The table starts zeroed.
+__global__ void delta_kernel(int B, double* delta)
+{
+    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= num_classes(B)) return;
+    int a, b;
+    class_orders(i, a, b);
+    dd cur = {1.0, 0.0}, prev = {0.0, 0.0};
+    for (int q = 0; q < a - b; ++q) cur = dd_div(dd_scale(cur, (double)(2 * a - q)), dd{(double)(q + 1), 0.0});
+    cur = dd_sqrt(cur);
+    cur.h = ldexp(cur.h, -a);
+    cur.l = ldexp(cur.l, -a);
+    auto at = [&](int M, int n, int l) {
+        const int lb = l >> 3, b0 = M >> 3;
+        return delta_offset(B, M) + 64 * (long long)(lb * (lb + 1) / 2 - b0 * (b0 + 1) / 2 + (n >> 3)) + (l & 7) * 8 + (n & 7);
+    };
+    dd sq = {0.0, 0.0};   // sqrt(q(l))
+    for (int l = a; l < B; ++l) {
+        // with a fourth root of the rows' squared norm, so that a product of two has its square root
+        const dd x = dd_mul(cur, dd_sqrt(dd_sqrt(dd{l + 0.5, 0.0})));
+        const double v = x.h + x.l;
+        delta[at(a, b, l)] = v;
+        if (a != b) delta[at(b, a, l)] = ((a - b) & 1) ? -v : v;
+        const double k2 = (double)(l + 1) * (l + 1);
+        const double q1 = (k2 - (double)a * a) * (k2 - (double)b * b);   // an exact integer
+        const dd sn = dd_sqrt(dd{q1, 0.0});
+        dd nx = {0.0, 0.0};
+        if (l > 0) {
+            nx = dd_add(dd_scale(cur, (double)(2 * l + 1) * a * b), dd_scale(dd_mul(sq, prev), (double)(l + 1)));
+            nx = dd_div(nx, dd_scale(sn, -(double)l));
+        }
+        prev = cur;
+        cur = nx;
+        sq = sn;
+    }
+}
+
 }  // namespace
 
 size_t tables_bytes(int B)
 {
-    const size_t N = 2 * (size_t)B, R = (size_t)rc_entries(B);
-    return 4 * align256(N * sizeof(double)) + align256(num_classes(B) * sizeof(double)) +
-           align256(N * sizeof(double2)) + 2 * align256(2 * (size_t)B * N * sizeof(double2)) +
-           align256(R * sizeof(double2)) + align256(R * sizeof(double));
+    const size_t N = 2 * (size_t)B;
+    return 4 * align256(N * sizeof(double)) + align256(N * sizeof(double2)) +
+           align256(B * sizeof(double2)) + align256((size_t)delta_entries(B) * sizeof(double)) +
+           align256((size_t)trig_entries(B) * sizeof(double));
 }
 
 cudaError_t tables_build(int B, void* mem, BandTables* t, cudaStream_t stream)
 {
     const size_t N = 2 * (size_t)B;
     char* p = static_cast<char*>(mem);
+    *t = BandTables();
     t->B = B;
     t->N = (int)N;
     t->block = mem;
-    t->cosb = reinterpret_cast<double*>(p);
-    p += align256(N * sizeof(double));
-    t->sinh = reinterpret_cast<double*>(p);
-    p += align256(N * sizeof(double));
-    t->cosh = reinterpret_cast<double*>(p);
-    p += align256(N * sizeof(double));
-    t->w = reinterpret_cast<double*>(p);
-    p += align256(N * sizeof(double));
+    auto take = [&](size_t bytes) {
+        char* q = p;
+        p += align256(bytes);
+        return q;
+    };
+    t->cosb = reinterpret_cast<double*>(take(N * sizeof(double)));
+    t->sinh = reinterpret_cast<double*>(take(N * sizeof(double)));
+    t->cosh = reinterpret_cast<double*>(take(N * sizeof(double)));
+    t->w = reinterpret_cast<double*>(take(N * sizeof(double)));
+    t->twiddle = reinterpret_cast<double2*>(take(N * sizeof(double2)));
+    t->ht = reinterpret_cast<double2*>(take(B * sizeof(double2)));
+    const size_t dbytes = (size_t)delta_entries(B) * sizeof(double);
+    t->delta = reinterpret_cast<double*>(take(dbytes));
+    t->trig = reinterpret_cast<double*>(take((size_t)trig_entries(B) * sizeof(double)));
+    const int threads = 64;
+    tables_kernel<<<((int)N + threads - 1) / threads, threads, 0, stream>>>(B, t->cosb, t->sinh, t->cosh, t->w,
+                                                                             t->twiddle, t->ht);
+    cudaError_t e = cudaGetLastError();
+    if (e == cudaSuccess) e = cudaMemsetAsync(t->delta, 0, dbytes, stream);
+    if (e != cudaSuccess) return e;
+    delta_kernel<<<(num_classes(B) + threads - 1) / threads, threads, 0, stream>>>(B, t->delta);
+    e = cudaGetLastError();
+    if (e != cudaSuccess) return e;
+    trig_kernel<<<(int)std::min<long long>((trig_entries(B) + 255) / 256, 1024), 256, 0, stream>>>(B, t->trig);
+    return cudaGetLastError();
+}
+
+size_t split_tables_bytes(int B)
+{
+    const size_t N = 2 * (size_t)B, R = (size_t)rc_entries(B);
+    return align256(num_classes(B) * sizeof(double)) + 2 * align256(N * N * sizeof(double2)) +
+           align256(R * sizeof(double2)) + align256(R * sizeof(double));
+}
+
+cudaError_t split_tables_build(int B, void* mem, BandTables* t, cudaStream_t stream)
+{
+    const size_t N = 2 * (size_t)B;
+    char* p = static_cast<char*>(mem);
     t->normf = reinterpret_cast<double*>(p);
     p += align256(num_classes(B) * sizeof(double));
-    t->twiddle = reinterpret_cast<double2*>(p);
-    p += align256(N * sizeof(double2));
     t->pw_sin = reinterpret_cast<double2*>(p);
-    p += align256(2 * (size_t)B * N * sizeof(double2));
+    p += align256(N * N * sizeof(double2));
     t->pw_cos = reinterpret_cast<double2*>(p);
-    p += align256(2 * (size_t)B * N * sizeof(double2));
+    p += align256(N * N * sizeof(double2));
     t->rc_cf = reinterpret_cast<double2*>(p);
     p += align256((size_t)rc_entries(B) * sizeof(double2));
     t->rc_f1 = reinterpret_cast<double*>(p);
     const int threads = 128;
-    int blocks = (int)((num_classes(B) + threads - 1) / threads);
-    if (blocks < 1) blocks = 1;
-    tables_kernel<<<blocks, threads, 0, stream>>>(B, t->cosb, t->sinh, t->cosh, t->w, t->normf, t->twiddle);
+    normf_kernel<<<(num_classes(B) + threads - 1) / threads, threads, 0, stream>>>(B, t->normf);
     cudaError_t e = cudaGetLastError();
     if (e != cudaSuccess) return e;
-    const long long total = (long long)2 * B * N;
+    const long long total = (long long)N * N;
     int pblocks = (int)((total + 255) / 256);
     if (pblocks > 4096) pblocks = 4096;
     powers_kernel<<<pblocks, 256, 0, stream>>>(B, t->sinh, t->cosh, t->pw_sin, t->pw_cos);
