@@ -7,7 +7,8 @@
 // and the last stage leaves the result in natural order. The first stage reads HBM directly
 // into registers and the last stage writes HBM directly from registers; the stages between
 // exchange through shared memory (ping-pong buffers). Radices 2, 4, 8, 16, 3, 5 have
-// register butterflies; any other prime uses a direct O(R^2) butterfly.
+// register butterflies; a length with any other prime factor runs the chirp pass (fft_chirp_kernel),
+// or, beyond its sizes, direct O(R^2) butterflies.
 //
 // Coalescing: each stage picks its butterfly -> thread map from the stride of the HBM side
 // it touches. If consecutive elements of a vector are contiguous in HBM (se == 1) threads run
@@ -456,129 +457,240 @@ __global__ void __launch_bounds__(256, Tile::kMinBlocks) fft_fused_kernel(const 
     }
 }
 
-// Bluestein pass: kBluesteinVec vectors per CTA, each loaded, multiplied by its chirp and
-// zero-padded to M in shared memory, transformed (radix-2 stages, two per pass over shared memory;
-// decimation in frequency: natural order in, bit-reversed out), multiplied by the bit-reversed
-// transform of the chirp kernel (1/M
-// included), transformed back (decimation in time: bit-reversed in, natural out), multiplied by
-// the chirp and stored. The same HBM access pattern as a pass kernel's first and last stages.
-constexpr int kBluesteinVec = 4;
+// Bluestein pass for a length n with a large prime factor. An even n is first split in two (decimation
+// in frequency): outputs 2k + s are the length n/2 DFT of (x_j + x_(j+n/2)) or (x_j - x_(j+n/2))
+// w_n^j. Each length-m DFT (m = n/2, or n when odd) is the chirp-z convolution
+//   X_k = w_k sum_j (x_j w_j) conj(w_(k-j)),  w_j = exp(-pi i j^2 / m),
+// by two transforms of the smallest planned length M >= 2m - 1: decimation in frequency with radices
+// R0, R1, R2 (natural order in, digit-reversed out), a product with the chirp's transform stored in
+// that order, and decimation in time back. The first stage reads HBM into registers (its upper half
+// of inputs is zero), the last forward stage, the product and the first backward stage work on one
+// thread's registers, and the last stage stores to HBM (its upper half of outputs is not needed), so
+// that a sequence crosses shared memory four times (two radices: twice). A backward DFT is the
+// forward one of the conjugate.
+// What bounds it: FP64 arithmetic and the shared-memory pipe, about 4 M (M/m) log2 M multiply-adds a
+// value. Measured on B200 per pass, against radix-4
+// stages in shared memory at M >= 2n - 1: n = 74 19 us (47), 202 207 us (673), 274 463 us (2592),
+// 502 2.58 ms (9.15 ms).
+template <int R0_, int R1_, int R2_, int V_>
+struct ChirpPlan {
+    static constexpr int R0 = R0_, R1 = R1_, R2 = R2_, V = V_;   // V vectors per CTA; R2 = 1: two radices
+    static constexpr int M = R0 * R1 * R2, h0 = M / R0, h1 = h0 / R1;
+    static constexpr int RL = R2 > 1 ? R2 : R1;                  // the last radix, on contiguous elements
+    // one pad slot per RL elements when RL is even: the threads' runs then start in distinct banks
+    static constexpr int kPad = RL == 16 ? 4 : (RL == 8 ? 3 : (RL == 4 ? 2 : 31));
+    static __device__ __forceinline__ int pos(int i) { return kPad < 31 ? i + (i >> (kPad & 15)) : i; }
+    static constexpr int kLen = kPad < 31 ? M + (M >> (kPad & 15)) : M;
+    // pitch of a sequence: consecutive vectors' elements in distinct banks
+    static constexpr int PM = V == 4 ? kLen + ((10 - kLen % 8) % 8) : (kLen | 1);
+    static constexpr size_t kSmem = (size_t)2 * V * PM * sizeof(double2);
+    static constexpr int kMinBlocks = kSmem <= 50 * 1024 ? 3 : 2;
+};
 
+// The radix-R0 = 8 butterfly of a first stage whose inputs 4..7 are zero.
 template <int SIGN>
-__global__ void __launch_bounds__(256) fft_bluestein_kernel(const double2* src, double2* dst, const FftPassArgs a, int logM)
+__device__ __forceinline__ void dft8_half(double2* v)
 {
-    const int M = 1 << logM;
-    extern __shared__ double2 smem[];   // [kBluesteinVec][M]
+    const double2 r2 = cmul_i<SIGN>(v[2]), r3 = cmul_i<SIGN>(v[3]);
+    const double2 e0 = cadd(v[0], v[2]), e2 = csub(v[0], v[2]), e1 = cadd(v[0], r2), e3 = csub(v[0], r2);
+    const double2 o0 = cadd(v[1], v[3]);
+    const double2 o1 = rot8<SIGN, 1>(cadd(v[1], r3)), o2 = rot8<SIGN, 2>(csub(v[1], v[3])), o3 = rot8<SIGN, 3>(csub(v[1], r3));
+    v[0] = cadd(e0, o0);
+    v[4] = csub(e0, o0);
+    v[1] = cadd(e1, o1);
+    v[5] = csub(e1, o1);
+    v[2] = cadd(e2, o2);
+    v[6] = csub(e2, o2);
+    v[3] = cadd(e3, o3);
+    v[7] = csub(e3, o3);
+}
+
+template <class P>
+__global__ void __launch_bounds__(256, P::kMinBlocks)
+    fft_chirp_kernel(const double2* src, double2* dst, const __grid_constant__ FftPassArgs a, int sign)
+{
+    constexpr int R0 = P::R0, R1 = P::R1, R2 = P::R2, RL = P::RL, V = P::V, M = P::M, h0 = P::h0, h1 = P::h1, PM = P::PM;
+    static_assert(R0 == 8, "the first stage's butterfly");
+    extern __shared__ double2 smem[];   // [2][V][PM]
     if (a.srcs) {
         src = a.srcs[blockIdx.z];
         dst = a.dsts[blockIdx.z];
     }
-    const int n = a.n, half = M >> 1;
-    const double2* wtab = a.bluestein;                                 // exp(-pi i e^2 / n)
-    const double2* fh = a.bluestein + n + (SIGN < 0 ? 0 : M);          // bit-reversed, 1/M included
-    const double2* tw = a.bluestein + n + 2 * M;                       // exp(-2 pi i t / M), t < M/2
-    const int v0 = blockIdx.x * kBluesteinVec;
-    const int nv = min(kBluesteinVec, a.nvec - v0);
+    const int n = a.n;
+    const bool split = (n & 1) == 0;
+    const int m = split ? n >> 1 : n, S = split ? 2 * V : V;
+    const double2* wtab = a.bluestein;               // w_j
+    const double2* ctab = wtab + m;                  // w_j w_n^j
+    const double2* fh = ctab + m;                    // the chirp's transform, digit-reversed, 1/M included
+    const double2* tw1 = fh + M;                     // w_M^(i q), [q - 1][i]
+    const double2* tw2 = tw1 + (R0 - 1) * h0;        // w_h0^(i q), [q - 1][i]
+    const int v0 = blockIdx.x * V;
+    const int nv = min(V, a.nvec - v0);
     const long long sbase = (long long)v0 * a.src.sv + (long long)blockIdx.y * a.src.sb;
     const long long dbase = (long long)v0 * a.dst.sv + (long long)blockIdx.y * a.dst.sb;
     const bool vfast_in = a.src.se != 1, vfast_out = a.dst.se != 1;   // vectors contiguous in HBM
-    for (int t = threadIdx.x; t < kBluesteinVec * M; t += blockDim.x) {
-        int v, e;
-        if (vfast_in) {
-            v = t % kBluesteinVec;
-            e = t / kBluesteinVec;
-        } else {
-            e = t & (M - 1);
-            v = t >> logM;
+    const double cj = sign < 0 ? 1.0 : -1.0;
+    for (int t = threadIdx.x; t < V * h0; t += 256) {
+        const int v = vfast_in ? t % V : t / h0, i = vfast_in ? t / V : t % h0;
+        const double2* p = src + sbase + (long long)v * a.src.sv;
+        double2 u[R0], z[R0], x[R0 / 2], y[R0 / 2];
+#pragma unroll
+        for (int q = 0; q < R0 / 2; ++q) {
+            const int j = i + q * h0;
+            const bool in = v < nv && j < m;
+            x[q] = y[q] = make_double2(0.0, 0.0);
+            if (in) x[q] = load_src(a, p + (long long)j * a.src.se);
+            if (in && split) y[q] = load_src(a, p + (long long)(j + m) * a.src.se);
         }
-        double2 x = make_double2(0.0, 0.0);
-        if (v < nv && e < n) {
-            double2 w = wtab[e];
-            if (SIGN > 0) w.y = -w.y;
-            x = cmul(load_src(a, src + sbase + (long long)v * a.src.sv + (long long)e * a.src.se), w);
+#pragma unroll
+        for (int q = 0; q < R0 / 2; ++q) {
+            const int j = min(i + q * h0, m - 1);
+            x[q].y *= cj;
+            y[q].y *= cj;
+            u[q] = cmul(cadd(x[q], y[q]), __ldg(wtab + j));
+            z[q] = cmul(csub(x[q], y[q]), __ldg(ctab + j));
         }
-        smem[v * M + e] = x;
+        dft8_half<-1>(u);
+        double2* o = smem + v * PM;
+        o[P::pos(i)] = u[0];
+#pragma unroll
+        for (int q = 1; q < R0; ++q) o[P::pos(i + q * h0)] = cmul(u[q], __ldg(tw1 + (q - 1) * h0 + i));
+        if (split) {
+            dft8_half<-1>(z);
+            o += V * PM;
+            o[P::pos(i)] = z[0];
+#pragma unroll
+            for (int q = 1; q < R0; ++q) o[P::pos(i + q * h0)] = cmul(z[q], __ldg(tw1 + (q - 1) * h0 + i));
+        }
     }
     __syncthreads();
-    // forward, decimation in frequency: two radix-2 stages (spans 2^ls and 2^(ls-1)) per pass over
-    // shared memory, the same arithmetic as one stage at a time
-    int ls = logM - 1;
-    for (; ls >= 1; ls -= 2) {
-        const int sp = 1 << ls, h = sp >> 1, tA = logM - 1 - ls, tB = logM - ls;
-        for (int b = threadIdx.x; b < kBluesteinVec * (M >> 2); b += blockDim.x) {
-            const int i = b & (h - 1);
-            const int p0 = ((b >> (ls - 1)) << (ls + 1)) + i, p1 = p0 + h, p2 = p0 + sp, p3 = p2 + h;
-            const double2 x0 = smem[p0], x1 = smem[p1], x2 = smem[p2], x3 = smem[p3];
-            const double2 a0 = cadd(x0, x2), a2 = cmul(csub(x0, x2), tw[i << tA]);
-            const double2 a1 = cadd(x1, x3), a3 = cmul(csub(x1, x3), tw[(i + h) << tA]);
-            const double2 wb = tw[i << tB];
-            smem[p0] = cadd(a0, a1);
-            smem[p1] = cmul(csub(a0, a1), wb);
-            smem[p2] = cadd(a2, a3);
-            smem[p3] = cmul(csub(a2, a3), wb);
+    if constexpr (R2 > 1) {
+        for (int t = threadIdx.x; t < S * (M / R1); t += 256) {
+            const int i = t % h1, blk = t / h1 % R0, sq = t / (M / R1);
+            double2* o = smem + sq * PM;
+            double2 u[R1];
+#pragma unroll
+            for (int q = 0; q < R1; ++q) u[q] = o[P::pos(blk * h0 + i + q * h1)];
+            butterfly<-1, R1>(u);
+            o[P::pos(blk * h0 + i)] = u[0];
+#pragma unroll
+            for (int q = 1; q < R1; ++q) o[P::pos(blk * h0 + i + q * h1)] = cmul(u[q], __ldg(tw2 + (q - 1) * h1 + i));
         }
         __syncthreads();
     }
-    if (ls == 0) {   // an odd number of stages: the last one alone (span 1, twiddle 1)
-        for (int b = threadIdx.x; b < kBluesteinVec * half; b += blockDim.x) {
-            const int p = b << 1;
-            const double2 u = smem[p], x = smem[p + 1];
-            smem[p] = cadd(u, x);
-            smem[p + 1] = csub(u, x);
-        }
-        __syncthreads();
+    for (int t = threadIdx.x; t < S * (M / RL); t += 256) {
+        const int e = t % (M / RL) * RL;
+        double2* o = smem + t / (M / RL) * PM;
+        double2 u[RL];
+#pragma unroll
+        for (int q = 0; q < RL; ++q) u[q] = o[P::pos(e + q)];
+        butterfly<-1, RL>(u);
+#pragma unroll
+        for (int q = 0; q < RL; ++q) u[q] = cmul(u[q], __ldg(fh + e + q));
+        butterfly<+1, RL>(u);
+#pragma unroll
+        for (int q = 0; q < RL; ++q) o[P::pos(e + q)] = u[q];
     }
-    for (int t = threadIdx.x; t < kBluesteinVec * M; t += blockDim.x) smem[t] = cmul(smem[t], fh[t & (M - 1)]);
     __syncthreads();
-    // inverse, decimation in time: spans 2^ls and 2^(ls+1) per pass (conjugate twiddles)
-    ls = 0;
-    for (; ls + 1 < logM; ls += 2) {
-        const int sp = 1 << ls, t1 = logM - 1 - ls, t2 = logM - 2 - ls;
-        for (int b = threadIdx.x; b < kBluesteinVec * (M >> 2); b += blockDim.x) {
-            const int i = b & (sp - 1);
-            const int p0 = ((b >> ls) << (ls + 2)) + i, p1 = p0 + sp, p2 = p1 + sp, p3 = p2 + sp;
-            double2 w = tw[i << t1];
-            w.y = -w.y;
-            const double2 x0 = smem[p0], x1 = cmul(smem[p1], w), x2 = smem[p2], x3 = cmul(smem[p3], w);
-            const double2 a0 = cadd(x0, x1), a1 = csub(x0, x1), a2 = cadd(x2, x3), a3 = csub(x2, x3);
-            double2 w0 = tw[i << t2], w1 = tw[(i + sp) << t2];
-            w0.y = -w0.y;
-            w1.y = -w1.y;
-            const double2 b2 = cmul(a2, w0), b3 = cmul(a3, w1);
-            smem[p0] = cadd(a0, b2);
-            smem[p2] = csub(a0, b2);
-            smem[p1] = cadd(a1, b3);
-            smem[p3] = csub(a1, b3);
+    if constexpr (R2 > 1) {
+        for (int t = threadIdx.x; t < S * (M / R1); t += 256) {
+            const int i = t % h1, blk = t / h1 % R0, sq = t / (M / R1);
+            double2* o = smem + sq * PM;
+            double2 u[R1];
+            u[0] = o[P::pos(blk * h0 + i)];
+#pragma unroll
+            for (int q = 1; q < R1; ++q) {
+                double2 w = __ldg(tw2 + (q - 1) * h1 + i);
+                w.y = -w.y;
+                u[q] = cmul(o[P::pos(blk * h0 + i + q * h1)], w);
+            }
+            butterfly<+1, R1>(u);
+#pragma unroll
+            for (int q = 0; q < R1; ++q) o[P::pos(blk * h0 + i + q * h1)] = u[q];
         }
         __syncthreads();
     }
-    if (ls == logM - 1) {   // the last stage alone (span M/2)
-        for (int b = threadIdx.x; b < kBluesteinVec * half; b += blockDim.x) {
-            const int i = b & (half - 1);
-            const int p = ((b >> (logM - 1)) << logM) + i, q = p + half;
-            double2 w = tw[i];
-            w.y = -w.y;
-            const double2 u = smem[p], x = cmul(smem[q], w);
-            smem[p] = cadd(u, x);
-            smem[q] = csub(u, x);
-        }
-        __syncthreads();
-    }
-    for (int t = threadIdx.x; t < kBluesteinVec * n; t += blockDim.x) {
-        int v, k;
-        if (vfast_out) {
-            v = t % kBluesteinVec;
-            k = t / kBluesteinVec;
-        } else {
-            k = t % n;
-            v = t / n;
-        }
+    for (int t = threadIdx.x; t < V * h0; t += 256) {
+        const int v = vfast_out ? t % V : t / h0, i = vfast_out ? t / V : t % h0;
         if (v >= nv) continue;
-        double2 w = wtab[k];
-        if (SIGN > 0) w.y = -w.y;
-        dst[dbase + (long long)v * a.dst.sv + (long long)k * a.dst.se] = cscale(cmul(smem[v * M + k], w), a.scale);
+        double2* p = dst + dbase + (long long)v * a.dst.sv;
+#pragma unroll
+        for (int s = 0; s < 2; ++s) {
+            if (s == 1 && !split) break;
+            const double2* o = smem + (s * V + v) * PM;
+            double2 u[R0];
+            u[0] = o[P::pos(i)];
+#pragma unroll
+            for (int q = 1; q < R0; ++q) {
+                double2 w = __ldg(tw1 + (q - 1) * h0 + i);
+                w.y = -w.y;
+                u[q] = cmul(o[P::pos(i + q * h0)], w);
+            }
+            butterfly<+1, R0>(u);
+#pragma unroll
+            for (int q = 0; q < R0 / 2; ++q) {
+                const int k = i + q * h0;
+                if (k < m) {
+                    double2 r = cscale(cmul(u[q], __ldg(wtab + k)), a.scale);
+                    r.y *= cj;
+                    store_out(a, p + (long long)(split ? 2 * k + s : k) * a.dst.se, r);
+                }
+            }
+        }
     }
 }
+
+// Planned convolution lengths: the radices and a launch of each.
+struct ChirpEntry {
+    int r0, r1, r2, v;
+    cudaError_t (*launch)(const double2*, double2*, const FftPassArgs&, int, int, cudaStream_t, int);
+};
+
+template <class P>
+cudaError_t chirp_launch(const double2* src, double2* dst, const FftPassArgs& a, int ntiles, int sign, cudaStream_t stream, int nz)
+{
+    if (P::kSmem > 48 * 1024) {
+        const cudaError_t e = cudaFuncSetAttribute(fft_chirp_kernel<P>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)P::kSmem);
+        if (e != cudaSuccess) return e;
+    }
+    fft_chirp_kernel<P><<<dim3((a.nvec + P::V - 1) / P::V, ntiles, nz), 256, P::kSmem, stream>>>(src, dst, a, sign);
+    return cudaGetLastError();
+}
+
+template <int R0, int R1, int R2, int V>
+constexpr ChirpEntry chirp_entry()
+{
+    return {R0, R1, R2, V, chirp_launch<ChirpPlan<R0, R1, R2, V>>};
+}
+
+const ChirpEntry kChirps[] = {
+    chirp_entry<8, 8, 1, 16>(),   // 64
+    chirp_entry<8, 4, 3, 16>(),   // 96
+    chirp_entry<8, 16, 1, 8>(),   // 128
+    chirp_entry<8, 4, 5, 8>(),    // 160
+    chirp_entry<8, 8, 3, 8>(),    // 192
+    chirp_entry<8, 8, 4, 8>(),    // 256
+    chirp_entry<8, 8, 5, 4>(),    // 320
+    chirp_entry<8, 16, 3, 4>(),   // 384
+    chirp_entry<8, 8, 8, 4>(),    // 512
+    chirp_entry<8, 16, 5, 4>(),   // 640
+    chirp_entry<8, 8, 16, 2>(),   // 1024
+};
+
+// The plan for length n: the smallest M >= 2m - 1.
+const ChirpEntry& chirp_for(int n)
+{
+    const int m = n % 2 ? n : n / 2;
+    for (const ChirpEntry& c : kChirps)
+        if (c.r0 * c.r1 * c.r2 >= 2 * m - 1) return c;
+    return kChirps[sizeof(kChirps) / sizeof(kChirps[0]) - 1];
+}
+
+// The largest prime factor that does not go to the chirp pass. Even lengths, whose tables are kept: 5,
+// as measured against direct stages of 7, 11 and 13, us per pass: N = 28 10 / 11, 112 43 / 62, 154
+// 82 / 224, 224 250 / 297, 308 597 / 2014, 448 1975 / 2387. Odd lengths, whose table is made on the
+// host for each call: 16.
+int largest_direct_radix(int n) { return n % 2 ? 16 : 5; }
 
 // Lengths that run the in-place kernel: tile vectors and radices (0 ends a shorter plan). 384 is
 // planned 8.4.4.3 rather than 16.8.3: radix 16 does not fit the kernel's 64 registers. Measured
@@ -669,7 +781,7 @@ int fft_plan_radices(int n, int* radix, int* ns)
 
 bool fft_needs_bluestein(int n)
 {
-    if (n < 2 || n > 512) return false;
+    if (n < 2 || (n % 2 ? n : n / 2) > 512) return false;
     int rem = n, big = 1;
     for (int p = 2; p * p <= rem; ++p)
         while (rem % p == 0) {
@@ -677,70 +789,65 @@ bool fft_needs_bluestein(int n)
             rem /= p;
         }
     if (rem > 1) big = rem > big ? rem : big;
-    return big > 16;
-}
-
-int fft_bluestein_m(int n)
-{
-    int m = 1;
-    while (m < 2 * n - 1) m <<= 1;
-    return m;
+    return big > largest_direct_radix(n);
 }
 
 size_t fft_bluestein_elems(int n)
 {
-    const int M = fft_bluestein_m(n);
-    return (size_t)n + 2 * (size_t)M + (size_t)(M / 2);
+    const ChirpEntry& c = chirp_for(n);
+    const int M = c.r0 * c.r1 * c.r2, m = n % 2 ? n : n / 2, h0 = M / c.r0;
+    return 2 * (size_t)m + M + (size_t)(c.r0 - 1) * h0 + (c.r2 > 1 ? (size_t)(c.r1 - 1) * (h0 / c.r1) : 0);
 }
 
 void fft_bluestein_fill(int n, double2* out)
 {
     typedef long double ld;
     const ld pi = 3.14159265358979323846264338327950288L;
-    const int M = fft_bluestein_m(n);
-    int bits = 0;
-    while ((1 << bits) < M) ++bits;
-    // w_e = exp(-pi i e^2 / n), the exponent reduced mod 2n first
-    std::vector<ld> wr(n), wi(n);
-    for (int e = 0; e < n; ++e) {
-        const long long r = ((long long)e * e) % (2ll * n);
-        const ld ang = pi * (ld)r / (ld)n;
-        wr[e] = cosl(ang);
-        wi[e] = -sinl(ang);
-        out[e] = make_double2((double)wr[e], (double)wi[e]);
+    const ChirpEntry& c = chirp_for(n);
+    const int M = c.r0 * c.r1 * c.r2, m = n % 2 ? n : n / 2, h0 = M / c.r0, h1 = h0 / c.r1;
+    // w_j = exp(-pi i j^2 / m), the exponent reduced mod 2m first, and w_j exp(-2 pi i j / (2m))
+    std::vector<ld> wr(m), wi(m);
+    for (int j = 0; j < m; ++j) {
+        const ld ang = pi * (ld)(((long long)j * j) % (2ll * m)) / (ld)m;
+        wr[j] = cosl(ang);
+        wi[j] = -sinl(ang);
+        out[j] = make_double2((double)wr[j], (double)wi[j]);
+        const ld both = pi * (ld)(((long long)j * j + j) % (2ll * m)) / (ld)m;
+        out[m + j] = make_double2((double)cosl(both), (double)-sinl(both));
     }
     std::vector<ld> cr(M), ci(M);   // exp(-2 pi i t / M)
     for (int t = 0; t < M; ++t) {
         cr[t] = cosl(2 * pi * (ld)t / (ld)M);
         ci[t] = -sinl(2 * pi * (ld)t / (ld)M);
     }
-    for (int sg = 0; sg < 2; ++sg) {
-        // kernel h_d = conj(w(sign)_d), w(-1) = w, w(+1) = conj(w): h = conj(w) for sign -1, w for +1;
-        // placed at d and M - d
-        std::vector<ld> hr(M, 0), hi(M, 0);
-        for (int d = 0; d < n; ++d) {
-            const ld re = wr[d], im = sg == 0 ? -wi[d] : wi[d];
-            hr[d] = re;
-            hi[d] = im;
-            if (d > 0) {
-                hr[M - d] = re;
-                hi[M - d] = im;
-            }
-        }
-        for (int k = 0; k < M; ++k) {   // DFT (exp(-2 pi i jk / M)) / M, stored bit-reversed
-            ld sr = 0, si = 0;
-            for (int j = 0; j < M; ++j) {
-                const int t = (int)(((long long)j * k) & (M - 1));
-                sr += hr[j] * cr[t] - hi[j] * ci[t];
-                si += hr[j] * ci[t] + hi[j] * cr[t];
-            }
-            int br = 0;
-            for (int b = 0; b < bits; ++b)
-                if (k & (1 << b)) br |= 1 << (bits - 1 - b);
-            out[n + sg * M + br] = make_double2((double)(sr / M), (double)(si / M));
+    // the convolution kernel conj(w_d) at d and M - d, its DFT / M in the order the forward stages leave:
+    // index k = k0 + R0 (k1 + R1 k2) at k0 h0 + k1 h1 + k2
+    std::vector<ld> hr(M, 0), hi(M, 0);
+    for (int d = 0; d < m; ++d) {
+        hr[d] = wr[d];
+        hi[d] = -wi[d];
+        if (d > 0) {
+            hr[M - d] = wr[d];
+            hi[M - d] = -wi[d];
         }
     }
-    for (int t = 0; t < M / 2; ++t) out[n + 2 * M + t] = make_double2((double)cr[t], (double)ci[t]);
+    double2* fh = out + 2 * m;
+    for (int k = 0; k < M; ++k) {
+        ld sr = 0, si = 0;
+        for (int j = 0; j < M; ++j) {
+            const int t = (int)(((long long)j * k) % M);
+            sr += hr[j] * cr[t] - hi[j] * ci[t];
+            si += hr[j] * ci[t] + hi[j] * cr[t];
+        }
+        const int k0 = k % c.r0, k1 = k / c.r0 % c.r1, k2 = k / (c.r0 * c.r1);
+        fh[k0 * h0 + k1 * h1 + k2] = make_double2((double)(sr / M), (double)(si / M));
+    }
+    double2* tw = fh + M;
+    for (int q = 1; q < c.r0; ++q)
+        for (int i = 0; i < h0; ++i) *tw++ = make_double2((double)cr[q * i % M], (double)ci[q * i % M]);
+    if (c.r2 > 1)
+        for (int q = 1; q < c.r1; ++q)
+            for (int i = 0; i < h1; ++i) *tw++ = make_double2((double)cr[c.r0 * q * i % M], (double)ci[c.r0 * q * i % M]);
 }
 
 int fft_tile_vectors(int n)
@@ -760,17 +867,9 @@ cudaError_t fft_pass_launch(const double2* src, double2* dst, const FftPassArgs&
                             cudaStream_t stream, int nz)
 {
     if (a.bluestein && fft_needs_bluestein(a.n)) {
-        const int M = fft_bluestein_m(a.n);
-        int logM = 0;
-        while ((1 << logM) < M) ++logM;
-        const size_t sm = (size_t)kBluesteinVec * M * sizeof(double2);
-        dim3 grid((a.nvec + kBluesteinVec - 1) / kBluesteinVec, ntiles, nz);
-        auto goB = [&](auto kern) {
-            if (sm > 48 * 1024) cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
-            kern<<<grid, 256, sm, stream>>>(src, dst, a, logM);
-        };
-        sign < 0 ? goB(fft_bluestein_kernel<-1>) : goB(fft_bluestein_kernel<1>);
-        return cudaGetLastError();
+        FftPassArgs ab = a;
+        ab.stream_out = 1;
+        return chirp_for(a.n).launch(src, dst, ab, ntiles, sign, stream, nz);
     }
     const InplacePlan* ip = inplace_plan_of(a);
     // one butterfly per thread in the widest stage, up to 256 threads (the in-place kernels run

@@ -32,19 +32,16 @@ struct FftPassArgs {
     // last-stage stores marked evict-first (st.global.cs): set by fft_pass_launch, whose output is
     // not read again before it has left L2; left 0 where another pass reads it through L2
     int stream_out;
-    // lengths with a prime factor above 16 (fft_needs_bluestein): Bluestein's chirp tables
-    // (fft_bluestein_fill); null keeps the direct O(R^2) stages for that factor
+    // lengths that fft_needs_bluestein names: the chirp tables (fft_bluestein_fill); null keeps direct
+    // O(R^2) stages for their prime factors
     const double2* bluestein;
 };
 
-// Bluestein's algorithm for a length n <= 512 whose largest prime factor exceeds 16: the DFT as a
-// cyclic convolution of length M (the power of two >= 2n - 1) done with two radix-2 transforms in
-// shared memory (X_k = w_k sum_e x_e w_e conj(w_(k-e)), w_e = exp(sign pi i e^2 / n)).
+// Bluestein's algorithm (fft_chirp_kernel) for a length n whose largest prime factor is too large for a
+// direct stage: n <= 512, or even and <= 1024.
 bool fft_needs_bluestein(int n);
-int fft_bluestein_m(int n);
 size_t fft_bluestein_elems(int n);   // double2 entries of the table
-// The table, computed on the host in long double: w_e (e < n, sign -1), the bit-reversed length-M
-// transforms of the chirp kernel for sign -1 and +1 (1/M included), exp(-2 pi i t / M) (t < M/2).
+// The table, computed on the host in long double (layout: fft_chirp_kernel).
 void fft_bluestein_fill(int n, double2* out);
 
 // Radix plan for length n; returns the number of stages (0 if n cannot be planned).
