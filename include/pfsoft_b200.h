@@ -277,10 +277,8 @@ long long pfsoft_launch_count(void);
 /* Tuning knob of earlier DWT kernels: direction 0 = DSOFT, 1 = IDSOFT; case_split 0, 1 or 2. The
  * values are checked; the present kernels have one form for all symmetry cases. */
 int pfsoft_tune_dwt_case_split(int direction, int case_split);
-/* Tuning knob: on != 0 runs the two FFT passes of a direction in one persistent launch, layer
- * chunk by layer chunk, so that the second pass reads the first pass's output from L2; 0 (the
- * default) runs them as two launches. For bandwidth B (B <= 0: every bandwidth, clearing the
- * per-bandwidth choices). Process-wide; for measurements and the autotuner. */
+/* Tuning knob of an earlier form (both FFT passes of a direction in one launch), for bandwidth B (B <= 0:
+ * every bandwidth). The bandwidth is checked; the passes always run as two launches. */
 int pfsoft_tune_fft_fused(int B, int on);
 /* Tuning knob: whether a plan created with PFSOFT_BATCH_SPLIT runs bandwidth B's DWT on the split
  * kernel (use_split != 0, the default) or on the FP64 kernels (0). B <= 0: every bandwidth,

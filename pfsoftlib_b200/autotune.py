@@ -5,8 +5,8 @@ caches the winners in a JSON table keyed by GPU name and the sorted bandwidth co
 
   tune_batch  the `transforms_per_cta` argument of a batch plan (1, 2, 4; the present DWT kernels
               take one transform per CTA whatever it is);
-  tune_plan   per bandwidth: the FFT stage as one fused launch or two passes
-              (pfsoft_tune_fft_fused), and the DWT of a PFSOFT_BATCH_SPLIT plan on the
+  tune_plan   per bandwidth: pfsoft_tune_fft_fused on or off (without effect in the present
+              passes), and the DWT of a PFSOFT_BATCH_SPLIT plan on the
               split-precision kernel or the FP64 kernels (pfsoft_tune_split_bandwidth); the
               choices are applied to the library and returned.
 

@@ -462,19 +462,13 @@ int run_dsoft(const double* d_grid, int B, double* d_coeffs, void* ws, cudaStrea
     // F2: vectors = layers k, tile = gamma bin r, elements = column c; in place on X
     FftPassArgs f2 = pass_args(N, N, t, FftStrides{1, n2, n}, FftStrides{1, n2, n}, 1.0);
     if (f1.nstages == 0) return fail(PFSOFT_EINVAL, "FFT length cannot be planned");
-    if (fft_fused_enabled(N) && fft_fused_chunk(f1, f2)) {
-        // both passes in one launch; the counters sit past the spectrum in the workspace
-        StageScope sc(ST_FFT_FWD_FUSED, s);
-        PF_CUDA(fft_fused_launch(-1, f1, f2, N, N, 1, G, X, X, X, X, (long long)grid_elems(B), s));
-    } else {
-        {
-            StageScope sc(ST_FFT_FWD_ROWS, s);
-            PF_CUDA(fft_pass_launch(G, X, f1, N, -1, s));
-        }
-        {
-            StageScope sc(ST_FFT_FWD_COLS, s);
-            PF_CUDA(fft_pass_launch(X, X, f2, N, -1, s));
-        }
+    {
+        StageScope sc(ST_FFT_FWD_ROWS, s);
+        PF_CUDA(fft_pass_launch(G, X, f1, N, -1, s));
+    }
+    {
+        StageScope sc(ST_FFT_FWD_COLS, s);
+        PF_CUDA(fft_pass_launch(X, X, f2, N, -1, s));
     }
     DwtArgs a = dwt_args(t);
     {
@@ -504,18 +498,13 @@ int run_idsoft(const double* d_coeffs, int B, double* d_grid, void* ws, cudaStre
     // I1: inverse DFT over gamma, X[r][c][k] -> G[k][c][r], scaled by 1/(4B^2) (src/fn_idsoft.cpp:289)
     FftPassArgs i1 = pass_args(N, N, t, FftStrides{1, n, n2}, FftStrides{n2, n, 1}, 1.0 / (4.0 * B * B));
     if (i1.nstages == 0) return fail(PFSOFT_EINVAL, "FFT length cannot be planned");
-    if (fft_fused_enabled(N) && fft_fused_chunk(i2, i1)) {
-        StageScope sc(ST_FFT_INV_FUSED, s);
-        PF_CUDA(fft_fused_launch(+1, i2, i1, N, N, 1, X, X, X, G, X, (long long)grid_elems(B), s));
-    } else {
-        {
-            StageScope sc(ST_FFT_INV_COLS, s);
-            PF_CUDA(fft_pass_launch(X, X, i2, N, +1, s));
-        }
-        {
-            StageScope sc(ST_FFT_INV_ROWS, s);
-            PF_CUDA(fft_pass_launch(X, G, i1, N, +1, s));
-        }
+    {
+        StageScope sc(ST_FFT_INV_COLS, s);
+        PF_CUDA(fft_pass_launch(X, X, i2, N, +1, s));
+    }
+    {
+        StageScope sc(ST_FFT_INV_ROWS, s);
+        PF_CUDA(fft_pass_launch(X, G, i1, N, +1, s));
     }
     return PFSOFT_OK;
 }
@@ -727,13 +716,16 @@ static int layer_wise(int cols, int rows, int lays, double* d_arr, double scale,
             blu = t.bluestein;
         } else {
             // odd length: a private table (rare); freed after the stream drains
-            std::vector<double2> h(n);
+            std::vector<double2> h(fft_twiddle_elems(n));
             for (int i = 0; i < n; ++i) {
                 const long double a = 6.283185307179586476925286766559005768L * (long double)i / (long double)n;
                 h[i] = make_double2((double)cosl(a), -(double)sinl(a));
             }
-            PF_CUDA(cudaMalloc(&tmp, n * sizeof(double2)));
-            PF_CUDA(cudaMemcpyAsync(tmp, h.data(), n * sizeof(double2), cudaMemcpyHostToDevice, s));
+            int ra, rb;
+            if (fft_two_radices(n, &ra, &rb))
+                for (int i = 0; i < n; ++i) h[n + i] = h[(size_t)(i / ra + 1) * (i % ra) % n];
+            PF_CUDA(cudaMalloc(&tmp, h.size() * sizeof(double2)));
+            PF_CUDA(cudaMemcpyAsync(tmp, h.data(), h.size() * sizeof(double2), cudaMemcpyHostToDevice, s));
             PF_CUDA(cudaStreamSynchronize(s));
             tw = static_cast<const double2*>(tmp);
             if (fft_needs_bluestein(n)) {
@@ -865,7 +857,7 @@ long long pfsoft_launch_count(void) { return g_launches.load(); }
 int pfsoft_tune_fft_fused(int B, int on)
 {
     if (B > kMaxBandwidth) return fail(PFSOFT_EINVAL, "bandwidth must be at most 512");
-    fft_set_fused(B <= 0 ? 0 : 2 * B, on);
+    (void)on;   // both passes in one launch was never the faster form; the knob has no effect any more
     return PFSOFT_OK;
 }
 

@@ -129,28 +129,21 @@ cudaError_t group_dwt_launch(int dir, const BandTables& t, int T, double2** ws, 
     return dir == 0 ? dwt_forward_launch(nullptr, nullptr, a, T, s) : dwt_inverse_launch(nullptr, nullptr, a, T, s);
 }
 
-// Both FFT passes of a group: one fused launch when the plan allows (its counters at double2 offset
-// sync_off of each workspace), else the two passes.
-cudaError_t group_fft_launch(int dir, const BandTables& t, int T, double2** grids, double2** ws, long long sync_off,
-                             cudaStream_t s)
+// Both FFT passes of a group.
+cudaError_t group_fft_launch(int dir, const BandTables& t, int T, double2** grids, double2** ws, cudaStream_t s)
 {
     const int sign = dir == 0 ? -1 : +1;
-    const FftPassArgs a = group_pass_args(dir, true, t, grids, ws), b = group_pass_args(dir, false, t, grids, ws);
-    if (fft_fused_enabled(t.N) && fft_fused_chunk(a, b))
-        return fft_fused_launch(sign, a, b, t.N, t.N, T, nullptr, nullptr, nullptr, nullptr, nullptr, sync_off, s);
-    cudaError_t e = fft_pass_launch(nullptr, nullptr, a, t.N, sign, s, T);
-    return e == cudaSuccess ? fft_pass_launch(nullptr, nullptr, b, t.N, sign, s, T) : e;
+    cudaError_t e = fft_pass_launch(nullptr, nullptr, group_pass_args(dir, true, t, grids, ws), t.N, sign, s, T);
+    return e == cudaSuccess ? fft_pass_launch(nullptr, nullptr, group_pass_args(dir, false, t, grids, ws), t.N, sign, s, T) : e;
 }
 
 // One same-bandwidth group of T transforms in direction dir (0 forward, 1 inverse) on stream s;
 // d_grids / d_coefs / d_ws are device tables of T pointers.
 int launch_group(int dir, const BandTables& t, int T, double2** d_grids, double2** d_coefs, double2** d_ws, cudaStream_t s)
 {
-    const long long sync_off = (long long)t.N * t.N * t.N;
-    cudaError_t e = dir == 0 ? group_fft_launch(dir, t, T, d_grids, d_ws, sync_off, s)
-                             : group_dwt_launch(dir, t, T, d_ws, d_coefs, s);
+    cudaError_t e = dir == 0 ? group_fft_launch(dir, t, T, d_grids, d_ws, s) : group_dwt_launch(dir, t, T, d_ws, d_coefs, s);
     if (e == cudaSuccess)
-        e = dir == 0 ? group_dwt_launch(dir, t, T, d_ws, d_coefs, s) : group_fft_launch(dir, t, T, d_grids, d_ws, sync_off, s);
+        e = dir == 0 ? group_dwt_launch(dir, t, T, d_ws, d_coefs, s) : group_fft_launch(dir, t, T, d_grids, d_ws, s);
     if (e != cudaSuccess) return fail(PFSOFT_ECUDA, std::string("group launch: ") + cudaGetErrorString(e));
     return PFSOFT_OK;
 }
@@ -199,8 +192,7 @@ int enqueue(pfsoft_batch* b, int dir, cudaStream_t s)
     typedef pfsoft_batch::Group Group;
     auto T = [](const Group& g) { return (int)g.members.size(); };
     auto fft = [&](const Group& g) {
-        const long long sync_off = (long long)g.N * g.N * g.N + (g.split ? (long long)dwt_split_aux_elems(g.B) : 0);
-        return group_fft_launch(dir, g.tables, T(g), b->grid_ptrs() + g.ptr_base, b->ws_ptrs() + g.ptr_base, sync_off, s);
+        return group_fft_launch(dir, g.tables, T(g), b->grid_ptrs() + g.ptr_base, b->ws_ptrs() + g.ptr_base, s);
     };
     cudaError_t e = cudaSuccess;
     if (dir == 0)
@@ -323,16 +315,6 @@ int pfsoft_batch_create(const int* bandwidths, int count, int transforms_per_cta
         for (size_t i = 0; i < g.members.size(); ++i)
             b->h_ptr[2 * (size_t)count + g.ptr_base + i] =
                 reinterpret_cast<double2*>(static_cast<char*>(b->ws) + ws_off[g.members[i]]);
-    // the fused FFT counters start cleared (a group whose FFT runs as two passes never writes them)
-    for (const auto& g : b->groups) {
-        const size_t sync = ((size_t)g.N * g.N * g.N + (g.split ? dwt_split_aux_elems(g.B) : 0)) * sizeof(double2);
-        for (size_t i = 0; i < g.members.size() && e == cudaSuccess; ++i)
-            e = cudaMemset(static_cast<char*>(b->ws) + ws_off[g.members[i]] + sync, 0, kFftSyncBytes);
-    }
-    if (e != cudaSuccess) {
-        free_batch(b);
-        return fail(PFSOFT_ECUDA, std::string("batch setup: ") + cudaGetErrorString(e));
-    }
     // group descriptors of the split-precision DWT (pointer tables inside the device array)
     std::vector<DwtGroup> dg;
     for (const auto& g : b->groups) {
@@ -405,16 +387,6 @@ int pfsoft_batch_status(pfsoft_batch* b)
     if (e == cudaSuccess) e = cudaMemcpy(st, b->d_split, sizeof(st), cudaMemcpyDeviceToHost);
     if (e != cudaSuccess) return fail(PFSOFT_ECUDA, std::string("batch status: ") + cudaGetErrorString(e));
     if (st[1]) return fail(PFSOFT_ETIMEOUT, "a bounded wait in the split-precision DWT ran out");
-    // the fused FFT launches' status word (counters past the first transform's spectrum of each
-    // group, cleared by every launch): a bounded wait of the last execution ran out
-    for (const auto& g : b->groups) {
-        const char* ws = reinterpret_cast<const char*>(b->h_ptr[2 * (size_t)b->count + g.ptr_base]);
-        const size_t off = ((size_t)g.N * g.N * g.N + (g.split ? dwt_split_aux_elems(g.B) : 0)) * sizeof(double2);
-        int word = 0;
-        e = cudaMemcpy(&word, ws + off + sizeof(int), sizeof(int), cudaMemcpyDeviceToHost);
-        if (e != cudaSuccess) return fail(PFSOFT_ECUDA, std::string("batch status: ") + cudaGetErrorString(e));
-        if (word) return fail(PFSOFT_ETIMEOUT, "a bounded wait in the fused FFT launch ran out");
-    }
     return PFSOFT_OK;
 }
 

@@ -15,7 +15,7 @@ struct BandTables {
     double* sinh = nullptr;     // sin(beta_k / 2)                [N]
     double* cosh = nullptr;     // cos(beta_k / 2)                [N]
     double* w = nullptr;        // quadrature weights w_B(k)      [N]   (fn_dwt.hpp:62-83)
-    double2* twiddle = nullptr; // exp(-2 pi i t / N)             [N]
+    double2* twiddle = nullptr; // exp(-2 pi i t / N) and the FFT's second copy (fft_twiddle_elems)
     double2* ht = nullptr;      // {cos, sin}(pi n / (2N))        [B]
     // the Wigner rows at beta = pi/2, ((2l+1)/2)^(1/4) P[l][n][M] (-1)^(n-M) for n > M, tiles of 8 degrees x 8 n per
     // order M (delta_offset); zero for l < M, n > l and l >= B          [delta_entries(B)]

@@ -24,14 +24,12 @@ struct FftPassArgs {
     int ns[kFftMaxStages];       // product of the radices of the earlier stages
     FftStrides src, dst;
     double scale;                // applied to the stored values (1 = none)
-    const double2* twiddle;      // twiddle[t] = exp(-2*pi*i*t/n), t < n
+    // twiddle[t] = exp(-2*pi*i*t/n), t < n; behind them, for two-stage plans, exp(-2*pi*i*r*j/n) at
+    // n + (r - 1) ra + j, 1 <= r < rb, j < ra (fft_twiddle_elems entries in all)
+    const double2* twiddle;
     // batched passes: when set, transform z = blockIdx.z reads srcs[z] and writes dsts[z]
     const double2* const* srcs;
     double2* const* dsts;
-    int coherent;                // first-stage loads through the coherent path (0: read-only path)
-    // last-stage stores marked evict-first (st.global.cs): set by fft_pass_launch, whose output is
-    // not read again before it has left L2; left 0 where another pass reads it through L2
-    int stream_out;
     // lengths that fft_needs_bluestein names: the chirp tables (fft_bluestein_fill); null keeps direct
     // O(R^2) stages for their prime factors
     const double2* bluestein;
@@ -44,6 +42,14 @@ size_t fft_bluestein_elems(int n);   // double2 entries of the table
 // The table, computed on the host in long double (layout: fft_chirp_kernel).
 void fft_bluestein_fill(int n, double2* out);
 
+// Lengths n = ra rb that the two-stage kernel takes (fft_two.cu), its tile vectors, and its launch.
+bool fft_two_radices(int n, int* ra, int* rb);
+int fft_two_vectors(int n);
+cudaError_t fft_two_launch(const double2* src, double2* dst, const FftPassArgs& a, int ntiles, int sign, cudaStream_t stream, int nz);
+
+// Entries of a length's twiddle table (FftPassArgs::twiddle).
+__host__ __device__ __forceinline__ size_t fft_twiddle_elems(int n) { return 2 * (size_t)n; }
+
 // Radix plan for length n; returns the number of stages (0 if n cannot be planned).
 int fft_plan_radices(int n, int* radix, int* ns);
 
@@ -54,27 +60,12 @@ cudaError_t fft_pass_launch(const double2* src, double2* dst, const FftPassArgs&
 
 size_t fft_pass_smem_bytes(const FftPassArgs& a);
 
-// Both passes of one direction in one persistent launch, chunk by chunk over the layers, so that
-// the second pass reads the first pass's output of a chunk from L2 (see fft.cu). p0 / p1: the
-// passes as fft_pass_launch takes them (same length, plan and tile vectors; ntiles0 / ntiles1
-// their tile counts), nz transforms (nz > 1: the pointer tables of both passes; nz == 1: the
-// pointers src0..dst1). Each transform's workspace -- the second pass's source, `ws` when nz == 1 --
-// holds kFftSyncBytes bytes of counters at double2 offset sync_off. Returns cudaErrorInvalidValue
-// when the passes cannot be fused (fft_fused_chunk == 0).
+// Bytes past a transform's spectrum that its workspace size has always included (they held the counters
+// of a launch of both passes at once).
 constexpr int kFftSyncBytes = 4096;
-int fft_fused_chunk(const FftPassArgs& p0, const FftPassArgs& p1);
-// Whether transforms of length n use the fused launch (default off; pfsoft_tune_fft_fused sets it
-// per length, or for every length with n <= 0).
-bool fft_fused_enabled(int n);
-void fft_set_fused(int n, int on);
-cudaError_t fft_fused_launch(int sign, const FftPassArgs& p0, const FftPassArgs& p1, int ntiles0, int ntiles1, int nz,
-                             const double2* src0, double2* dst0, const double2* src1, double2* dst1, double2* ws,
-                             long long sync_off, cudaStream_t stream);
 
-// Vectors per tile for length n: 8 (128 contiguous bytes on the transposed side) unless the
-// ping-pong buffers of 8 vectors would leave a single CTA per SM, then 4; plans of three or more
-// radix-8 stages (n = 512) run the in-place kernel with as many vectors as keep one butterfly
-// per thread (4).
+// Vectors per tile for length n: 8 (128 contiguous bytes on the transposed side), or 4 where the buffers
+// of 8 vectors would leave a single CTA per SM, or the radices few.
 int fft_tile_vectors(int n);
 
 }  // namespace pfsoft_dev

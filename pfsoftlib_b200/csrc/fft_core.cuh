@@ -1,9 +1,10 @@
-// Device building blocks of the DFT kernels: register butterflies (radix 2, 3, 4, 5, 8, 16), the
+// Device building blocks of the DFT kernels: register butterflies (radix 2 .. 16 and products up to 32), the
 // twiddle table access, and the padded shared-memory position of an element. Shared by the grid's FFT
 // passes (fft.cu) and the beta transforms of the discrete Wigner transform (dwt.cu).
 #pragma once
 
 #include "common.cuh"
+#include "fft_roots.cuh"
 
 namespace pfsoft_dev {
 namespace fftk {
@@ -127,16 +128,83 @@ __device__ __forceinline__ int spos(int i) { return i + (i >> 4); }
 
 __host__ __device__ __forceinline__ int padded_len(int n) { return n + (n >> 4) + 1; }
 
+template <int SIGN, int R>
+__device__ __forceinline__ void butterfly(double2* v);
+
+// An odd prime R: the inputs k and R - k enter by their sum and difference.
+template <int SIGN, int R>
+__device__ __forceinline__ void dft_prime(double2* v)
+{
+    constexpr int h = (R - 1) / 2;
+    double2 t[h], d[h];
+#pragma unroll
+    for (int k = 1; k <= h; ++k) {
+        t[k - 1] = cadd(v[k], v[R - k]);
+        d[k - 1] = csub(v[k], v[R - k]);
+    }
+    double2 sum = v[0];
+#pragma unroll
+    for (int q = 1; q <= h; ++q) {
+        double2 a = v[0], b = make_double2(0.0, 0.0);
+#pragma unroll
+        for (int k = 1; k <= h; ++k) {
+            const double c = root<R>(k * q % R).x, s = root<R>(k * q % R).y;
+            a = make_double2(fma(c, t[k - 1].x, a.x), fma(c, t[k - 1].y, a.y));
+            b = k == 1 ? cscale(d[0], s) : make_double2(fma(s, d[k - 1].x, b.x), fma(s, d[k - 1].y, b.y));
+        }
+        b = cmul_i<SIGN>(b);
+        v[q] = cadd(a, b);
+        v[R - q] = csub(a, b);
+        sum = cadd(sum, t[q - 1]);
+    }
+    v[0] = sum;
+}
+
+// R = P Q: P-point DFTs of every Q-th input, the roots between, Q-point DFTs.
+template <int SIGN, int P, int Q>
+__device__ __forceinline__ void dft_product(double2* v)
+{
+    constexpr int R = P * Q;
+    double2 u[Q][P];
+#pragma unroll
+    for (int j = 0; j < Q; ++j) {
+#pragma unroll
+        for (int i = 0; i < P; ++i) u[j][i] = v[i * Q + j];
+        butterfly<SIGN, P>(u[j]);
+    }
+#pragma unroll
+    for (int i = 0; i < P; ++i) {
+        double2 w[Q];
+#pragma unroll
+        for (int j = 0; j < Q; ++j) {
+            const int e = i * j % R;
+            w[j] = e == 0 ? u[j][i] : cmul(u[j][i], make_double2(root<R>(e).x, SIGN * root<R>(e).y));
+        }
+        butterfly<SIGN, Q>(w);
+#pragma unroll
+        for (int j = 0; j < Q; ++j) v[i + P * j] = w[j];
+    }
+}
+
 // Radix-R butterfly in registers (R = 1: a copy).
 template <int SIGN, int R>
 __device__ __forceinline__ void butterfly(double2* v)
 {
-    if (R == 2) dft2<SIGN>(v);
-    else if (R == 3) dft3<SIGN>(v);
-    else if (R == 4) dft4<SIGN>(v[0], v[1], v[2], v[3]);
-    else if (R == 5) dft5<SIGN>(v);
-    else if (R == 8) dft8<SIGN>(v);
-    else if (R == 16) dft16<SIGN>(v);
+    if constexpr (R == 2) dft2<SIGN>(v);
+    else if constexpr (R == 3) dft3<SIGN>(v);
+    else if constexpr (R == 4) dft4<SIGN>(v[0], v[1], v[2], v[3]);
+    else if constexpr (R == 5) dft5<SIGN>(v);
+    else if constexpr (R == 8) dft8<SIGN>(v);
+    else if constexpr (R == 16) dft16<SIGN>(v);
+    else if constexpr (R == 7 || R == 11 || R == 13) dft_prime<SIGN, R>(v);
+    else if constexpr (R == 32) dft_product<SIGN, 4, 8>(v);
+    else if constexpr (R == 24) dft_product<SIGN, 3, 8>(v);
+    else if constexpr (R == 25) dft_product<SIGN, 5, 5>(v);
+    else if constexpr (R == 30) dft_product<SIGN, 5, 6>(v);
+    else if constexpr (R % 4 == 0) dft_product<SIGN, R / 4, 4>(v);       // 12, 20, 28
+    else if constexpr (R % 3 == 0) dft_product<SIGN, R / 3, 3>(v);       // 6, 9, 15, 18, 21
+    else if constexpr (R % 2 == 0) dft_product<SIGN, R / 2, 2>(v);       // 10, 14, 22, 26
+    else static_assert(R == 1, "no butterfly for this radix");
 }
 
 }  // namespace fftk

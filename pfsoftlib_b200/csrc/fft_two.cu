@@ -1,0 +1,186 @@
+// DFT passes of lengths n = ra rb with ra, rb <= 32, each factor one register butterfly: one exchange
+// through shared memory between the load from HBM and the store to HBM (sm_100a).
+//
+// Stage 1 takes butterfly j < rb of a vector, inputs x[j + r rb], r < ra, and leaves its outputs as row j
+// (pitch ra | 1) of the vector's block in shared memory. Stage 2 takes column j < ra, inputs
+// row r times w_n^(r j), and stores outputs j + q ra. With two stages no index needs a division, the
+// twiddles of a stage-2 load lie side by side (a.twiddle + n, fft_two_twiddle), and the rows' and
+// vectors' odd pitches keep both thread maps (along the vector, or across the tile's vectors: the side
+// that is contiguous in HBM) clear of bank conflicts.
+//
+// What bounds it: HBM. Against the ping-pong and in-place kernels of three or four stages that ran these
+// lengths before, us per pass (of the 32 N^3 bytes at the measured copy rate): N = 112 17 against
+// 31 .. 62, 200 66 against 108 (0.60), 256 90 against 98 (0.92), 320 199 against about 290 (0.82), 384 345
+// against 553 (0.82), 400 390 against 760 (0.81), 512 885 against 1210 (0.75).
+//
+// Tiles of 8 vectors move 128-byte runs on the transposed side; at radices 18 .. 26 four vectors and four
+// CTAs per SM measured faster (N = 320 199 us against 230), at 28 .. 32 eight (N = 512 885 against 1000).
+
+#include <algorithm>
+#include <type_traits>
+
+#include "common.cuh"
+#include "fft.cuh"
+#include "fft_core.cuh"
+
+namespace pfsoft_dev {
+
+namespace {
+
+using namespace fftk;
+
+// Vectors of a tile are this far apart in shared memory: 8 vectors (or 4 vectors x 2 butterflies) of one
+// access meet distinct 16-byte banks.
+__host__ __device__ __forceinline__ int block_pitch(int ra, int rb, int kb)
+{
+    const int len = rb * (ra | 1);
+    return kb == 8 ? (len | 1) : len + (10 - len % 8) % 8;
+}
+
+// butterfly t of a stage with m butterflies per vector: its vector and index
+__device__ __forceinline__ void place(bool across, int t, int lg, int m, unsigned inv, int& kk, int& j)
+{
+    if (across) {
+        kk = t & ((1 << lg) - 1);
+        j = t >> lg;
+    } else {
+        kk = m == 1 ? t : (int)__umulhi((unsigned)t, inv);   // t / m
+        j = t - kk * m;
+    }
+}
+
+template <int SIGN, int R>
+__device__ __forceinline__ void stage_one(const FftPassArgs& a, const double2* src, double2* smem, int nv, int lg, int vp)
+{
+    const int m = a.n / R, pitch = R | 1;
+    const bool across = a.src.se != 1;
+    const unsigned inv = 0xffffffffu / (unsigned)m + 1u;
+    for (int t = threadIdx.x; t < m << lg; t += blockDim.x) {
+        int kk, j;
+        place(across, t, lg, m, inv, kk, j);
+        if (kk >= nv) continue;
+        const double2* p = src + (long long)kk * a.src.sv + (long long)j * a.src.se;
+        const long long step = (long long)m * a.src.se;
+        double2 v[R];
+#pragma unroll
+        for (int r = 0; r < R; ++r) v[r] = __ldg(p + r * step);
+        butterfly<SIGN, R>(v);
+        double2* o = smem + kk * vp + j * pitch;
+#pragma unroll
+        for (int q = 0; q < R; ++q) o[q] = v[q];
+    }
+}
+
+template <int SIGN, int R>
+__device__ __forceinline__ void stage_two(const FftPassArgs& a, double2* dst, const double2* smem, int nv, int lg, int vp)
+{
+    const int m = a.n / R, pitch = m | 1;
+    const bool across = a.dst.se != 1;
+    const unsigned inv = 0xffffffffu / (unsigned)m + 1u;
+    const double2* tw = a.twiddle + a.n;
+    for (int t = threadIdx.x; t < m << lg; t += blockDim.x) {
+        int kk, j;
+        place(across, t, lg, m, inv, kk, j);
+        if (kk >= nv) continue;
+        const double2* o = smem + kk * vp + j;
+        double2 v[R];
+        v[0] = o[0];
+#pragma unroll
+        for (int r = 1; r < R; ++r) {
+            double2 w = __ldg(tw + (r - 1) * m + j);
+            if (SIGN > 0) w.y = -w.y;
+            v[r] = cmul(o[r * pitch], w);
+        }
+        butterfly<SIGN, R>(v);
+        double2* p = dst + (long long)kk * a.dst.sv + (long long)j * a.dst.se;
+        const long long step = (long long)m * a.dst.se;
+#pragma unroll
+        for (int q = 0; q < R; ++q) __stcs(p + q * step, cscale(v[q], a.scale));   // evict-first: next read from HBM
+    }
+}
+
+// Radices of the kernels: kernel 0 up to 16, kernel 1 up to 26, kernel 2 up to 32, so that no length pays
+// the registers of a radix that it does not need.
+constexpr int kMaxRadix[3] = {16, 26, 32};
+constexpr int kMinRadix[3] = {2, 7, 14};
+constexpr bool has_radix(int r)
+{
+    return (r >= 2 && r <= 16) || r == 18 || r == 20 || r == 21 || r == 22 || r == 24 || r == 25 || r == 26 || r == 28 || r == 30 ||
+           r == 32;
+}
+
+// f.template run<R>() for the kernel's radix R == r
+template <int KIND, int R, class Fn>
+__device__ __forceinline__ void with_radix(int r, const Fn& f)
+{
+    if constexpr (R <= kMaxRadix[KIND]) {
+        if constexpr (has_radix(R)) {
+            if (r == R) {
+                f(std::integral_constant<int, R>());
+                return;
+            }
+        }
+        with_radix<KIND, R + 1>(r, f);
+    }
+}
+
+template <int SIGN, int KIND>
+__global__ void __launch_bounds__(128, KIND == 2 ? 2 : 4)
+    fft_two_kernel(const double2* src, double2* dst, const __grid_constant__ FftPassArgs a)
+{
+    extern __shared__ double2 smem[];
+    if (a.srcs) {
+        src = a.srcs[blockIdx.z];
+        dst = a.dsts[blockIdx.z];
+    }
+    const int v0 = blockIdx.x * a.kb;
+    const int nv = min(a.kb, a.nvec - v0), lg = a.kb == 8 ? 3 : 2;
+    const int vp = block_pitch(a.radix[0], a.radix[1], a.kb);
+    src += (long long)v0 * a.src.sv + (long long)blockIdx.y * a.src.sb;
+    dst += (long long)v0 * a.dst.sv + (long long)blockIdx.y * a.dst.sb;
+    with_radix<KIND, kMinRadix[KIND]>(a.radix[0], [&](auto R) { stage_one<SIGN, decltype(R)::value>(a, src, smem, nv, lg, vp); });
+    __syncthreads();   // in place: every input of the tile has been read
+    with_radix<KIND, kMinRadix[KIND]>(a.radix[1], [&](auto R) { stage_two<SIGN, decltype(R)::value>(a, dst, smem, nv, lg, vp); });
+}
+
+}  // namespace
+
+bool fft_two_radices(int n, int* ra, int* rb)
+{
+    // the pair with the smallest larger factor, the larger one last
+    for (int hi = 4; hi <= 32; ++hi)
+        if (has_radix(hi) && n % hi == 0 && n / hi <= hi && n / hi >= 2 && has_radix(n / hi)) {
+            *ra = n / hi;
+            *rb = hi;
+            const int kind = hi <= kMaxRadix[0] ? 0 : (hi <= kMaxRadix[1] ? 1 : 2);
+            return *ra >= kMinRadix[kind];
+        }
+    return false;
+}
+
+int fft_two_vectors(int n)
+{
+    int ra, rb;
+    return fft_two_radices(n, &ra, &rb) && rb > kMaxRadix[0] && rb <= kMaxRadix[1] ? 4 : 8;
+}
+
+cudaError_t fft_two_launch(const double2* src, double2* dst, const FftPassArgs& a, int ntiles, int sign, cudaStream_t stream, int nz)
+{
+    const int ra = a.radix[0], rb = a.radix[1];
+    const int kind = rb <= kMaxRadix[0] ? 0 : (rb <= kMaxRadix[1] ? 1 : 2);
+    const size_t smem = (size_t)a.kb * block_pitch(ra, rb, a.kb) * sizeof(double2);
+    const int threads = std::min(128, (a.kb * rb + 31) / 32 * 32);
+    auto go = [&](auto k) -> cudaError_t {
+        if (smem > 48 * 1024) {
+            const cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+            if (e != cudaSuccess) return e;
+        }
+        k<<<dim3((a.nvec + a.kb - 1) / a.kb, ntiles, nz), threads, smem, stream>>>(src, dst, a);
+        return cudaGetLastError();
+    };
+    if (kind == 0) return sign < 0 ? go(fft_two_kernel<-1, 0>) : go(fft_two_kernel<1, 0>);
+    if (kind == 1) return sign < 0 ? go(fft_two_kernel<-1, 1>) : go(fft_two_kernel<1, 1>);
+    return sign < 0 ? go(fft_two_kernel<-1, 2>) : go(fft_two_kernel<1, 2>);
+}
+
+}  // namespace pfsoft_dev

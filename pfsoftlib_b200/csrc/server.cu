@@ -42,7 +42,7 @@ namespace pfsoft_dev {
 int tables_for(int B, cudaStream_t s, BandTables* out, bool split = false);   // api.cu
 int launch_group(int dir, const BandTables& t, int T, double2** d_grids, double2** d_coefs, double2** d_ws,
                  cudaStream_t s);   // batch.cu
-FftPassArgs group_pass_args(int dir, bool first, const BandTables& t, double2** grids, double2** ws);   // batch.cu
+cudaError_t group_fft_launch(int dir, const BandTables& t, int T, double2** grids, double2** ws, cudaStream_t s);   // batch.cu
 cudaError_t zero_nyquist_launch(double2** ws, int B, int T, cudaStream_t s);   // batch.cu
 }  // namespace pfsoft_dev
 
@@ -203,17 +203,7 @@ int launch_split_batch(pfsoft_server* s, Batch* b, const std::vector<Request>& i
     for (int i = 0; i < k && e == cudaSuccess; ++i)
         if (io[i].ready) e = cudaStreamWaitEvent(sl.stream, io[i].ready, 0);
     if (e == cudaSuccess) e = cudaMemcpyAsync(sl.d_stage, sl.h_stage, s->stage_bytes, cudaMemcpyHostToDevice, sl.stream);
-    const int sign = dir == 0 ? -1 : +1;
-    auto fft = [&](size_t g) -> cudaError_t {
-        const FftPassArgs a = group_pass_args(dir, true, tabs[g], d_tab + gbase[g], d_tab + 2 * cap + gbase[g]);
-        const FftPassArgs c = group_pass_args(dir, false, tabs[g], d_tab + gbase[g], d_tab + 2 * cap + gbase[g]);
-        const int N = tabs[g].N;
-        if (fft_fused_enabled(N) && fft_fused_chunk(a, c))
-            return fft_fused_launch(sign, a, c, N, N, gT[g], nullptr, nullptr, nullptr, nullptr, nullptr,
-                                    (long long)N * N * N + (long long)dwt_split_aux_elems(gB[g]), sl.stream);
-        cudaError_t e2 = fft_pass_launch(nullptr, nullptr, a, N, sign, sl.stream, gT[g]);
-        return e2 == cudaSuccess ? fft_pass_launch(nullptr, nullptr, c, N, sign, sl.stream, gT[g]) : e2;
-    };
+    auto fft = [&](size_t g) { return group_fft_launch(dir, tabs[g], gT[g], d_tab + gbase[g], d_tab + 2 * cap + gbase[g], sl.stream); };
     for (size_t g = 0; g < tabs.size() && e == cudaSuccess; ++g) {
         double2** ws = d_tab + 2 * cap + gbase[g];
         double2** cf = d_tab + cap + gbase[g];
@@ -477,7 +467,6 @@ int pfsoft_server_submit(pfsoft_server* s, int direction, int B, const double* d
     if (!d_in || !d_out) return fail(PFSOFT_EINVAL, "null buffer");
     if ((reinterpret_cast<uintptr_t>(d_in) & 15) || (reinterpret_cast<uintptr_t>(d_out) & 15))
         return fail(PFSOFT_EINVAL, "buffers must be 16-byte aligned");
-    // pfsoft_workspace_bytes includes the FFT counters; in split mode they follow the scale table
     const size_t bytes = pfsoft_workspace_bytes(B) + (s->split ? dwt_split_aux_elems(B) * sizeof(double2) : 0);
     {
         std::lock_guard<std::mutex> lk(s->mu);

@@ -19,6 +19,7 @@
 #include "common.cuh"
 #include "dwt.cuh"
 #include "dwt_common.cuh"
+#include "fft.cuh"
 
 namespace pfsoft_dev {
 
@@ -63,7 +64,7 @@ __global__ void powers_kernel(int B, const double* sinh, const double* cosh, dou
 }
 
 __global__ void tables_kernel(int B, double* cosb, double* sinh, double* cosh, double* w,
-                              double2* tw, double2* ht)
+                              double2* tw, double2* ht, int ra)
 {
     const int N = 2 * B;
     const int tid = blockIdx.x * blockDim.x + threadIdx.x;
@@ -79,6 +80,11 @@ __global__ void tables_kernel(int B, double* cosb, double* sinh, double* cosh, d
         double ts, tc;
         sincospi(2.0 * (double)k / (double)N, &ts, &tc);
         tw[k] = make_double2(tc, -ts);
+        // the two-stage kernel's copy: exp(-2 pi i (r j mod N) / N), r = k / ra + 1, j = k mod ra
+        if (ra) {
+            sincospi(2.0 * (double)((k / ra + 1) * (k % ra) % N) / (double)N, &ts, &tc);
+            tw[N + k] = make_double2(tc, -ts);
+        }
         if (k < B) {
             sincospi((double)k / (double)(2 * N), &ts, &tc);
             ht[k] = make_double2(tc, ts);
@@ -232,7 +238,7 @@ __global__ void delta_kernel(int B, double* delta)
 size_t tables_bytes(int B)
 {
     const size_t N = 2 * (size_t)B;
-    return 4 * align256(N * sizeof(double)) + align256(N * sizeof(double2)) +
+    return 4 * align256(N * sizeof(double)) + align256(fft_twiddle_elems((int)N) * sizeof(double2)) +
            align256(B * sizeof(double2)) + align256((size_t)delta_entries(B) * sizeof(double)) +
            align256((size_t)trig_entries(B) * sizeof(double));
 }
@@ -254,14 +260,16 @@ cudaError_t tables_build(int B, void* mem, BandTables* t, cudaStream_t stream)
     t->sinh = reinterpret_cast<double*>(take(N * sizeof(double)));
     t->cosh = reinterpret_cast<double*>(take(N * sizeof(double)));
     t->w = reinterpret_cast<double*>(take(N * sizeof(double)));
-    t->twiddle = reinterpret_cast<double2*>(take(N * sizeof(double2)));
+    t->twiddle = reinterpret_cast<double2*>(take(fft_twiddle_elems((int)N) * sizeof(double2)));
     t->ht = reinterpret_cast<double2*>(take(B * sizeof(double2)));
     const size_t dbytes = (size_t)delta_entries(B) * sizeof(double);
     t->delta = reinterpret_cast<double*>(take(dbytes));
     t->trig = reinterpret_cast<double*>(take((size_t)trig_entries(B) * sizeof(double)));
     const int threads = 64;
+    int ra = 0, rb = 0;
+    if (!fft_two_radices((int)N, &ra, &rb)) ra = 0;
     tables_kernel<<<((int)N + threads - 1) / threads, threads, 0, stream>>>(B, t->cosb, t->sinh, t->cosh, t->w,
-                                                                             t->twiddle, t->ht);
+                                                                             t->twiddle, t->ht, ra);
     cudaError_t e = cudaGetLastError();
     if (e == cudaSuccess) e = cudaMemsetAsync(t->delta, 0, dbytes, stream);
     if (e != cudaSuccess) return e;
