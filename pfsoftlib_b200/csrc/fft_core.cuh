@@ -1,4 +1,4 @@
-// Device building blocks of the DFT kernels: register butterflies (radix 2 .. 16 and products up to 32), the
+// Device building blocks of the DFT kernels: register butterflies (radix 2 .. 32), the
 // twiddle table access, and the padded shared-memory position of an element. Shared by the grid's FFT
 // passes (fft.cu) and the beta transforms of the discrete Wigner transform (dwt.cu).
 #pragma once
@@ -196,7 +196,7 @@ __device__ __forceinline__ void butterfly(double2* v)
     else if constexpr (R == 5) dft5<SIGN>(v);
     else if constexpr (R == 8) dft8<SIGN>(v);
     else if constexpr (R == 16) dft16<SIGN>(v);
-    else if constexpr (R == 7 || R == 11 || R == 13) dft_prime<SIGN, R>(v);
+    else if constexpr (R == 7 || R == 11 || R == 13 || R == 17 || R == 19 || R == 23 || R == 29 || R == 31) dft_prime<SIGN, R>(v);
     else if constexpr (R == 32) dft_product<SIGN, 4, 8>(v);
     else if constexpr (R == 24) dft_product<SIGN, 3, 8>(v);
     else if constexpr (R == 25) dft_product<SIGN, 5, 5>(v);

@@ -11,7 +11,9 @@
 // What bounds it: HBM. Against the ping-pong and in-place kernels of three or four stages that ran these
 // lengths before, us per pass (of the 32 N^3 bytes at the measured copy rate): N = 112 17 against
 // 31 .. 62, 200 66 against 108 (0.60), 256 90 against 98 (0.92), 320 199 against about 290 (0.82), 384 345
-// against 553 (0.82), 400 390 against 760 (0.81), 512 885 against 1210 (0.75).
+// against 553 (0.82), 400 390 against 760 (0.81), 512 885 against 1210 (0.75). The primes 17 .. 31 cost R
+// multiply-adds per point, under the 90 that fit the HBM time; against the chirp pass, us per pass: N =
+// 136 32 / 64, 184 81 / 145, 248 179 / 292, 272 131 / 449, 304 183 / 571, 408 426 / 1480, 496 970 / 2274.
 //
 // Tiles of 8 vectors move 128-byte runs on the transposed side; at radices 18 .. 26 four vectors and four
 // CTAs per SM measured faster (N = 320 199 us against 230), at 28 .. 32 eight (N = 512 885 against 1000).
@@ -99,14 +101,22 @@ __device__ __forceinline__ void stage_two(const FftPassArgs& a, double2* dst, co
     }
 }
 
-// Radices of the kernels: kernel 0 up to 16, kernel 1 up to 26, kernel 2 up to 32, so that no length pays
-// the registers of a radix that it does not need.
-constexpr int kMaxRadix[3] = {16, 26, 32};
-constexpr int kMinRadix[3] = {2, 7, 14};
-constexpr bool has_radix(int r)
+// The kernels: 0 for radices up to 16, 1 up to 26, 2 up to 32, 3 and 4 the same with the primes from 17
+// on (23 only in 4: its sums would spill in 3), so that no length pays the registers or the code of a
+// radix that it does not need (N = 512 with the primes in kernel 2: 913 us per pass, without 885).
+constexpr int kKinds = 5;
+constexpr int kMaxRadix[kKinds] = {16, 26, 32, 26, 32};
+constexpr bool is_prime17(int r) { return r == 17 || r == 19 || r == 23 || r == 29 || r == 31; }
+constexpr bool has_radix(int kind, int r)
 {
-    return (r >= 2 && r <= 16) || r == 18 || r == 20 || r == 21 || r == 22 || r == 24 || r == 25 || r == 26 || r == 28 || r == 30 ||
-           r == 32;
+    return r >= (kind == 1 ? 7 : (kind == 2 ? 14 : 2)) && r <= kMaxRadix[kind] && r != 27 && (kind >= 3 || !is_prime17(r)) &&
+           (kind != 3 || r != 23);
+}
+constexpr int kind_of(int ra, int rb)
+{
+    for (int kind = 0; kind < kKinds; ++kind)
+        if (has_radix(kind, ra) && has_radix(kind, rb)) return kind;
+    return -1;
 }
 
 // f.template run<R>() for the kernel's radix R == r
@@ -114,7 +124,7 @@ template <int KIND, int R, class Fn>
 __device__ __forceinline__ void with_radix(int r, const Fn& f)
 {
     if constexpr (R <= kMaxRadix[KIND]) {
-        if constexpr (has_radix(R)) {
+        if constexpr (has_radix(KIND, R)) {
             if (r == R) {
                 f(std::integral_constant<int, R>());
                 return;
@@ -125,7 +135,7 @@ __device__ __forceinline__ void with_radix(int r, const Fn& f)
 }
 
 template <int SIGN, int KIND>
-__global__ void __launch_bounds__(128, KIND == 2 ? 2 : 4)
+__global__ void __launch_bounds__(128, KIND == 2 || KIND == 4 ? 2 : 4)
     fft_two_kernel(const double2* src, double2* dst, const __grid_constant__ FftPassArgs a)
 {
     extern __shared__ double2 smem[];
@@ -138,9 +148,9 @@ __global__ void __launch_bounds__(128, KIND == 2 ? 2 : 4)
     const int vp = block_pitch(a.radix[0], a.radix[1], a.kb);
     src += (long long)v0 * a.src.sv + (long long)blockIdx.y * a.src.sb;
     dst += (long long)v0 * a.dst.sv + (long long)blockIdx.y * a.dst.sb;
-    with_radix<KIND, kMinRadix[KIND]>(a.radix[0], [&](auto R) { stage_one<SIGN, decltype(R)::value>(a, src, smem, nv, lg, vp); });
+    with_radix<KIND, 2>(a.radix[0], [&](auto R) { stage_one<SIGN, decltype(R)::value>(a, src, smem, nv, lg, vp); });
     __syncthreads();   // in place: every input of the tile has been read
-    with_radix<KIND, kMinRadix[KIND]>(a.radix[1], [&](auto R) { stage_two<SIGN, decltype(R)::value>(a, dst, smem, nv, lg, vp); });
+    with_radix<KIND, 2>(a.radix[1], [&](auto R) { stage_two<SIGN, decltype(R)::value>(a, dst, smem, nv, lg, vp); });
 }
 
 }  // namespace
@@ -148,26 +158,29 @@ __global__ void __launch_bounds__(128, KIND == 2 ? 2 : 4)
 bool fft_two_radices(int n, int* ra, int* rb)
 {
     // the pair with the smallest larger factor, the larger one last
-    for (int hi = 4; hi <= 32; ++hi)
-        if (has_radix(hi) && n % hi == 0 && n / hi <= hi && n / hi >= 2 && has_radix(n / hi)) {
-            *ra = n / hi;
-            *rb = hi;
-            const int kind = hi <= kMaxRadix[0] ? 0 : (hi <= kMaxRadix[1] ? 1 : 2);
-            return *ra >= kMinRadix[kind];
-        }
+    for (int hi = 4; hi <= 32; ++hi) {
+        const int lo = n / hi;
+        if (n % hi || lo > hi || lo < 2) continue;
+        const int kind = kind_of(lo, hi);
+        // 2 x 17 .. 2 x 31 fill too few threads (n = 58, us per pass: 19, the chirp pass 13)
+        if (kind < 0 || (kind >= 3 && (lo < 3 || !(is_prime17(lo) || is_prime17(hi))))) continue;
+        *ra = lo;
+        *rb = hi;
+        return true;
+    }
     return false;
 }
 
 int fft_two_vectors(int n)
 {
     int ra, rb;
-    return fft_two_radices(n, &ra, &rb) && rb > kMaxRadix[0] && rb <= kMaxRadix[1] ? 4 : 8;
+    return fft_two_radices(n, &ra, &rb) && kind_of(ra, rb) % 2 ? 4 : 8;
 }
 
 cudaError_t fft_two_launch(const double2* src, double2* dst, const FftPassArgs& a, int ntiles, int sign, cudaStream_t stream, int nz)
 {
     const int ra = a.radix[0], rb = a.radix[1];
-    const int kind = rb <= kMaxRadix[0] ? 0 : (rb <= kMaxRadix[1] ? 1 : 2);
+    const int kind = kind_of(ra, rb);
     const size_t smem = (size_t)a.kb * block_pitch(ra, rb, a.kb) * sizeof(double2);
     const int threads = std::min(128, (a.kb * rb + 31) / 32 * 32);
     auto go = [&](auto k) -> cudaError_t {
@@ -178,9 +191,14 @@ cudaError_t fft_two_launch(const double2* src, double2* dst, const FftPassArgs& 
         k<<<dim3((a.nvec + a.kb - 1) / a.kb, ntiles, nz), threads, smem, stream>>>(src, dst, a);
         return cudaGetLastError();
     };
-    if (kind == 0) return sign < 0 ? go(fft_two_kernel<-1, 0>) : go(fft_two_kernel<1, 0>);
-    if (kind == 1) return sign < 0 ? go(fft_two_kernel<-1, 1>) : go(fft_two_kernel<1, 1>);
-    return sign < 0 ? go(fft_two_kernel<-1, 2>) : go(fft_two_kernel<1, 2>);
+    switch (kind) {
+        case 0: return sign < 0 ? go(fft_two_kernel<-1, 0>) : go(fft_two_kernel<1, 0>);
+        case 1: return sign < 0 ? go(fft_two_kernel<-1, 1>) : go(fft_two_kernel<1, 1>);
+        case 2: return sign < 0 ? go(fft_two_kernel<-1, 2>) : go(fft_two_kernel<1, 2>);
+        case 3: return sign < 0 ? go(fft_two_kernel<-1, 3>) : go(fft_two_kernel<1, 3>);
+        case 4: return sign < 0 ? go(fft_two_kernel<-1, 4>) : go(fft_two_kernel<1, 4>);
+        default: return cudaErrorInvalidValue;
+    }
 }
 
 }  // namespace pfsoft_dev

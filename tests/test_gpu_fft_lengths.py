@@ -40,3 +40,10 @@ def test_every_short_length(lib):
     for n in range(1, 300):
         _check(n, 5, 3, n)
         _check(9, n, 2, n)
+
+
+@pytest.mark.parametrize("n", [323, 361, 408, 456, 460, 496, 506, 529, 551, 713, 899, 961, 992])
+def test_prime_radices_17_to_31(lib, n):
+    _check(n, 3, 5, n)
+    _check(3, n, 19, n)
+    _check(19, n, 2, n)
