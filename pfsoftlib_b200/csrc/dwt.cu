@@ -23,17 +23,21 @@
 // multiply-adds for each; the series has l + 1 coefficients per degree, B^4/8 over all classes, each
 // one product of two table values, and the beta sums add either a DFT or a matrix product per column.
 // Against the recurrence kernels that this replaces (us per launch on B200, forward / inverse):
-// B = 64 29 / 29 (31 / 46), 100 103 / 111 (131 / 138), 128 180 / 177 (263 / 265), 137 457 / 450
-// (610 / 605), 200 895 / 936 (1810 / 1793), 251 3182 / 3085 (3911 / 3705), 256 1879 / 1932
+// B = 64 29 / 29 (31 / 46), 100 98 / 103 (131 / 138), 128 180 / 177 (263 / 265), 137 457 / 450
+// (610 / 605), 200 888 / 904 (1810 / 1793), 251 3182 / 3085 (3911 / 3705), 256 1879 / 1932
 // (4092 / 3903); the error against 64 bits falls four- to twelvefold (B = 256 DSOFT 1.4e-14 to 1.1e-15).
 //
 // What bounds it at B = 128: the shared-memory pipe (65 % of its cycles) and latency at 16 warps per
 // SM; the MMA takes 34 of the 180 us, the other FP64 work 30.
 //
-// The beta sums: a compile-time DFT for the lengths in dispatch(), else the MMA form. The DFT costs
-// N log N per column but passes the columns through shared memory three times between barriers; the
-// matrix product costs B^2 per column and has one barrier. Measured: N = 96 the MMA form 17 / 18 us
-// against 18 / 18, N = 128 33 / 33 against 29 / 29, N = 256 259 / 248 against 180 / 177.
+// The beta sums: a DFT of compile-time radices (fixed_plan) where N = 98 .. 512 is a product of two or
+// three of at most 20, else the MMA form. The DFT costs N log N per column but passes the columns
+// through shared memory once per stage between barriers; the matrix product costs B^2 per column and has
+// one barrier. Measured, MMA form against DFT, us forward / inverse: N = 96 17 / 18 against 19 / 19,
+// 98 25 / 26 against 20 / 22, 128 33 / 33 against 29 / 29, 168 70 / 77 against 60 / 64, 224 168 / 168
+// against 126 / 123, 272 428 / 434 against 309 / 300, 360 956 / 1007 against 699 / 664, 480 2699 / 2658
+// against 1602 / 1628; the radices 17 and 19 at N = 114 and 152 break even, 23 spills. Two large
+// radices beat three small ones (N = 240 16.15 152 / 152 against 16.3.5 160 / 168).
 //
 // One CTA per item, a class of one transform; longest classes first.
 
@@ -749,21 +753,63 @@ cudaError_t launch_mma(int dir, const double2* X, double2* coeffs, const DwtArgs
                     : launch(dwt_inverse_mma_kernel<NW, KP, MB>, (const double2*)coeffs, const_cast<double2*>(X), 32 * NW, smem, a, T, s);
 }
 
+// The radices of a DFT length N: of the products of two or three of at most 20, the first even, the one
+// whose stages hold the fewest points in the block's registers, a stage's last butterflies rounded up to
+// a whole one per thread, and a stage's two barriers counted as 4 points; r0 = 0 if there is none that
+// fits the registers (24 points).
+struct FixedPlan {
+    int r0, r1, r2;
+};
+
+constexpr FixedPlan fixed_plan(int N, int NT)
+{
+    FixedPlan best = {0, 0, 0};
+    int least = 0, widest = 0;
+    for (int r0 = 20; r0 >= 2; r0 -= 2)
+        for (int r1 = 20; r1 >= 2; --r1) {
+            if (N % (r0 * r1) || N / (r0 * r1) > 20) continue;
+            const int r[3] = {r0, r1, N / (r0 * r1)};
+            int sum = 0, wide = 0;
+            bool fits = true;
+            for (int i = 0; i < 3; ++i) {
+                const int points = r[i] > 1 ? (8 * (N / r[i]) + NT - 1) / NT * r[i] : 0;
+                sum += points + (points ? 4 : 0);
+                fits = fits && points <= 24;
+                wide = r[i] > wide ? r[i] : wide;
+            }
+            if (fits && (best.r0 == 0 || sum < least || (sum == least && wide < widest))) {
+                best = {r[0], r[1], r[2]};
+                least = sum;
+                widest = wide;
+            }
+        }
+    return best;
+}
+
+typedef cudaError_t (*LaunchFn)(int, const double2*, double2*, const DwtArgs&, int, cudaStream_t);
+
+template <int N>
+constexpr LaunchFn fixed_launch()
+{
+    constexpr int NW = N <= 256 ? 4 : 8;
+    constexpr FixedPlan p = fixed_plan(N, 32 * NW);
+    if constexpr (p.r0 > 0) return launch_fft<FixedFft<N, NW, p.r0, p.r1, p.r2>, ((N + 15) / 16 + NW - 1) / NW>;
+    else return nullptr;
+}
+
+constexpr int kFixedFirst = 98, kFixedLast = 512;
+
+template <int... I>
+LaunchFn fixed_launch_of(int N, std::integer_sequence<int, I...>)
+{
+    static constexpr LaunchFn table[] = {fixed_launch<kFixedFirst + 2 * I>()...};
+    return N < kFixedFirst || N > kFixedLast ? nullptr : table[(N - kFixedFirst) / 2];
+}
+
 cudaError_t dispatch(int dir, const double2* X, double2* coeffs, const DwtArgs& a, int T, cudaStream_t s)
 {
-    switch (a.N) {
-        case 128: return launch_fft<FixedFft<128, 4, 16, 8, 1>, 2>(dir, X, coeffs, a, T, s);
-        case 160: return launch_fft<FixedFft<160, 4, 8, 4, 5>, 3>(dir, X, coeffs, a, T, s);
-        case 192: return launch_fft<FixedFft<192, 4, 8, 8, 3>, 3>(dir, X, coeffs, a, T, s);
-        case 200: return launch_fft<FixedFft<200, 4, 8, 5, 5>, 4>(dir, X, coeffs, a, T, s);
-        case 240: return launch_fft<FixedFft<240, 4, 16, 3, 5>, 4>(dir, X, coeffs, a, T, s);
-        case 256: return launch_fft<FixedFft<256, 4, 16, 16, 1>, 4>(dir, X, coeffs, a, T, s);
-        case 320: return launch_fft<FixedFft<320, 8, 8, 8, 5>, 3>(dir, X, coeffs, a, T, s);
-        case 384: return launch_fft<FixedFft<384, 8, 16, 8, 3>, 3>(dir, X, coeffs, a, T, s);
-        case 400: return launch_fft<FixedFft<400, 8, 16, 5, 5>, 4>(dir, X, coeffs, a, T, s);
-        case 512: return launch_fft<FixedFft<512, 8, 8, 8, 8>, 4>(dir, X, coeffs, a, T, s);
-        default: break;
-    }
+    const LaunchFn fixed = fixed_launch_of(a.N, std::make_integer_sequence<int, (kFixedLast - kFixedFirst) / 2 + 1>());
+    if (fixed) return fixed(dir, X, coeffs, a, T, s);
     if (a.B <= 16) return launch_mma<2, 1, 12>(dir, X, coeffs, a, T, s);
     if (a.B <= 32) return launch_mma<2, 2, 12>(dir, X, coeffs, a, T, s);
     if (a.B <= 40) return launch_mma<4, 2, 5>(dir, X, coeffs, a, T, s);

@@ -49,3 +49,9 @@ def test_dwt_matches_oracle_classes(lib, oracle, B):
     ref = oracle.dwt_inverse(c, B, cls, np.full(N ** 3, np.nan + 0j))
     at = ~np.isnan(ref)
     assert orc.rel_l2(x.cpu().numpy()[at], ref[at]) <= REL_TOL
+
+
+@pytest.mark.parametrize("B", [48, 49, 51, 57, 66, 75, 84, 104, 119, 121, 125, 130, 133, 143, 147, 169, 187, 196, 209, 225, 245, 255])
+def test_dwt_dft_lengths(lib, oracle, B):
+    """Compile-time DFT lengths of two and three radices, odd ones and the primes 7 .. 19 among them."""
+    test_dwt_matches_oracle_classes(lib, oracle, B)
