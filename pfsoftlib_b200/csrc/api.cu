@@ -362,7 +362,7 @@ int get_tables(int B, cudaStream_t stream, BandTables* out, bool split = false)
         int rc = build(tables_bytes(B), [&](void* mem) { return tables_build(B, mem, &t, stream); });
         if (rc) return rc;
         if (fft_needs_bluestein(2 * B)) {
-            // the FFT's chirp table, computed on the host
+            // the table of the FFT's matrix or chirp pass, computed on the host
             std::vector<double2> h(fft_bluestein_elems(2 * B));
             fft_bluestein_fill(2 * B, h.data());
             void* bt = nullptr;

@@ -24,7 +24,7 @@ struct BandTables {
     // [cos, sin][q][m / 8][k / 8], row-major, zero past either end            [trig_entries(B)]
     double* trig = nullptr;
     void* block = nullptr;      // single allocation holding all of the above
-    double2* bluestein = nullptr;   // fft_needs_bluestein(N): the FFT's chirp table (own allocation)
+    double2* bluestein = nullptr;   // fft_needs_bluestein(N): the FFT pass's table (own allocation)
     // only for the split-precision DWT (split_tables_build; null until a caller asks for them)
     double* normf = nullptr;    // seed norm per order class      [B(B+1)/2] (fn_dwt.hpp:117-121)
     double2* pw_sin = nullptr;  // sin(beta_k/2)^p as {mantissa, exponent}  [2B][N], p < 2B

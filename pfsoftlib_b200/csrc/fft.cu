@@ -1,8 +1,9 @@
 // Batched 1D DFT passes over the (alpha, gamma) plane of every beta layer (sm_100a): the choice of a
-// pass's kernel, and two of the three.
+// pass's kernel, and two of the four.
 //
 //   fft_two.cu         n = ra rb with register butterflies up to 32: one shared-memory exchange
-//   fft_chirp_kernel   n with a large prime factor: Bluestein's convolution
+//   fft_matrix.cu      n = R p, p odd and 17 .. 249: a matrix product on the FP64 MMA
+//   fft_chirp_kernel   n with a larger prime, or one with too many other factors: Bluestein's convolution
 //   fft_pass_kernel    what is left (n below 4, 5, 7, 11 and 13, lengths such as 343, n above 1024):
 //                      mixed-radix Stockham autosort (Govindaraju et al., SC'08 formulation). A stage of
 //     radix R over n points with Ns = product of the earlier radices maps butterfly j to
@@ -181,17 +182,15 @@ __global__ void __launch_bounds__(256, 2) fft_pass_kernel(const double2* src, do
 // that order, and decimation in time back. The first stage reads HBM into registers (its upper half
 // of inputs is zero), the last forward stage, the product and the first backward stage work on one
 // thread's registers, and the last stage stores to HBM (its upper half of outputs is not needed), so
-// that a sequence crosses shared memory four times (two radices: twice). A backward DFT is the
-// forward one of the conjugate.
+// that a sequence crosses shared memory four times. A backward DFT is the forward one of the conjugate.
 // What bounds it: FP64 arithmetic and the shared-memory pipe, about 4 M (M/m) log2 M multiply-adds a
-// value. Measured on B200 per pass, against radix-4
-// stages in shared memory at M >= 2n - 1: n = 74 19 us (47), 202 207 us (673), 274 463 us (2592),
-// 502 2.58 ms (9.15 ms).
+// value. Measured on B200 at n = 502, per pass: 2.37 ms, radix-4 stages in shared memory at M >= 2n - 1
+// 9.15 ms, the matrix pass 2.41 ms: the larger primes stay here.
 template <int R0_, int R1_, int R2_, int V_>
 struct ChirpPlan {
-    static constexpr int R0 = R0_, R1 = R1_, R2 = R2_, V = V_;   // V vectors per CTA; R2 = 1: two radices
+    static constexpr int R0 = R0_, R1 = R1_, R2 = R2_, V = V_;   // V vectors per CTA
     static constexpr int M = R0 * R1 * R2, h0 = M / R0, h1 = h0 / R1;
-    static constexpr int RL = R2 > 1 ? R2 : R1;                  // the last radix, on contiguous elements
+    static constexpr int RL = R2;                                // the last radix, on contiguous elements
     // one pad slot per RL elements when RL is even: the threads' runs then start in distinct banks
     static constexpr int kPad = RL == 16 ? 4 : (RL == 8 ? 3 : (RL == 4 ? 2 : 31));
     static __device__ __forceinline__ int pos(int i) { return kPad < 31 ? i + (i >> (kPad & 15)) : i; }
@@ -279,20 +278,18 @@ __global__ void __launch_bounds__(256, P::kMinBlocks)
         }
     }
     __syncthreads();
-    if constexpr (R2 > 1) {
-        for (int t = threadIdx.x; t < S * (M / R1); t += 256) {
-            const int i = t % h1, blk = t / h1 % R0, sq = t / (M / R1);
-            double2* o = smem + sq * PM;
-            double2 u[R1];
+    for (int t = threadIdx.x; t < S * (M / R1); t += 256) {
+        const int i = t % h1, blk = t / h1 % R0, sq = t / (M / R1);
+        double2* o = smem + sq * PM;
+        double2 u[R1];
 #pragma unroll
-            for (int q = 0; q < R1; ++q) u[q] = o[P::pos(blk * h0 + i + q * h1)];
-            butterfly<-1, R1>(u);
-            o[P::pos(blk * h0 + i)] = u[0];
+        for (int q = 0; q < R1; ++q) u[q] = o[P::pos(blk * h0 + i + q * h1)];
+        butterfly<-1, R1>(u);
+        o[P::pos(blk * h0 + i)] = u[0];
 #pragma unroll
-            for (int q = 1; q < R1; ++q) o[P::pos(blk * h0 + i + q * h1)] = cmul(u[q], __ldg(tw2 + (q - 1) * h1 + i));
-        }
-        __syncthreads();
+        for (int q = 1; q < R1; ++q) o[P::pos(blk * h0 + i + q * h1)] = cmul(u[q], __ldg(tw2 + (q - 1) * h1 + i));
     }
+    __syncthreads();
     for (int t = threadIdx.x; t < S * (M / RL); t += 256) {
         const int e = t % (M / RL) * RL;
         double2* o = smem + t / (M / RL) * PM;
@@ -307,24 +304,22 @@ __global__ void __launch_bounds__(256, P::kMinBlocks)
         for (int q = 0; q < RL; ++q) o[P::pos(e + q)] = u[q];
     }
     __syncthreads();
-    if constexpr (R2 > 1) {
-        for (int t = threadIdx.x; t < S * (M / R1); t += 256) {
-            const int i = t % h1, blk = t / h1 % R0, sq = t / (M / R1);
-            double2* o = smem + sq * PM;
-            double2 u[R1];
-            u[0] = o[P::pos(blk * h0 + i)];
+    for (int t = threadIdx.x; t < S * (M / R1); t += 256) {
+        const int i = t % h1, blk = t / h1 % R0, sq = t / (M / R1);
+        double2* o = smem + sq * PM;
+        double2 u[R1];
+        u[0] = o[P::pos(blk * h0 + i)];
 #pragma unroll
-            for (int q = 1; q < R1; ++q) {
-                double2 w = __ldg(tw2 + (q - 1) * h1 + i);
-                w.y = -w.y;
-                u[q] = cmul(o[P::pos(blk * h0 + i + q * h1)], w);
-            }
-            butterfly<+1, R1>(u);
-#pragma unroll
-            for (int q = 0; q < R1; ++q) o[P::pos(blk * h0 + i + q * h1)] = u[q];
+        for (int q = 1; q < R1; ++q) {
+            double2 w = __ldg(tw2 + (q - 1) * h1 + i);
+            w.y = -w.y;
+            u[q] = cmul(o[P::pos(blk * h0 + i + q * h1)], w);
         }
-        __syncthreads();
+        butterfly<+1, R1>(u);
+#pragma unroll
+        for (int q = 0; q < R1; ++q) o[P::pos(blk * h0 + i + q * h1)] = u[q];
     }
+    __syncthreads();
     for (int t = threadIdx.x; t < V * h0; t += 256) {
         const int v = vfast_out ? t % V : t / h0, i = vfast_out ? t / V : t % h0;
         if (v >= nv) continue;
@@ -379,14 +374,6 @@ constexpr ChirpEntry chirp_entry()
 }
 
 const ChirpEntry kChirps[] = {
-    chirp_entry<8, 8, 1, 16>(),   // 64
-    chirp_entry<8, 4, 3, 16>(),   // 96
-    chirp_entry<8, 16, 1, 8>(),   // 128
-    chirp_entry<8, 4, 5, 8>(),    // 160
-    chirp_entry<8, 8, 3, 8>(),    // 192
-    chirp_entry<8, 8, 4, 8>(),    // 256
-    chirp_entry<8, 8, 5, 4>(),    // 320
-    chirp_entry<8, 16, 3, 4>(),   // 384
     chirp_entry<8, 8, 8, 4>(),    // 512
     chirp_entry<8, 16, 5, 4>(),   // 640
     chirp_entry<8, 8, 16, 2>(),   // 1024
@@ -401,10 +388,9 @@ const ChirpEntry& chirp_for(int n)
     return kChirps[sizeof(kChirps) / sizeof(kChirps[0]) - 1];
 }
 
-// The largest prime factor that does not go to the chirp pass. Even lengths, whose tables are kept: 5,
-// as measured against direct stages of 7, 11 and 13, us per pass: N = 28 10 / 11, 112 43 / 62, 154
-// 82 / 224, 224 250 / 297, 308 597 / 2014, 448 1975 / 2387. Odd lengths, whose table is made on the
-// host for each call: 16.
+// The largest prime factor that does not go to the chirp pass, for what the other kernels leave: even
+// lengths (tables kept) such as 686, direct stages of 7, 11 and 13 measured slower at every length
+// from 28 to 448 (N = 308 597 us against 2014); odd ones (table made on the host for each call) such as 343.
 int largest_direct_radix(int n) { return n % 2 ? 16 : 5; }
 
 // Whether passes of length n run the two-stage kernel.
@@ -412,6 +398,24 @@ bool two_stage(int n)
 {
     int ra, rb;
     return fft_two_radices(n, &ra, &rb);
+}
+
+int largest_prime(int n)
+{
+    int big = 1;
+    for (int p = 2; p * p <= n; ++p)
+        while (n % p == 0) {
+            big = p;
+            n /= p;
+        }
+    return std::max(big, n);
+}
+
+// The odd factor p of a length n = R p that passes on the matrix kernel, or 0.
+int matrix_factor(int n)
+{
+    int r, p;
+    return !two_stage(n) && largest_prime(n) > largest_direct_radix(n) && fft_matrix_radices(n, &r, &p) ? p : 0;
 }
 
 }  // namespace
@@ -466,26 +470,21 @@ int fft_plan_radices(int n, int* radix, int* ns)
 
 bool fft_needs_bluestein(int n)
 {
-    if (n < 2 || (n % 2 ? n : n / 2) > 512 || two_stage(n)) return false;
-    int rem = n, big = 1;
-    for (int p = 2; p * p <= rem; ++p)
-        while (rem % p == 0) {
-            big = p;
-            rem /= p;
-        }
-    if (rem > 1) big = rem > big ? rem : big;
-    return big > largest_direct_radix(n);
+    if (matrix_factor(n)) return true;
+    return n >= 2 && (n % 2 ? n : n / 2) <= 512 && !two_stage(n) && largest_prime(n) > largest_direct_radix(n);
 }
 
 size_t fft_bluestein_elems(int n)
 {
+    if (const int p = matrix_factor(n)) return fft_matrix_elems(p);
     const ChirpEntry& c = chirp_for(n);
     const int M = c.r0 * c.r1 * c.r2, m = n % 2 ? n : n / 2, h0 = M / c.r0;
-    return 2 * (size_t)m + M + (size_t)(c.r0 - 1) * h0 + (c.r2 > 1 ? (size_t)(c.r1 - 1) * (h0 / c.r1) : 0);
+    return 2 * (size_t)m + M + (size_t)(c.r0 - 1) * h0 + (size_t)(c.r1 - 1) * (h0 / c.r1);
 }
 
 void fft_bluestein_fill(int n, double2* out)
 {
+    if (const int p = matrix_factor(n)) return fft_matrix_fill(p, out);
     typedef long double ld;
     const ld pi = 3.14159265358979323846264338327950288L;
     const ChirpEntry& c = chirp_for(n);
@@ -530,14 +529,14 @@ void fft_bluestein_fill(int n, double2* out)
     double2* tw = fh + M;
     for (int q = 1; q < c.r0; ++q)
         for (int i = 0; i < h0; ++i) *tw++ = make_double2((double)cr[q * i % M], (double)ci[q * i % M]);
-    if (c.r2 > 1)
-        for (int q = 1; q < c.r1; ++q)
-            for (int i = 0; i < h1; ++i) *tw++ = make_double2((double)cr[c.r0 * q * i % M], (double)ci[c.r0 * q * i % M]);
+    for (int q = 1; q < c.r1; ++q)
+        for (int i = 0; i < h1; ++i) *tw++ = make_double2((double)cr[c.r0 * q * i % M], (double)ci[c.r0 * q * i % M]);
 }
 
 int fft_tile_vectors(int n)
 {
     if (two_stage(n)) return fft_two_vectors(n);
+    if (matrix_factor(n)) return 8;
     const size_t two_buffers = 2 * (size_t)8 * padded_len(n) * sizeof(double2);
     return two_buffers > (size_t)110 * 1024 ? 4 : 8;
 }
@@ -552,6 +551,7 @@ cudaError_t fft_pass_launch(const double2* src, double2* dst, const FftPassArgs&
                             cudaStream_t stream, int nz)
 {
     if (a.bluestein && fft_needs_bluestein(a.n)) {
+        if (matrix_factor(a.n)) return fft_matrix_launch(src, dst, a, ntiles, sign, stream, nz);
         return chirp_for(a.n).launch(src, dst, a, ntiles, sign, stream, nz);
     }
     if (two_stage(a.n)) return fft_two_launch(src, dst, a, ntiles, sign, stream, nz);

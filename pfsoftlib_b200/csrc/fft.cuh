@@ -30,22 +30,31 @@ struct FftPassArgs {
     // batched passes: when set, transform z = blockIdx.z reads srcs[z] and writes dsts[z]
     const double2* const* srcs;
     double2* const* dsts;
-    // lengths that fft_needs_bluestein names: the chirp tables (fft_bluestein_fill); null keeps direct
-    // O(R^2) stages for their prime factors
+    // lengths that fft_needs_bluestein names: the table of the matrix or the chirp kernel
+    // (fft_bluestein_fill); null keeps direct O(R^2) stages for their prime factors
     const double2* bluestein;
 };
 
-// Bluestein's algorithm (fft_chirp_kernel) for a length n whose largest prime factor is too large for a
-// direct stage: n <= 512, or even and <= 1024.
+// Lengths with a prime factor too large for a direct stage whose passes need a table: the matrix kernel's
+// (fft_matrix.cu), or the chirps of Bluestein's algorithm (fft_chirp_kernel) for n <= 512, or even and
+// <= 1024.
 bool fft_needs_bluestein(int n);
 size_t fft_bluestein_elems(int n);   // double2 entries of the table
-// The table, computed on the host in long double (layout: fft_chirp_kernel).
+// The table, computed on the host in long double (layout: fft_matrix_fill, fft_chirp_kernel).
 void fft_bluestein_fill(int n, double2* out);
 
 // Lengths n = ra rb that the two-stage kernel takes (fft_two.cu), its tile vectors, and its launch.
 bool fft_two_radices(int n, int* ra, int* rb);
 int fft_two_vectors(int n);
 cudaError_t fft_two_launch(const double2* src, double2* dst, const FftPassArgs& a, int ntiles, int sign, cudaStream_t stream, int nz);
+
+// Lengths n = r p that the matrix kernel takes (fft_matrix.cu), its table for p (double2 entries, contents)
+// and its launch.
+bool fft_matrix_radices(int n, int* r, int* p);
+size_t fft_matrix_elems(int p);
+void fft_matrix_fill(int p, double2* out);
+cudaError_t fft_matrix_launch(const double2* src, double2* dst, const FftPassArgs& a, int ntiles, int sign, cudaStream_t stream,
+                              int nz);
 
 // Entries of a length's twiddle table (FftPassArgs::twiddle).
 __host__ __device__ __forceinline__ size_t fft_twiddle_elems(int n) { return 2 * (size_t)n; }

@@ -47,3 +47,11 @@ def test_prime_radices_17_to_31(lib, n):
     _check(n, 3, 5, n)
     _check(3, n, 19, n)
     _check(19, n, 2, n)
+
+
+@pytest.mark.parametrize("n", [38, 46, 86, 106, 111, 129, 185, 222, 259, 289, 333, 407, 444, 490, 505, 514, 578, 654, 1028])
+def test_matrix_lengths(lib, n):
+    """n = R p: the first and last p, every parity of the tiles of four and eight, R = 1 .. 12."""
+    _check(n, 3, 5, n)
+    _check(3, n, 19, n)
+    _check(19, n, 2, n)
