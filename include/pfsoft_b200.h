@@ -89,8 +89,9 @@ int pfsoft_cuda_dsoft_noalloc(const double* d_grid, int B, double* d_coeffs, voi
  * transform (pfsoft_batch_workspace_bytes). Pointer tables are host arrays of `count` device
  * pointers in the caller's order; every buffer has the single-transform layouts above. Stream
  * ordered. Calls on one plan are serialised by the plan.
- * PFSOFT_BATCH_SPLIT runs the DWT of the bandwidths that pfsoft_split_supported() accepts
- * (1 <= B <= 256) on the tensor cores instead, all of them in one launch per direction: the FP64
+ * PFSOFT_BATCH_SPLIT lets the plan run the DWT of the bandwidths that pfsoft_split_supported()
+ * accepts (1 <= B <= 256) on the tensor cores instead, where that is the faster form or
+ * pfsoft_tune_split_bandwidth asks for it, all of them in one launch per direction: the FP64
  * Wigner rows and FP64 data are cut into six signed 8-bit digit planes, multiplied exactly
  * (8-bit x 8-bit products summed in 32-bit integers) and combined in FP64; relative L2 error
  * about 1e-13 against the FP64 path. Two transforms of one bandwidth share each generated Wigner
@@ -281,8 +282,9 @@ int pfsoft_tune_dwt_case_split(int direction, int case_split);
  * every bandwidth). The bandwidth is checked; the passes always run as two launches. */
 int pfsoft_tune_fft_fused(int B, int on);
 /* Tuning knob: whether a plan created with PFSOFT_BATCH_SPLIT runs bandwidth B's DWT on the split
- * kernel (use_split != 0, the default) or on the FP64 kernels (0). B <= 0: every bandwidth,
- * clearing the per-bandwidth choices. Set by the autotuner; read when a plan is created. */
+ * kernel (use_split != 0) or on the FP64 kernels (0). B <= 0: every bandwidth, clearing the
+ * per-bandwidth choices; use_split != 0 then is the default, the faster form for each bandwidth and
+ * number of transforms. Set by the autotuner; read when a plan is created. */
 int pfsoft_tune_split_bandwidth(int B, int use_split);
 /* Test knob for the split-precision DWT's failure path (no counterpart in the reference): when
  * wait_ns > 0, every later split launch first waits up to wait_ns nanoseconds on a barrier that

@@ -7,9 +7,9 @@
 
 A plan groups its transforms by bandwidth, runs the FFT passes and one DWT launch over every (order
 class, transform) per bandwidth, and replays the whole sequence from a CUDA graph. Create it once per bandwidth mix (it builds tables, work lists
-and the graph) and reuse it with any buffers. ``split=True`` runs the DWT of bandwidths 16..128
-(multiples of 16) on the tensor cores in split precision (relative error about 1e-13 against the
-FP64 path). Calls are ordered on torch's current stream unless ``stream`` is given.
+and the graph) and reuse it with any buffers. ``split=True`` lets it run the DWT of
+bandwidths up to 256 on the tensor cores in split precision (relative error about 1e-13 against the
+FP64 path) where that is faster. Calls are ordered on torch's current stream unless ``stream`` is given.
 """
 from __future__ import annotations
 

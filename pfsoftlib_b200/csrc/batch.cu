@@ -32,15 +32,24 @@ int tables_for(int B, cudaStream_t s, BandTables* out, bool split = false);   //
 
 namespace {
 
-// Autotuner's split-precision choice per bandwidth (0 default = split where supported, 1 split,
-// -1 FP64), read when a PFSOFT_BATCH_SPLIT plan is created.
+// The split-precision choice per bandwidth (0 default, 1 split, -1 FP64) and of the rest (default or
+// FP64), read when a PFSOFT_BATCH_SPLIT plan is created.
 signed char g_split_choice[513] = {};
 bool g_split_all = true;
 
-bool split_wanted(int B)
+// Default: the faster DWT for T transforms of bandwidth B. The FP64 kernels' sums over the series take
+// fewer steps than the split kernel's digit products; only without a DFT over beta, whose matrix product
+// grows as B^4, and with pairs of transforms to share the split kernel's Wigner tiles, the split kernel
+// is ahead from about B = 140 on. Whole plans, split over FP64, iDSOFT / DSOFT: B = 32 (T = 4) 2.0 / 2.5, 64 1.4 /
+// 1.6, 128 1.3 / 1.3, 256 1.1 / 1.2; without DFT and T >= 2: 116 1.1, 137 1.0, 166 0.98, 184 0.94, 251
+// 0.92, T = 1: 1.1 and more. Up to B = 16, where calls of a few transforms are bound by their launches, the split kernel
+// stays although FP64 is 5 to 15 us ahead: it is the one whose failure is reported by pfsoft_batch_status.
+bool split_faster(int B, int T) { return B <= 16 || (B >= 140 && T >= 2 && !dwt_has_dft(2 * B)); }
+
+bool split_wanted(int B, int T)
 {
     if (B >= 1 && B <= 512 && g_split_choice[B]) return g_split_choice[B] > 0;
-    return g_split_all;
+    return g_split_all && split_faster(B, T);
 }
 
 __global__ void zero_nyquist_batched(double2* const* X, int B)
@@ -262,7 +271,7 @@ int pfsoft_batch_create(const int* bandwidths, int count, int transforms_per_cta
         g.members = kv.second;
         g.ptr_base = base;
         base += g.members.size();
-        g.split = (flags & PFSOFT_BATCH_SPLIT) && dwt_split_supported(g.B) && split_wanted(g.B);
+        g.split = (flags & PFSOFT_BATCH_SPLIT) && dwt_split_supported(g.B) && split_wanted(g.B, (int)g.members.size());
         for (int t : g.members) {
             ws_off[t] = ws_total;
             ws_total += ((((size_t)g.N * g.N * g.N + (g.split ? dwt_split_aux_elems(g.B) : 0)) * sizeof(double2) + kFftSyncBytes

@@ -806,10 +806,14 @@ LaunchFn fixed_launch_of(int N, std::integer_sequence<int, I...>)
     return N < kFixedFirst || N > kFixedLast ? nullptr : table[(N - kFixedFirst) / 2];
 }
 
+LaunchFn fixed_launch_for(int N)
+{
+    return fixed_launch_of(N, std::make_integer_sequence<int, (kFixedLast - kFixedFirst) / 2 + 1>());
+}
+
 cudaError_t dispatch(int dir, const double2* X, double2* coeffs, const DwtArgs& a, int T, cudaStream_t s)
 {
-    const LaunchFn fixed = fixed_launch_of(a.N, std::make_integer_sequence<int, (kFixedLast - kFixedFirst) / 2 + 1>());
-    if (fixed) return fixed(dir, X, coeffs, a, T, s);
+    if (const LaunchFn fixed = fixed_launch_for(a.N)) return fixed(dir, X, coeffs, a, T, s);
     if (a.B <= 16) return launch_mma<2, 1, 12>(dir, X, coeffs, a, T, s);
     if (a.B <= 32) return launch_mma<2, 2, 12>(dir, X, coeffs, a, T, s);
     if (a.B <= 40) return launch_mma<4, 2, 5>(dir, X, coeffs, a, T, s);
@@ -836,6 +840,8 @@ DwtArgs dwt_args_for(const BandTables& t)
     a.trig = t.trig;
     return a;
 }
+
+bool dwt_has_dft(int N) { return fixed_launch_for(N) != nullptr; }
 
 cudaError_t dwt_forward_launch(const double2* X, double2* coeffs, const DwtArgs& a, int T, cudaStream_t s)
 {

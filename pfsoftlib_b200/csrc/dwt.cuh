@@ -91,6 +91,9 @@ DwtArgs dwt_args_for(const BandTables& t);
 
 // T transforms (T > 1: a.Xs and a.coefs; X and coeffs are then unused).
 // Forward: X (beta-innermost spectrum, N^3) -> packed coefficients, scale pi/(2B^2).
+// Whether the columns of length N have a compile-time DFT over beta (dwt.cu) instead of a matrix product.
+bool dwt_has_dft(int N);
+
 cudaError_t dwt_forward_launch(const double2* X, double2* coeffs, const DwtArgs& a, int T, cudaStream_t stream);
 // Inverse: packed coefficients -> X (all non-Nyquist beta columns), scale 2B^2/pi.
 cudaError_t dwt_inverse_launch(const double2* coeffs, double2* X, const DwtArgs& a, int T, cudaStream_t stream);

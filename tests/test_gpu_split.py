@@ -149,3 +149,27 @@ def test_mixed_plan_split_and_fp64(lib):
     for t, B in enumerate(bws):
         assert _rel(gsp[t], g64[t]) <= REL_TOL, f"B={B}"
         assert _rel(csp[t], c64[t]) <= REL_TOL, f"B={B}"
+
+
+@pytest.mark.parametrize("B,T", [(1, 1), (17, 2), (20, 3), (32, 6), (37, 3), (64, 4), (97, 2), (128, 2), (200, 1), (251, 2), (256, 2)])
+def test_split_form_by_default_and_by_choice(lib, B, T):
+    """The form that a split plan takes by default where FP64 is faster (bit for bit the FP64 plan's), where
+    it is not, and the split kernel wherever the tuning knob asks for it."""
+    import torch
+    bws = [B] * T
+    cs = _coeffs(lib, bws, seed0=7000 + B)
+    g64, c64 = _run(lib, bws, cs, 0)
+    by_default = B <= 16 or B == 251
+    try:
+        for on, split in ((None, by_default), (1, True), (0, False)):
+            if on is not None:
+                assert lib.pfsoft_tune_split_bandwidth(B, on) == 0
+            g, c = _run(lib, bws, cs, SPLIT)
+            for t in range(T):
+                assert _rel(g[t], g64[t]) <= REL_TOL and _rel(c[t], c64[t]) <= REL_TOL
+                if not split:
+                    assert torch.equal(g[t], g64[t]) and torch.equal(c[t], c64[t])
+            if split and B > 1:
+                assert not all(torch.equal(g[t], g64[t]) for t in range(T))
+    finally:
+        lib.pfsoft_tune_split_bandwidth(0, 1)
