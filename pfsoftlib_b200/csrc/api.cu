@@ -475,11 +475,14 @@ int run_dsoft(const double* d_grid, int B, double* d_coeffs, void* ws, cudaStrea
     // F2: vectors = layers k, tile = gamma bin r, elements = column c; in place on X
     FftPassArgs f2 = pass_args(N, N, t, FftStrides{1, n2, n}, FftStrides{1, n2, n}, 1.0);
     if (f1.nstages == 0) return fail(PFSOFT_EINVAL, "FFT length cannot be planned");
-    {
+    if (fft_plane_supported(N, 1)) {   // both passes
         StageScope sc(ST_FFT_FWD_ROWS, s);
-        PF_CUDA(fft_pass_launch(G, X, f1, N, -1, s));
-    }
-    {
+        PF_CUDA(fft_plane_launch(G, X, FftPlaneArgs{N, 0, 0, 1.0, t.twiddle, nullptr, nullptr}, -1, s, 1));
+    } else {
+        {
+            StageScope sc(ST_FFT_FWD_ROWS, s);
+            PF_CUDA(fft_pass_launch(G, X, f1, N, -1, s));
+        }
         StageScope sc(ST_FFT_FWD_COLS, s);
         PF_CUDA(fft_pass_launch(X, X, f2, N, -1, s));
     }
@@ -511,11 +514,14 @@ int run_idsoft(const double* d_coeffs, int B, double* d_grid, void* ws, cudaStre
     // I1: inverse DFT over gamma, X[r][c][k] -> G[k][c][r], scaled by 1/(4B^2) (src/fn_idsoft.cpp:289)
     FftPassArgs i1 = pass_args(N, N, t, FftStrides{1, n, n2}, FftStrides{n2, n, 1}, 1.0 / (4.0 * B * B));
     if (i1.nstages == 0) return fail(PFSOFT_EINVAL, "FFT length cannot be planned");
-    {
+    if (fft_plane_supported(N, 1)) {   // both passes
         StageScope sc(ST_FFT_INV_COLS, s);
-        PF_CUDA(fft_pass_launch(X, X, i2, N, +1, s));
-    }
-    {
+        PF_CUDA(fft_plane_launch(X, G, FftPlaneArgs{N, 0, 0, i1.scale, t.twiddle, nullptr, nullptr}, +1, s, 1));
+    } else {
+        {
+            StageScope sc(ST_FFT_INV_COLS, s);
+            PF_CUDA(fft_pass_launch(X, X, i2, N, +1, s));
+        }
         StageScope sc(ST_FFT_INV_ROWS, s);
         PF_CUDA(fft_pass_launch(X, G, i1, N, +1, s));
     }

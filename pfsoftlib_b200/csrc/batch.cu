@@ -142,6 +142,11 @@ cudaError_t group_dwt_launch(int dir, const BandTables& t, int T, double2** ws, 
 cudaError_t group_fft_launch(int dir, const BandTables& t, int T, double2** grids, double2** ws, cudaStream_t s)
 {
     const int sign = dir == 0 ? -1 : +1;
+    if (fft_plane_supported(t.N, T)) {
+        const double scale = dir == 0 ? 1.0 : 1.0 / (4.0 * t.B * t.B);
+        return fft_plane_launch(nullptr, nullptr, FftPlaneArgs{t.N, 0, 0, scale, t.twiddle, dir == 0 ? grids : ws, dir == 0 ? ws : grids},
+                                sign, s, T);
+    }
     cudaError_t e = fft_pass_launch(nullptr, nullptr, group_pass_args(dir, true, t, grids, ws), t.N, sign, s, T);
     return e == cudaSuccess ? fft_pass_launch(nullptr, nullptr, group_pass_args(dir, false, t, grids, ws), t.N, sign, s, T) : e;
 }

@@ -48,6 +48,18 @@ bool fft_two_radices(int n, int* ra, int* rb);
 int fft_two_vectors(int n);
 cudaError_t fft_two_launch(const double2* src, double2* dst, const FftPassArgs& a, int ntiles, int sign, cudaStream_t stream, int nz);
 
+// Both passes of a transform in one launch, for small even N = n (fft_two.cu): forward G[k][c][r] to X[r][c][k],
+// backward X to G scaled; for nz > 1 transforms the device tables srcs and dsts.
+struct FftPlaneArgs {
+    int n, ra, rb;
+    double scale;
+    const double2* twiddle;
+    const double2* const* srcs;
+    double2* const* dsts;
+};
+bool fft_plane_supported(int n, int nz);
+cudaError_t fft_plane_launch(const double2* src, double2* dst, const FftPlaneArgs& a, int sign, cudaStream_t stream, int nz);
+
 // Lengths n = r p that the matrix kernel takes (fft_matrix.cu), its table for p (double2 entries, contents)
 // and its launch.
 bool fft_matrix_radices(int n, int* r, int* p);
