@@ -339,9 +339,8 @@ size_t grid_elems(int B)
     return N * N * N;
 }
 
-// Tables for bandwidth B on the current device; built on first use (the split-precision DWT's own
-// ones when `split` is first asked for).
-int get_tables(int B, cudaStream_t stream, BandTables* out, bool split = false)
+// Tables for bandwidth B on the current device, each set built on first use.
+int get_tables(int B, cudaStream_t stream, BandTables* out, int sets = kSeriesTables)
 {
     int dev = 0;
     PF_CUDA(cudaGetDevice(&dev));
@@ -349,12 +348,13 @@ int get_tables(int B, cudaStream_t stream, BandTables* out, bool split = false)
     std::lock_guard<std::mutex> lk(st->mu);
     auto it = st->tables.find(B);
     const bool have = it != st->tables.end();
-    if (have && (!split || it->second.rc_cf)) {
-        *out = it->second;
-        return PFSOFT_OK;
-    }
     BandTables t;
     if (have) t = it->second;
+    const bool series = (sets & kSeriesTables) && !t.delta, split = (sets & kSplitTables) && !t.rc_cf;
+    if (have && !series && !split) {
+        *out = t;
+        return PFSOFT_OK;
+    }
     // one block: allocate, fill on the stream, wait
     auto build = [&](size_t bytes, auto fill) -> int {
         void* mem = nullptr;
@@ -390,6 +390,11 @@ int get_tables(int B, cudaStream_t stream, BandTables* out, bool split = false)
         }
         st->tables[B] = t;
     }
+    if (series) {
+        int rc = build(series_tables_bytes(B), [&](void* mem) { return series_tables_build(B, mem, &t, stream); });
+        if (rc) return rc;
+        st->tables[B] = t;
+    }
     if (split) {
         int rc = build(split_tables_bytes(B), [&](void* mem) { return split_tables_build(B, mem, &t, stream); });
         if (rc) return rc;
@@ -403,7 +408,6 @@ int get_tables(int B, cudaStream_t stream, BandTables* out, bool split = false)
 
 namespace pfsoft_dev {
 void set_last_error(const char* msg) { g_last_error = msg; }
-int tables_for(int B, cudaStream_t s, BandTables* out, bool split);
 }  // namespace pfsoft_dev
 
 namespace {
@@ -615,8 +619,7 @@ __global__ void wigner_matrix_kernel(int B, int M, int Mp, const double* w, cons
 }  // namespace
 
 namespace pfsoft_dev {
-// Cached tables of a bandwidth on the current device (used by the batch plans).
-int tables_for(int B, cudaStream_t s, BandTables* out, bool split) { return get_tables(B, s, out, split); }
+int tables_for(int B, cudaStream_t s, BandTables* out, int sets) { return get_tables(B, s, out, sets); }
 }  // namespace pfsoft_dev
 
 extern "C" {
@@ -729,7 +732,7 @@ static int layer_wise(int cols, int rows, int lays, double* d_arr, double scale,
         void* tmp_b = nullptr;
         if (n % 2 == 0 && valid_bandwidth(n / 2)) {
             BandTables t;
-            int rc = get_tables(n / 2, s, &t);
+            int rc = get_tables(n / 2, s, &t, 0);
             if (rc) return rc;
             tw = t.twiddle;
             blu = t.bluestein;

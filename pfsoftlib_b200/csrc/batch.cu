@@ -26,10 +26,6 @@
 
 using namespace pfsoft_dev;
 
-namespace pfsoft_dev {
-int tables_for(int B, cudaStream_t s, BandTables* out, bool split = false);   // api.cu: cached tables of a bandwidth
-}
-
 namespace {
 
 // The split-precision choice per bandwidth (0 default, 1 split, -1 FP64) and of the rest (default or
@@ -282,7 +278,7 @@ int pfsoft_batch_create(const int* bandwidths, int count, int transforms_per_cta
             ws_total += ((((size_t)g.N * g.N * g.N + (g.split ? dwt_split_aux_elems(g.B) : 0)) * sizeof(double2) + kFftSyncBytes
                           + 255) & ~(size_t)255);   // each workspace 256-byte aligned
         }
-        int rc = tables_for(g.B, nullptr, &g.tables, g.split);
+        int rc = tables_for(g.B, nullptr, &g.tables, kSeriesTables | (g.split ? kSplitTables : 0));
         if (rc) {
             free_batch(b);
             return rc;

@@ -17,14 +17,15 @@ struct BandTables {
     double* w = nullptr;        // quadrature weights w_B(k)      [N]   (fn_dwt.hpp:62-83)
     double2* twiddle = nullptr; // exp(-2 pi i t / N) and the FFT's second copy (fft_twiddle_elems)
     double2* ht = nullptr;      // {cos, sin}(pi n / (2N))        [B]
+    void* block = nullptr;      // single allocation holding all of the above
+    double2* bluestein = nullptr;   // fft_needs_bluestein(N): the FFT pass's table (own allocation)
+    // only for the FP64 DWT (series_tables_build; null until a caller asks for them)
     // the Wigner rows at beta = pi/2, ((2l+1)/2)^(1/4) P[l][n][M] (-1)^(n-M) for n > M, tiles of 8 degrees x 8 n per
     // order M (delta_offset); zero for l < M, n > l and l >= B          [delta_entries(B)]
     double* delta = nullptr;
     // (2 - [n = 0]) cos(n beta_k) and sin, n = 2 m + q < B, k < B, tiles of 8 m x 8 k in the order
     // [cos, sin][q][m / 8][k / 8], row-major, zero past either end            [trig_entries(B)]
     double* trig = nullptr;
-    void* block = nullptr;      // single allocation holding all of the above
-    double2* bluestein = nullptr;   // fft_needs_bluestein(N): the FFT pass's table (own allocation)
     // only for the split-precision DWT (split_tables_build; null until a caller asks for them)
     double* normf = nullptr;    // seed norm per order class      [B(B+1)/2] (fn_dwt.hpp:117-121)
     double2* pw_sin = nullptr;  // sin(beta_k/2)^p as {mantissa, exponent}  [2B][N], p < 2B
@@ -62,9 +63,16 @@ __host__ __device__ __forceinline__ long long trig_entries(int B)
 size_t tables_bytes(int B);
 // Carve the tables out of `mem` (tables_bytes(B) bytes, 256-byte aligned) and fill them.
 cudaError_t tables_build(int B, void* mem, BandTables* t, cudaStream_t stream);
-// The split-precision DWT's own tables, after tables_build, from another block.
+// The FP64 DWT's own tables, and the split-precision DWT's, after tables_build, each from another block.
+size_t series_tables_bytes(int B);
+cudaError_t series_tables_build(int B, void* mem, BandTables* t, cudaStream_t stream);
 size_t split_tables_bytes(int B);
 cudaError_t split_tables_build(int B, void* mem, BandTables* t, cudaStream_t stream);
+
+// The cached tables of a bandwidth on the current device (api.cu), with the DWTs' named by `sets` built on
+// first use: what a process keeps is what its calls need.
+constexpr int kSeriesTables = 1, kSplitTables = 2;
+int tables_for(int B, cudaStream_t s, BandTables* out, int sets = kSeriesTables);
 
 struct DwtArgs {
     int B, N;

@@ -89,8 +89,10 @@ int pfsoft_cuda_dsoft_noalloc(const double* d_grid, int B, double* d_coeffs, voi
     if (cap != cudaStreamCaptureStatusNone) d.captured = true;
     if (d.captured || d.tables_B != B) {
         // recorded into the captured work too, so that every replay builds the tables it reads
-        if (tables_bytes(B) > kTableBytes) return fail(PFSOFT_EINVAL, "pfsoft_cuda_dsoft_noalloc: tables exceed the reserve");
-        if (tables_build(B, d.base + kSpectrumBytes, &d.tables, s) != cudaSuccess) {
+        if (tables_bytes(B) + series_tables_bytes(B) > kTableBytes) return fail(PFSOFT_EINVAL, "pfsoft_cuda_dsoft_noalloc: tables exceed the reserve");
+        unsigned char* mem = d.base + kSpectrumBytes;
+        if (tables_build(B, mem, &d.tables, s) != cudaSuccess ||
+            series_tables_build(B, mem + tables_bytes(B), &d.tables, s) != cudaSuccess) {
             d.tables_B = 0;
             return fail(PFSOFT_ECUDA, "pfsoft_cuda_dsoft_noalloc: table kernels failed to launch");
         }

@@ -39,7 +39,6 @@
 using namespace pfsoft_dev;
 
 namespace pfsoft_dev {
-int tables_for(int B, cudaStream_t s, BandTables* out, bool split = false);   // api.cu
 int launch_group(int dir, const BandTables& t, int T, double2** d_grids, double2** d_coefs, double2** d_ws,
                  cudaStream_t s);   // batch.cu
 cudaError_t group_fft_launch(int dir, const BandTables& t, int T, double2** grids, double2** ws, cudaStream_t s);   // batch.cu
@@ -164,7 +163,7 @@ int launch_split_batch(pfsoft_server* s, Batch* b, const std::vector<Request>& i
     int pos = 0;
     for (const auto& kv : byB) {
         BandTables t;
-        const int rc = tables_for(kv.first, sl.stream, &t, true);
+        const int rc = tables_for(kv.first, sl.stream, &t, kSplitTables);
         if (rc) return rc;
         const int g = (int)tabs.size();
         for (size_t m = 0; m < kv.second.size(); ++m) {
@@ -481,7 +480,7 @@ int pfsoft_server_submit(pfsoft_server* s, int direction, int B, const double* d
     // latency, counted from the end of this call, does not include them
     {
         BandTables t;
-        const int rc = tables_for(B, s->table_stream, &t, s->split);
+        const int rc = tables_for(B, s->table_stream, &t, s->split ? kSplitTables : kSeriesTables);
         if (rc) return rc;
     }
     cudaEvent_t ready = nullptr;

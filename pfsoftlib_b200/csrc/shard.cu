@@ -31,10 +31,6 @@
 using namespace pfsoft_dev;
 using pfsoft_shard::Run;
 
-namespace pfsoft_dev {
-int tables_for(int B, cudaStream_t s, BandTables* out, bool split = false);   // api.cu: cached tables of a bandwidth
-}
-
 namespace {
 
 struct DstTable {

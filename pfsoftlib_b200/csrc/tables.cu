@@ -239,8 +239,7 @@ size_t tables_bytes(int B)
 {
     const size_t N = 2 * (size_t)B;
     return 4 * align256(N * sizeof(double)) + align256(fft_twiddle_elems((int)N) * sizeof(double2)) +
-           align256(B * sizeof(double2)) + align256((size_t)delta_entries(B) * sizeof(double)) +
-           align256((size_t)trig_entries(B) * sizeof(double));
+           align256(B * sizeof(double2));
 }
 
 cudaError_t tables_build(int B, void* mem, BandTables* t, cudaStream_t stream)
@@ -262,21 +261,33 @@ cudaError_t tables_build(int B, void* mem, BandTables* t, cudaStream_t stream)
     t->w = reinterpret_cast<double*>(take(N * sizeof(double)));
     t->twiddle = reinterpret_cast<double2*>(take(fft_twiddle_elems((int)N) * sizeof(double2)));
     t->ht = reinterpret_cast<double2*>(take(B * sizeof(double2)));
-    const size_t dbytes = (size_t)delta_entries(B) * sizeof(double);
-    t->delta = reinterpret_cast<double*>(take(dbytes));
-    t->trig = reinterpret_cast<double*>(take((size_t)trig_entries(B) * sizeof(double)));
     const int threads = 64;
     int ra = 0, rb = 0;
     if (!fft_two_radices((int)N, &ra, &rb)) ra = 0;
     tables_kernel<<<((int)N + threads - 1) / threads, threads, 0, stream>>>(B, t->cosb, t->sinh, t->cosh, t->w,
                                                                              t->twiddle, t->ht, ra);
-    cudaError_t e = cudaGetLastError();
-    if (e == cudaSuccess) e = cudaMemsetAsync(t->delta, 0, dbytes, stream);
+    return cudaGetLastError();
+}
+
+size_t series_tables_bytes(int B)
+{
+    return align256((size_t)delta_entries(B) * sizeof(double)) + align256((size_t)trig_entries(B) * sizeof(double));
+}
+
+cudaError_t series_tables_build(int B, void* mem, BandTables* t, cudaStream_t stream)
+{
+    const size_t dbytes = (size_t)delta_entries(B) * sizeof(double);
+    double* delta = static_cast<double*>(mem);
+    double* trig = reinterpret_cast<double*>(static_cast<char*>(mem) + align256(dbytes));
+    const int threads = 64;
+    cudaError_t e = cudaMemsetAsync(delta, 0, dbytes, stream);
     if (e != cudaSuccess) return e;
-    delta_kernel<<<(num_classes(B) + threads - 1) / threads, threads, 0, stream>>>(B, t->delta);
+    delta_kernel<<<(num_classes(B) + threads - 1) / threads, threads, 0, stream>>>(B, delta);
     e = cudaGetLastError();
     if (e != cudaSuccess) return e;
-    trig_kernel<<<(int)std::min<long long>((trig_entries(B) + 255) / 256, 1024), 256, 0, stream>>>(B, t->trig);
+    trig_kernel<<<(int)std::min<long long>((trig_entries(B) + 255) / 256, 1024), 256, 0, stream>>>(B, trig);
+    t->delta = delta;
+    t->trig = trig;
     return cudaGetLastError();
 }
 
