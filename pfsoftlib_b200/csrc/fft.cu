@@ -223,7 +223,7 @@ template <class P>
 __global__ void __launch_bounds__(256, P::kMinBlocks)
     fft_chirp_kernel(const double2* src, double2* dst, const __grid_constant__ FftPassArgs a, int sign)
 {
-    constexpr int R0 = P::R0, R1 = P::R1, R2 = P::R2, RL = P::RL, V = P::V, M = P::M, h0 = P::h0, h1 = P::h1, PM = P::PM;
+    constexpr int R0 = P::R0, R1 = P::R1, RL = P::RL, V = P::V, M = P::M, h0 = P::h0, h1 = P::h1, PM = P::PM;
     static_assert(R0 == 8, "the first stage's butterfly");
     extern __shared__ double2 smem[];   // [2][V][PM]
     if (a.srcs) {

@@ -10,13 +10,13 @@
 //
 // What bounds it: HBM. Against the ping-pong and in-place kernels of three or four stages that ran these
 // lengths before, us per pass (of the 32 N^3 bytes at the measured copy rate): N = 112 17 against
-// 31 .. 62, 200 66 against 108 (0.60), 256 90 against 98 (0.92), 320 199 against about 290 (0.82), 384 345
-// against 553 (0.82), 400 390 against 760 (0.81), 512 885 against 1210 (0.75). The primes 17 .. 31 cost R
+// 31 .. 62, 200 66 against 108 (0.60), 256 89 against 98 (0.93), 320 199 against about 290 (0.82), 384 345
+// against 553 (0.82), 400 390 against 760 (0.81), 512 853 against 1210 (0.78). The primes 17 .. 31 cost R
 // multiply-adds per point, under the 90 that fit the HBM time; against the chirp pass, us per pass: N =
 // 136 32 / 64, 184 81 / 145, 248 179 / 292, 272 131 / 449, 304 183 / 571, 408 426 / 1480, 496 970 / 2274.
 //
 // Tiles of 8 vectors move 128-byte runs on the transposed side; at radices 18 .. 26 four vectors and four
-// CTAs per SM measured faster (N = 320 199 us against 230), at 28 .. 32 eight (N = 512 885 against 1000).
+// CTAs per SM measured faster (N = 320 199 us against 230), from 28 on eight (N = 512 885 against 1000).
 
 #include <algorithm>
 #include <type_traits>
@@ -101,19 +101,24 @@ __device__ __forceinline__ void stage_two(const FftPassArgs& a, double2* dst, co
     }
 }
 
-// The kernels: 0 for radices up to 16, 1 up to 26, 2 up to 32, 3 and 4 the same with the primes from 17
-// on (23 only in 4: its sums would spill in 3), so that no length pays the registers or the code of a
-// radix that it does not need (N = 512 with the primes in kernel 2: 913 us per pass, without 885).
-constexpr int kKinds = 5;
-constexpr int kMaxRadix[kKinds] = {16, 26, 32, 26, 32};
+// The kernels: 0 for radices up to 16, 1 up to 26, 2 up to 30, 4 and 5 up to 26 and 32 with the primes from
+// 17 on (23 only in 5: its sums would spill in 4), 3 and 6 for 16.32, 32.32 and 16.16 alone, so that no length
+// pays the registers or the code of a radix that it does not need (us per pass: N = 256 in kernel 0 93.2,
+// alone 88.9; 512 with the primes 913, without 885, alone 853). CTAs per SM: up to 16 five are faster than four (N =
+// 128 21.2 against 23.1, 192 44.8 against 47.3, 240 78.2 against 80.7; not for 16.16), up to 30 three
+// faster than two (N = 448 545 against 653), at 32 two (N = 512 885 against 947).
+constexpr int kKinds = 7;
+constexpr int kMaxRadix[kKinds] = {16, 26, 30, 32, 26, 32, 16}, kBlocks[kKinds] = {5, 4, 3, 2, 4, 2, 4};
 constexpr bool is_prime17(int r) { return r == 17 || r == 19 || r == 23 || r == 29 || r == 31; }
 constexpr bool has_radix(int kind, int r)
 {
-    return r >= (kind == 1 ? 7 : (kind == 2 ? 14 : 2)) && r <= kMaxRadix[kind] && r != 27 && (kind >= 3 || !is_prime17(r)) &&
-           (kind != 3 || r != 23);
+    if (kind == 3 || kind == 6) return r == 16 || (kind == 3 && r == 32);
+    return r >= (kind == 1 ? 7 : (kind == 2 ? 14 : 2)) && r <= kMaxRadix[kind] && r != 27 &&
+           (kind == 4 || kind == 5 || !is_prime17(r)) && (kind != 4 || r != 23);
 }
 constexpr int kind_of(int ra, int rb)
 {
+    if (ra == 16 && rb == 16) return 6;
     for (int kind = 0; kind < kKinds; ++kind)
         if (has_radix(kind, ra) && has_radix(kind, rb)) return kind;
     return -1;
@@ -135,7 +140,7 @@ __device__ __forceinline__ void with_radix(int r, const Fn& f)
 }
 
 template <int SIGN, int KIND>
-__global__ void __launch_bounds__(128, KIND == 2 || KIND == 4 ? 2 : 4)
+__global__ void __launch_bounds__(128, kBlocks[KIND])
     fft_two_kernel(const double2* src, double2* dst, const __grid_constant__ FftPassArgs a)
 {
     extern __shared__ double2 smem[];
@@ -284,7 +289,7 @@ bool fft_two_radices(int n, int* ra, int* rb)
         if (n % hi || lo > hi || lo < 2) continue;
         const int kind = kind_of(lo, hi);
         // 2 x 17 .. 2 x 31 fill too few threads (n = 58, us per pass: 19, the chirp pass 13)
-        if (kind < 0 || (kind >= 3 && (lo < 3 || !(is_prime17(lo) || is_prime17(hi))))) continue;
+        if (kind < 0 || ((kind == 4 || kind == 5) && lo < (is_prime17(lo) || is_prime17(hi) ? 3 : 14))) continue;
         *ra = lo;
         *rb = hi;
         return true;
@@ -295,7 +300,7 @@ bool fft_two_radices(int n, int* ra, int* rb)
 int fft_two_vectors(int n)
 {
     int ra, rb;
-    return fft_two_radices(n, &ra, &rb) && kind_of(ra, rb) % 2 ? 4 : 8;
+    return fft_two_radices(n, &ra, &rb) && (kind_of(ra, rb) == 1 || kind_of(ra, rb) == 4) ? 4 : 8;
 }
 
 cudaError_t fft_two_launch(const double2* src, double2* dst, const FftPassArgs& a, int ntiles, int sign, cudaStream_t stream, int nz)
@@ -318,6 +323,8 @@ cudaError_t fft_two_launch(const double2* src, double2* dst, const FftPassArgs& 
         case 2: return sign < 0 ? go(fft_two_kernel<-1, 2>) : go(fft_two_kernel<1, 2>);
         case 3: return sign < 0 ? go(fft_two_kernel<-1, 3>) : go(fft_two_kernel<1, 3>);
         case 4: return sign < 0 ? go(fft_two_kernel<-1, 4>) : go(fft_two_kernel<1, 4>);
+        case 5: return sign < 0 ? go(fft_two_kernel<-1, 5>) : go(fft_two_kernel<1, 5>);
+        case 6: return sign < 0 ? go(fft_two_kernel<-1, 6>) : go(fft_two_kernel<1, 6>);
         default: return cudaErrorInvalidValue;
     }
 }
