@@ -17,6 +17,7 @@
 #include <algorithm>
 
 #include "common.cuh"
+#include "dd.cuh"
 #include "dwt.cuh"
 #include "dwt_common.cuh"
 #include "fft.cuh"
@@ -154,48 +155,10 @@ __global__ void trig_kernel(int B, double* trig)
     }
 }
 
-// ---- the rows at beta = pi/2, in double-double arithmetic (Dekker 1971, Knuth; products by FMA) ----
-struct dd {
-    double h, l;
-};
-__device__ __forceinline__ dd quick_sum(double a, double b)   // |a| >= |b|
-{
-    const double s = a + b;
-    return {s, b - (s - a)};
-}
-__device__ __forceinline__ dd dd_add(dd a, dd b)
-{
-    const double s = a.h + b.h, v = s - a.h;
-    const double e = (a.h - (s - v)) + (b.h - v);
-    return quick_sum(s, e + a.l + b.l);
-}
-__device__ __forceinline__ dd dd_mul(dd a, dd b)
-{
-    const double p = a.h * b.h;
-    return quick_sum(p, fma(a.h, b.h, -p) + (a.h * b.l + a.l * b.h));
-}
-__device__ __forceinline__ dd dd_scale(dd a, double b)
-{
-    const double p = a.h * b;
-    return quick_sum(p, fma(a.h, b, -p) + a.l * b);
-}
-__device__ __forceinline__ dd dd_div(dd a, dd b)
-{
-    const double q = a.h / b.h;
-    const dd r = dd_add(a, dd_scale(b, -q));
-    return quick_sum(q, (r.h + r.l) / b.h);
-}
-__device__ __forceinline__ dd dd_sqrt(dd a)
-{
-    if (a.h == 0.0) return {0.0, 0.0};
-    const double r = sqrt(a.h);
-    return quick_sum(r, (fma(-r, r, a.h) + a.l) / (2.0 * r));
-}
-
 // P[l][a][b] for one pair a >= b per thread, l = a .. B-1, and its mirror image: the recurrence of
 // fn_dwt.hpp:167-199 at cos beta = 0 without its normalisation,
 //   P(l+1) = -((2l+1) a b P(l) + (l+1) sqrt(q(l)) P(l-1)) / (l sqrt(q(l+1))),  q(l) = (l^2-a^2)(l^2-b^2),
-// from P(a) = sqrt(binomial(2a, a-b)) 2^-a. Double-double keeps the products of two entries within
+// from delta_seed, in double-double arithmetic (dd.cuh), which keeps the products of two entries within
 // two ulp over any number of steps. The table starts zeroed.
 __global__ void delta_kernel(int B, double* delta)
 {
@@ -203,11 +166,7 @@ __global__ void delta_kernel(int B, double* delta)
     if (i >= num_classes(B)) return;
     int a, b;
     class_orders(i, a, b);
-    dd cur = {1.0, 0.0}, prev = {0.0, 0.0};
-    for (int q = 0; q < a - b; ++q) cur = dd_div(dd_scale(cur, (double)(2 * a - q)), dd{(double)(q + 1), 0.0});
-    cur = dd_sqrt(cur);
-    cur.h = ldexp(cur.h, -a);
-    cur.l = ldexp(cur.l, -a);
+    dd cur = delta_seed(a, b), prev = {0.0, 0.0};
     auto at = [&](int M, int n, int l) {
         const int lb = l >> 3, b0 = M >> 3;
         return delta_offset(B, M) + 64 * (long long)(lb * (lb + 1) / 2 - b0 * (b0 + 1) / 2 + (n >> 3)) + (l & 7) * 8 + (n & 7);
