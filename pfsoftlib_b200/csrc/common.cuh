@@ -16,6 +16,20 @@
 
 namespace pfsoft_dev {
 
+constexpr size_t kMaxShared = 227 * 1024;   // of a CTA
+
+// Leave for a launch with `need` bytes of dynamic shared memory. The leave belongs to the kernel, not to the
+// launch, and host threads launch one kernel with different sizes: it is always set to the kernel's
+// largest size, so that no thread takes back what another is about to use. (48 KB with a kernel's static
+// part need none.)
+template <class K>
+cudaError_t allow_shared(K kernel, size_t need, size_t largest)
+{
+    if (need > largest) return cudaErrorInvalidValue;
+    if (need <= 47 * 1024) return cudaSuccess;
+    return cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)largest);
+}
+
 __host__ __device__ __forceinline__ double2 cadd(double2 a, double2 b) { return make_double2(a.x + b.x, a.y + b.y); }
 __host__ __device__ __forceinline__ double2 csub(double2 a, double2 b) { return make_double2(a.x - b.x, a.y - b.y); }
 __host__ __device__ __forceinline__ double2 cmul(double2 a, double2 b)

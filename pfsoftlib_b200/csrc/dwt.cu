@@ -722,15 +722,13 @@ __global__ void zero_nyquist_kernel(double2* X, int B)
 }
 
 template <class K, class In, class Out>
-cudaError_t launch(K kernel, In in, Out out, int threads, size_t smem, const DwtArgs& a, int T, cudaStream_t s)
+cudaError_t launch(K kernel, In in, Out out, int threads, size_t smem, size_t largest, const DwtArgs& a, int T, cudaStream_t s)
 {
     DwtArgs b = a;
     b.T = T;
     b.items = (a.classes ? a.n_classes : num_classes(a.B)) * T;
-    if (smem > 47 * 1024) {   // the static part included, 48 KB need no leave
-        cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-        if (e != cudaSuccess) return e;
-    }
+    const cudaError_t e = allow_shared(kernel, smem, largest);
+    if (e != cudaSuccess) return e;
     kernel<<<b.items, threads, smem, s>>>(in, out, b);
     return cudaGetLastError();
 }
@@ -739,18 +737,18 @@ template <class F, int KP>
 cudaError_t launch_fft(int dir, const double2* X, double2* coeffs, const DwtArgs& a, int T, cudaStream_t s)
 {
     // the columns' DFT, and behind it the forward's B fragments or the inverse's coefficients
-    const size_t smem = (F::kElems + ((a.B + 7) / 8) * (dir == 0 ? 64 : 8 * kGS)) * sizeof(double2);
-    return dir == 0 ? launch(dwt_forward_fft_kernel<F, KP>, X, coeffs, F::NT, smem, a, T, s)
-                    : launch(dwt_inverse_fft_kernel<F, KP>, (const double2*)coeffs, const_cast<double2*>(X), F::NT, smem, a, T, s);
+    const size_t smem = (F::kElems + ((F::B + 7) / 8) * (dir == 0 ? 64 : 8 * kGS)) * sizeof(double2);
+    return dir == 0 ? launch(dwt_forward_fft_kernel<F, KP>, X, coeffs, F::NT, smem, smem, a, T, s)
+                    : launch(dwt_inverse_fft_kernel<F, KP>, (const double2*)coeffs, const_cast<double2*>(X), F::NT, smem, smem, a, T, s);
 }
 
 template <int NW, int KP, int MB>
 cudaError_t launch_mma(int dir, const double2* X, double2* coeffs, const DwtArgs& a, int T, cudaStream_t s)
 {
-    const int nb = (a.B + 7) / 8, mb = (nb + 1) / 2;
-    const size_t smem = (dir == 0 ? 192 * nb : 128 * mb + 8 * kGS * nb) * sizeof(double2);
-    return dir == 0 ? launch(dwt_forward_mma_kernel<NW, KP, MB>, X, coeffs, 32 * NW, smem, a, T, s)
-                    : launch(dwt_inverse_mma_kernel<NW, KP, MB>, (const double2*)coeffs, const_cast<double2*>(X), 32 * NW, smem, a, T, s);
+    auto bytes = [&](int nb) { return (dir == 0 ? 192 * nb : 128 * ((nb + 1) / 2) + 8 * kGS * nb) * sizeof(double2); };
+    const size_t smem = bytes((a.B + 7) / 8), largest = bytes(NW * KP);   // the warps' accumulators hold NW KP tiles
+    return dir == 0 ? launch(dwt_forward_mma_kernel<NW, KP, MB>, X, coeffs, 32 * NW, smem, largest, a, T, s)
+                    : launch(dwt_inverse_mma_kernel<NW, KP, MB>, (const double2*)coeffs, const_cast<double2*>(X), 32 * NW, smem, largest, a, T, s);
 }
 
 // The radices of a DFT length N: of the products of two or three of at most 20, the first even, the one

@@ -359,10 +359,8 @@ struct ChirpEntry {
 template <class P>
 cudaError_t chirp_launch(const double2* src, double2* dst, const FftPassArgs& a, int ntiles, int sign, cudaStream_t stream, int nz)
 {
-    if (P::kSmem > 48 * 1024) {
-        const cudaError_t e = cudaFuncSetAttribute(fft_chirp_kernel<P>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)P::kSmem);
-        if (e != cudaSuccess) return e;
-    }
+    const cudaError_t e = allow_shared(fft_chirp_kernel<P>, P::kSmem, P::kSmem);
+    if (e != cudaSuccess) return e;
     fft_chirp_kernel<P><<<dim3((a.nvec + P::V - 1) / P::V, ntiles, nz), 256, P::kSmem, stream>>>(src, dst, a, sign);
     return cudaGetLastError();
 }
@@ -561,13 +559,14 @@ cudaError_t fft_pass_launch(const double2* src, double2* dst, const FftPassArgs&
     const int nthreads = std::min(256, ((a.kb * widest + 31) / 32) * 32);
     dim3 grid((a.nvec + a.kb - 1) / a.kb, ntiles, nz);
     const size_t smem = fft_pass_smem_bytes(a);
-    auto go = [&](auto kern) {
-        if (smem > 48 * 1024) cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    auto go = [&](auto kern) -> cudaError_t {
+        const cudaError_t e = allow_shared(kern, smem, kMaxShared);
+        if (e != cudaSuccess) return e;
         kern<<<grid, nthreads, smem, stream>>>(src, dst, a);
+        return cudaGetLastError();
     };
     // the kernel indexes two buffers; with a single buffer the second is never used
-    sign < 0 ? go(fft_pass_kernel<-1>) : go(fft_pass_kernel<1>);
-    return cudaGetLastError();
+    return sign < 0 ? go(fft_pass_kernel<-1>) : go(fft_pass_kernel<1>);
 }
 
 }  // namespace pfsoft_dev

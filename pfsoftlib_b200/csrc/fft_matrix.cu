@@ -233,10 +233,8 @@ cudaError_t fft_matrix_launch(const double2* src, double2* dst, const FftPassArg
     const int R = a.radix[0], nt = ((a.radix[1] + 1) / 2 + 7) / 8;
     const size_t smem = (size_t)R * 128 * nt * sizeof(double2);
     auto go = [&](auto k, int threads) -> cudaError_t {
-        if (smem > 48 * 1024) {
-            const cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-            if (e != cudaSuccess) return e;
-        }
+        const cudaError_t e = allow_shared(k, smem, (size_t)kMaxTiles * 128 * sizeof(double2));
+        if (e != cudaSuccess) return e;
         k<<<dim3((a.nvec + 7) / 8, ntiles, nz), threads, smem, stream>>>(src, dst, a);
         return cudaGetLastError();
     };

@@ -308,12 +308,12 @@ cudaError_t fft_two_launch(const double2* src, double2* dst, const FftPassArgs& 
     const int ra = a.radix[0], rb = a.radix[1];
     const int kind = kind_of(ra, rb);
     const size_t smem = (size_t)a.kb * block_pitch(ra, rb, a.kb) * sizeof(double2);
+    const int top = kMaxRadix[kind < 0 ? 0 : kind];
+    const size_t largest = (size_t)8 * block_pitch(top, top, 8) * sizeof(double2);   // the kind's largest radices
     const int threads = std::min(128, (a.kb * rb + 31) / 32 * 32);
     auto go = [&](auto k) -> cudaError_t {
-        if (smem > 48 * 1024) {
-            const cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-            if (e != cudaSuccess) return e;
-        }
+        const cudaError_t e = allow_shared(k, smem, largest);
+        if (e != cudaSuccess) return e;
         k<<<dim3((a.nvec + a.kb - 1) / a.kb, ntiles, nz), threads, smem, stream>>>(src, dst, a);
         return cudaGetLastError();
     };
@@ -341,11 +341,7 @@ cudaError_t fft_plane_launch(const double2* src, double2* dst, const FftPlaneArg
     if (!fft_plane_supported(a.n, nz) || !fft_two_radices(a.n, &a.ra, &a.rb)) return cudaErrorInvalidValue;
     const size_t smem = (size_t)a.n * Plane(a.n, a.ra, a.rb).pl * sizeof(double2);
     const int threads = std::min(512, (a.n * a.rb + 31) / 32 * 32);
-    auto go = [&](auto k) -> cudaError_t {
-        if (smem > 48 * 1024) {
-            const cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-            if (e != cudaSuccess) return e;
-        }
+    auto go = [&](auto k) -> cudaError_t {   // 42 KB of shared memory at most
         k<<<dim3(a.n, 1, nz), threads, smem, stream>>>(src, dst, a);
         return cudaGetLastError();
     };
