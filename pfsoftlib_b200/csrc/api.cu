@@ -235,6 +235,7 @@ cudaError_t copy_out(StagingContext* st, void* host, const void* dev, size_t byt
 struct DeviceState {
     std::mutex mu;
     std::map<int, BandTables> tables;
+    cudaStream_t table_stream = nullptr;   // builds them
     void* ws = nullptr;          // library-owned workspace (NULL-workspace calls)
     size_t ws_bytes = 0;
     // host-staged calls
@@ -339,8 +340,17 @@ size_t grid_elems(int B)
     return N * N * N;
 }
 
-// Tables for bandwidth B on the current device, each set built on first use.
-int get_tables(int B, cudaStream_t stream, BandTables* out, int sets = kSeriesTables)
+// The calling thread's capture mode is relaxed while it lives: a first call may come while a stream is
+// being captured, and allocating would invalidate the capture in the other modes.
+struct RelaxedCapture {
+    cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
+    RelaxedCapture() { cudaThreadExchangeStreamCaptureMode(&mode); }
+    ~RelaxedCapture() { cudaThreadExchangeStreamCaptureMode(&mode); }
+};
+
+// Tables for bandwidth B on the current device, each set built on first use, on a stream of its own: the
+// caller's may be under capture, and the tables belong to no recording.
+int get_tables(int B, BandTables* out, int sets = kSeriesTables)
 {
     int dev = 0;
     PF_CUDA(cudaGetDevice(&dev));
@@ -355,6 +365,9 @@ int get_tables(int B, cudaStream_t stream, BandTables* out, int sets = kSeriesTa
         *out = t;
         return PFSOFT_OK;
     }
+    RelaxedCapture relaxed;
+    if (!st->table_stream) PF_CUDA(cudaStreamCreateWithFlags(&st->table_stream, cudaStreamNonBlocking));
+    const cudaStream_t stream = st->table_stream;
     // one block: allocate, fill on the stream, wait
     auto build = [&](size_t bytes, auto fill) -> int {
         void* mem = nullptr;
@@ -380,7 +393,8 @@ int get_tables(int B, cudaStream_t stream, BandTables* out, int sets = kSeriesTa
             fft_bluestein_fill(2 * B, h.data());
             void* bt = nullptr;
             cudaError_t e = cudaMalloc(&bt, h.size() * sizeof(double2));
-            if (e == cudaSuccess) e = cudaMemcpy(bt, h.data(), h.size() * sizeof(double2), cudaMemcpyHostToDevice);
+            if (e == cudaSuccess) e = cudaMemcpyAsync(bt, h.data(), h.size() * sizeof(double2), cudaMemcpyHostToDevice, stream);
+            if (e == cudaSuccess) e = cudaStreamSynchronize(stream);
             if (e != cudaSuccess) {
                 cudaFree(bt);
                 cudaFree(t.block);
@@ -468,7 +482,7 @@ int check_transform_args(const void* a, const void* b, int B, void*& ws, size_t 
 int run_dsoft(const double* d_grid, int B, double* d_coeffs, void* ws, cudaStream_t s)
 {
     BandTables t;
-    int rc = get_tables(B, s, &t);
+    int rc = get_tables(B, &t);
     if (rc) return rc;
     const int N = 2 * B;
     const long long n = N, n2 = n * n;
@@ -501,7 +515,7 @@ int run_dsoft(const double* d_grid, int B, double* d_coeffs, void* ws, cudaStrea
 int run_idsoft(const double* d_coeffs, int B, double* d_grid, void* ws, cudaStream_t s)
 {
     BandTables t;
-    int rc = get_tables(B, s, &t);
+    int rc = get_tables(B, &t);
     if (rc) return rc;
     const int N = 2 * B;
     const long long n = N, n2 = n * n;
@@ -619,7 +633,7 @@ __global__ void wigner_matrix_kernel(int B, int M, int Mp, const double* w, cons
 }  // namespace
 
 namespace pfsoft_dev {
-int tables_for(int B, cudaStream_t s, BandTables* out, int sets) { return get_tables(B, s, out, sets); }
+int tables_for(int B, BandTables* out, int sets) { return get_tables(B, out, sets); }
 }  // namespace pfsoft_dev
 
 extern "C" {
@@ -732,7 +746,7 @@ static int layer_wise(int cols, int rows, int lays, double* d_arr, double scale,
         void* tmp_b = nullptr;
         if (n % 2 == 0 && valid_bandwidth(n / 2)) {
             BandTables t;
-            int rc = get_tables(n / 2, s, &t, 0);
+            int rc = get_tables(n / 2, &t, 0);
             if (rc) return rc;
             tw = t.twiddle;
             blu = t.bluestein;
@@ -851,7 +865,7 @@ int pfsoft_cuda_quadrature_weights(int B, double* d_w, void* stream)
     if (!d_w) return fail(PFSOFT_EINVAL, "null output pointer");
     cudaStream_t s = static_cast<cudaStream_t>(stream);
     BandTables t;
-    int rc = get_tables(B, s, &t);
+    int rc = get_tables(B, &t);
     if (rc) return rc;
     copy_weights_kernel<<<(2 * B + 255) / 256, 256, 0, s>>>(t.w, d_w, 2 * B);
     PF_CUDA(cudaGetLastError());
@@ -866,7 +880,7 @@ int pfsoft_cuda_wigner_d_matrix(int B, int M, int Mp, int weighted, double* d_ou
     if (M <= -B || M >= B || Mp <= -B || Mp >= B) return fail(PFSOFT_EINVAL, "orders must satisfy |M|,|M'| < B");
     cudaStream_t s = static_cast<cudaStream_t>(stream);
     BandTables t;
-    int rc = get_tables(B, s, &t);
+    int rc = get_tables(B, &t);
     if (rc) return rc;
     wigner_matrix_kernel<<<(2 * B + 127) / 128, 128, 0, s>>>(B, M, Mp, weighted ? t.w : nullptr, t.cosb, t.sinh,
                                                               t.cosh, d_out);

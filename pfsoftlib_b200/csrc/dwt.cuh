@@ -72,7 +72,7 @@ cudaError_t split_tables_build(int B, void* mem, BandTables* t, cudaStream_t str
 // The cached tables of a bandwidth on the current device (api.cu), with the DWTs' named by `sets` built on
 // first use: what a process keeps is what its calls need.
 constexpr int kSeriesTables = 1, kSplitTables = 2;
-int tables_for(int B, cudaStream_t s, BandTables* out, int sets = kSeriesTables);
+int tables_for(int B, BandTables* out, int sets = kSeriesTables);
 
 struct DwtArgs {
     int B, N;

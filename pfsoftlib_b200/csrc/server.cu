@@ -100,7 +100,6 @@ struct pfsoft_server {
     int max_batch = 16;
     bool split = false;          // PFSOFT_SERVER_SPLIT
     size_t stage_bytes = 0;
-    cudaStream_t table_stream = nullptr;   // builds a bandwidth's tables at submission
     std::vector<Slot> slots;
     void* arena_base = nullptr;
     pfsoft_serving::Arena arena;
@@ -163,7 +162,7 @@ int launch_split_batch(pfsoft_server* s, Batch* b, const std::vector<Request>& i
     int pos = 0;
     for (const auto& kv : byB) {
         BandTables t;
-        const int rc = tables_for(kv.first, sl.stream, &t, kSplitTables);
+        const int rc = tables_for(kv.first, &t, kSplitTables);
         if (rc) return rc;
         const int g = (int)tabs.size();
         for (size_t m = 0; m < kv.second.size(); ++m) {
@@ -228,7 +227,7 @@ int launch_batch(pfsoft_server* s, Batch* b, const std::vector<Request>& io)
     Slot& sl = s->slots[b->slot];
     const int B = b->plan.B, k = (int)b->plan.ids.size(), dir = b->plan.dir;
     BandTables t;
-    int rc = tables_for(B, sl.stream, &t);
+    int rc = tables_for(B, &t);
     if (rc) return rc;
     const size_t cap = (size_t)s->max_batch;
     double2** h_tab = reinterpret_cast<double2**>(sl.h_stage);
@@ -392,7 +391,6 @@ int pfsoft_server_create_ex(size_t budget_bytes, int max_batch, int streams, int
     s->sched.set_mixed(s->split);
     cudaError_t e = cudaGetDevice(&s->device);
     if (e == cudaSuccess && s->split) e = dwt_split_prepare();
-    if (e == cudaSuccess) e = cudaStreamCreateWithFlags(&s->table_stream, cudaStreamNonBlocking);
     if (e == cudaSuccess) e = cudaMalloc(&s->arena_base, budget_bytes);
     s->arena.reset(e == cudaSuccess ? budget_bytes : 0, 256);
     s->slots.resize(streams);
@@ -420,7 +418,6 @@ int pfsoft_server_create_ex(size_t budget_bytes, int max_batch, int streams, int
             cudaFree(sl.d_stage);
             cudaFreeHost(sl.h_status);
         }
-        if (s->table_stream) cudaStreamDestroy(s->table_stream);
         cudaFree(s->arena_base);
         delete s;
         cudaGetLastError();
@@ -447,7 +444,6 @@ int pfsoft_server_destroy(pfsoft_server* s)
         cudaFree(sl.d_stage);
         cudaFreeHost(sl.h_status);
     }
-    if (s->table_stream) cudaStreamDestroy(s->table_stream);
     for (cudaEvent_t ev : s->dead_events)
         if (ev) cudaEventDestroy(ev);
     cudaFree(s->arena_base);
@@ -476,11 +472,11 @@ int pfsoft_server_submit(pfsoft_server* s, int direction, int B, const double* d
         }
     }
     // the bandwidth's constant tables are built here, at admission (once per device and
-    // bandwidth, on the server's own stream), so that no batch waits for them and the request's
+    // bandwidth), so that no batch waits for them and the request's
     // latency, counted from the end of this call, does not include them
     {
         BandTables t;
-        const int rc = tables_for(B, s->table_stream, &t, s->split ? kSplitTables : kSeriesTables);
+        const int rc = tables_for(B, &t, s->split ? kSplitTables : kSeriesTables);
         if (rc) return rc;
     }
     cudaEvent_t ready = nullptr;
