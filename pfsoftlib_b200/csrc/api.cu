@@ -865,7 +865,7 @@ int pfsoft_cuda_quadrature_weights(int B, double* d_w, void* stream)
     if (!d_w) return fail(PFSOFT_EINVAL, "null output pointer");
     cudaStream_t s = static_cast<cudaStream_t>(stream);
     BandTables t;
-    int rc = get_tables(B, &t);
+    int rc = get_tables(B, &t, 0);
     if (rc) return rc;
     copy_weights_kernel<<<(2 * B + 255) / 256, 256, 0, s>>>(t.w, d_w, 2 * B);
     PF_CUDA(cudaGetLastError());
@@ -880,7 +880,7 @@ int pfsoft_cuda_wigner_d_matrix(int B, int M, int Mp, int weighted, double* d_ou
     if (M <= -B || M >= B || Mp <= -B || Mp >= B) return fail(PFSOFT_EINVAL, "orders must satisfy |M|,|M'| < B");
     cudaStream_t s = static_cast<cudaStream_t>(stream);
     BandTables t;
-    int rc = get_tables(B, &t);
+    int rc = get_tables(B, &t, 0);
     if (rc) return rc;
     wigner_matrix_kernel<<<(2 * B + 127) / 128, 128, 0, s>>>(B, M, Mp, weighted ? t.w : nullptr, t.cosb, t.sinh,
                                                               t.cosh, d_out);

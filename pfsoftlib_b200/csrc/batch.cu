@@ -278,7 +278,7 @@ int pfsoft_batch_create(const int* bandwidths, int count, int transforms_per_cta
             ws_total += ((((size_t)g.N * g.N * g.N + (g.split ? dwt_split_aux_elems(g.B) : 0)) * sizeof(double2) + kFftSyncBytes
                           + 255) & ~(size_t)255);   // each workspace 256-byte aligned
         }
-        int rc = tables_for(g.B, &g.tables, kSeriesTables | (g.split ? kSplitTables : 0));
+        int rc = tables_for(g.B, &g.tables, g.split ? kSplitTables : kSeriesTables);
         if (rc) {
             free_batch(b);
             return rc;

@@ -312,7 +312,7 @@ int pfsoft_shard_fft_forward(pfsoft_shard_plan* plan, const double* d_slab_grid,
     if (d_slab_grid == d_slab_spectrum) return fail(PFSOFT_EINVAL, "slab grid and slab spectrum must not alias");
     cudaStream_t s = static_cast<cudaStream_t>(stream);
     BandTables t;
-    if ((rc = tables_for(p.B, &t))) return rc;
+    if ((rc = tables_for(p.B, &t, 0))) return rc;
     const long long N = p.N, n2 = N * N, K = nk;
     // F1: gamma DFT of each layer row, G[kk][c][e] -> S[e][c][kk]; F2: alpha DFT in place
     FftPassArgs f1 = slab_pass(p.N, nk, t, FftStrides{n2, N, 1}, FftStrides{1, K, N * K}, 1.0);
@@ -337,7 +337,7 @@ int pfsoft_shard_fft_inverse(pfsoft_shard_plan* plan, double* d_slab_spectrum, d
     if (d_slab_grid == d_slab_spectrum) return fail(PFSOFT_EINVAL, "slab grid and slab spectrum must not alias");
     cudaStream_t s = static_cast<cudaStream_t>(stream);
     BandTables t;
-    if ((rc = tables_for(p.B, &t))) return rc;
+    if ((rc = tables_for(p.B, &t, 0))) return rc;
     const long long N = p.N, n2 = N * N, K = nk;
     FftPassArgs i2 = slab_pass(p.N, nk, t, FftStrides{1, N * K, K}, FftStrides{1, N * K, K}, 1.0);
     // scaled by 1/(4B^2) as the single-GPU path (src/fn_idsoft.cpp:289)
