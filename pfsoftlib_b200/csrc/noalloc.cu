@@ -8,14 +8,16 @@
 // per-bandwidth tables, both allocated on first use; this entry point takes both from one
 // file-scope device array instead.
 //
-// Limit: bandwidth B <= 32 (a 64^3 complex128 spectrum, 4 MiB, plus 320 KiB reserved for the
-// tables, of which B = 32 needs about 125 KiB). Every GPU that loads the library holds this
-// array until the process exits. All calls on a device share it and it keeps the last call's
-// contents; nothing in it has to start at zero (the first FFT pass overwrites the whole spectrum
-// before anything reads it, and the tables are rebuilt whenever the bandwidth changes). Calls
-// that overlap on the GPU race on it. Once a call has been recorded into a CUDA graph on a
-// device, every later call on that device rebuilds the tables (two small kernels and a clear): a graph
-// replay rewrites the array with its own bandwidth's tables, which the host cannot see.
+// Limit: bandwidth B <= 32 (a 64^3 complex128 spectrum, 4 MiB, plus the tables of every bandwidth, 1.8 MiB,
+// 141 KiB of them for B = 32). Every GPU that loads the library holds this array until the process
+// exits. All calls on a device share it; nothing in it has to start at zero (the first FFT pass overwrites
+// the whole spectrum before anything reads it, and a bandwidth's first call builds its tables). Calls that
+// overlap on the GPU race on it. Each bandwidth's tables have a place of their own, so that they stay
+// as its first call leaves them whatever runs in between, a replayed graph among it: one place for all
+// costs three small kernels and a clear whenever the bandwidth changes, and once a call has been recorded in
+// every later call and replay (us per call, B = 16 after a recorded call 57 against 14, its replay 47
+// against 12; B = 16 and 32 in turn 144 against 35). Only a recording made before the bandwidth's first
+// direct call holds the kernels that build the tables, since the host does not see whether it is replayed.
 
 #include <cuda_runtime.h>
 
@@ -34,7 +36,7 @@ namespace {
 
 constexpr int kNoAllocMaxB = 32;
 constexpr size_t kSpectrumBytes = (size_t)(2 * kNoAllocMaxB) * (2 * kNoAllocMaxB) * (2 * kNoAllocMaxB) * sizeof(double2);
-constexpr size_t kTableBytes = 320 * 1024;
+constexpr size_t kTableBytes = 1875 * 1024;
 constexpr int kMaxDevices = 64;
 
 // The scratch: spectrum first, tables after it. In host code this name is only a handle for
@@ -43,11 +45,12 @@ __device__ __align__(256) unsigned char g_noalloc_scratch[kSpectrumBytes + kTabl
 
 struct NoAllocDevice {
     bool ready;          // symbol address resolved on this device
-    bool captured;       // a call was recorded into a graph: the host no longer knows the tables
     unsigned char* base; // device address of g_noalloc_scratch
-    int tables_B;        // bandwidth whose tables the array holds (0 = unknown)
-    BandTables tables;
+    bool built[kNoAllocMaxB + 1];   // a direct call has queued the bandwidth's table kernels
+    BandTables tables[kNoAllocMaxB + 1];
 };
+
+size_t all_tables_bytes(int B) { return tables_bytes(B) + series_tables_bytes(B); }
 
 std::mutex g_mu;                       // guards g_dev (host bookkeeping only)
 NoAllocDevice g_dev[kMaxDevices] = {};
@@ -81,24 +84,20 @@ int pfsoft_cuda_dsoft_noalloc(const double* d_grid, int B, double* d_coeffs, voi
         if (e != cudaSuccess || !p) return fail(PFSOFT_ECUDA, "pfsoft_cuda_dsoft_noalloc: cudaGetSymbolAddress failed");
         d.base = static_cast<unsigned char*>(p);
         d.ready = true;
-        d.tables_B = 0;
     }
     cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
     if (cudaStreamIsCapturing(s, &cap) != cudaSuccess)
         return fail(PFSOFT_ECUDA, "pfsoft_cuda_dsoft_noalloc: cudaStreamIsCapturing failed");
-    if (cap != cudaStreamCaptureStatusNone) d.captured = true;
-    if (d.captured || d.tables_B != B) {
-        // recorded into the captured work too, so that every replay builds the tables it reads
-        if (tables_bytes(B) + series_tables_bytes(B) > kTableBytes) return fail(PFSOFT_EINVAL, "pfsoft_cuda_dsoft_noalloc: tables exceed the reserve");
-        unsigned char* mem = d.base + kSpectrumBytes;
-        if (tables_build(B, mem, &d.tables, s) != cudaSuccess ||
-            series_tables_build(B, mem + tables_bytes(B), &d.tables, s) != cudaSuccess) {
-            d.tables_B = 0;
+    if (!d.built[B]) {
+        size_t at = kSpectrumBytes;
+        for (int b = 1; b < B; ++b) at += all_tables_bytes(b);
+        if (at + all_tables_bytes(B) > sizeof(g_noalloc_scratch)) return fail(PFSOFT_EINVAL, "pfsoft_cuda_dsoft_noalloc: tables exceed the reserve");
+        if (tables_build(B, d.base + at, &d.tables[B], s) != cudaSuccess ||
+            series_tables_build(B, d.base + at + tables_bytes(B), &d.tables[B], s) != cudaSuccess)
             return fail(PFSOFT_ECUDA, "pfsoft_cuda_dsoft_noalloc: table kernels failed to launch");
-        }
-        d.tables_B = d.captured ? 0 : B;
+        d.built[B] = cap == cudaStreamCaptureStatusNone;
     }
-    const BandTables& t = d.tables;
+    const BandTables& t = d.tables[B];
     const int N = 2 * B;
     const long long n = N, n2 = n * n;
     double2* X = reinterpret_cast<double2*>(d.base);
