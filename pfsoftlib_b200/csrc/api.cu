@@ -368,52 +368,44 @@ int get_tables(int B, BandTables* out, int sets = kSeriesTables)
     RelaxedCapture relaxed;
     if (!st->table_stream) PF_CUDA(cudaStreamCreateWithFlags(&st->table_stream, cudaStreamNonBlocking));
     const cudaStream_t stream = st->table_stream;
-    // one block: allocate, fill on the stream, wait
-    auto build = [&](size_t bytes, auto fill) -> int {
+    // a block for each set, all filled on the stream, one wait
+    std::vector<void*> blocks;
+    std::vector<double2> h;   // the table of the FFT's matrix or chirp pass, computed on the host
+    cudaError_t e = cudaSuccess;
+    bool no_memory = false;
+    auto block = [&](size_t bytes) {
         void* mem = nullptr;
-        cudaError_t e = cudaMalloc(&mem, bytes);
-        if (e != cudaSuccess) return fail(PFSOFT_ENOMEM, std::string("table allocation: ") + cudaGetErrorString(e));
-        {
-            StageScope sc(ST_TABLES, stream);
-            e = fill(mem);
+        if (e == cudaSuccess) {
+            e = cudaMalloc(&mem, bytes);
+            no_memory = e != cudaSuccess;
         }
-        if (e == cudaSuccess) e = cudaStreamSynchronize(stream);
-        if (e != cudaSuccess) {
-            cudaFree(mem);
-            return cuda_fail(e, "tables_build");
-        }
-        return PFSOFT_OK;
+        if (mem) blocks.push_back(mem);
+        return mem;
+    };
+    auto build = [&](size_t bytes, auto fill) {
+        void* mem = block(bytes);
+        if (e != cudaSuccess) return;
+        StageScope sc(ST_TABLES, stream);
+        e = fill(mem);
     };
     if (!have) {
-        int rc = build(tables_bytes(B), [&](void* mem) { return tables_build(B, mem, &t, stream); });
-        if (rc) return rc;
-        if (fft_needs_bluestein(2 * B)) {
-            // the table of the FFT's matrix or chirp pass, computed on the host
-            std::vector<double2> h(fft_bluestein_elems(2 * B));
+        build(tables_bytes(B), [&](void* mem) { return tables_build(B, mem, &t, stream); });
+        if (e == cudaSuccess && fft_needs_bluestein(2 * B)) {
+            h.resize(fft_bluestein_elems(2 * B));
             fft_bluestein_fill(2 * B, h.data());
-            void* bt = nullptr;
-            cudaError_t e = cudaMalloc(&bt, h.size() * sizeof(double2));
-            if (e == cudaSuccess) e = cudaMemcpyAsync(bt, h.data(), h.size() * sizeof(double2), cudaMemcpyHostToDevice, stream);
-            if (e == cudaSuccess) e = cudaStreamSynchronize(stream);
-            if (e != cudaSuccess) {
-                cudaFree(bt);
-                cudaFree(t.block);
-                return cuda_fail(e, "tables_build");
-            }
-            t.bluestein = static_cast<double2*>(bt);
+            t.bluestein = static_cast<double2*>(block(h.size() * sizeof(double2)));
+            if (e == cudaSuccess) e = cudaMemcpyAsync(t.bluestein, h.data(), h.size() * sizeof(double2), cudaMemcpyHostToDevice, stream);
         }
-        st->tables[B] = t;
     }
-    if (series) {
-        int rc = build(series_tables_bytes(B), [&](void* mem) { return series_tables_build(B, mem, &t, stream); });
-        if (rc) return rc;
-        st->tables[B] = t;
+    if (series) build(series_tables_bytes(B), [&](void* mem) { return series_tables_build(B, mem, &t, stream); });
+    if (split) build(split_tables_bytes(B), [&](void* mem) { return split_tables_build(B, mem, &t, stream); });
+    const cudaError_t waited = cudaStreamSynchronize(stream);
+    if (e == cudaSuccess) e = waited;
+    if (e != cudaSuccess) {
+        for (void* mem : blocks) cudaFree(mem);
+        return no_memory ? fail(PFSOFT_ENOMEM, std::string("table allocation: ") + cudaGetErrorString(e)) : cuda_fail(e, "tables_build");
     }
-    if (split) {
-        int rc = build(split_tables_bytes(B), [&](void* mem) { return split_tables_build(B, mem, &t, stream); });
-        if (rc) return rc;
-        st->tables[B] = t;
-    }
+    st->tables[B] = t;
     *out = t;
     return PFSOFT_OK;
 }

@@ -44,23 +44,29 @@ __host__ __device__ __forceinline__ dd dd_sqrt(dd a)
     return quick_sum(r, (fma(-r, r, a.h) + a.l) / (2.0 * r));
 }
 
-// P[a][a][b] = sqrt(binomial(2a, a - b)) 2^-a, a >= b >= 0. The binomial passes the double range from a = 511
-// on (its largest, times the next factor, 2^1025.7); an even power of two taken out on the way keeps every step
-// in range and the digits as they are.
-__host__ __device__ __forceinline__ dd delta_seed(int a, int b)
+// P[a][a][b] = sqrt(binomial(2a, a - b)) 2^-a, a >= b >= 0, the binomial as eight partial products of every
+// eighth factor (2a - q) / (q + 1), q < a - b, which are all at least 1: no product in between passes the
+// whole, 2^1016.7 at a = 511 (one long product, multiplied before it is divided, passes the double range
+// there).
+constexpr int kSeedParts = 8;
+__host__ __device__ __forceinline__ dd seed_part(int a, int b, int first)
 {
     dd c = {1.0, 0.0};
-    int e = 0;
-    for (int q = 0; q < a - b; ++q) {
-        c = dd_div(dd_scale(c, (double)(2 * a - q)), dd{(double)(q + 1), 0.0});
-        if (c.h >= 0x1p600) {
-            c.h *= 0x1p-600;
-            c.l *= 0x1p-600;
-            e += 300;   // of the square root
-        }
-    }
-    c = dd_sqrt(c);
-    return {ldexp(c.h, e - a), ldexp(c.l, e - a)};
+    for (int q = first; q < a - b; q += kSeedParts) c = dd_div(dd_scale(c, (double)(2 * a - q)), dd{(double)(q + 1), 0.0});
+    return c;
+}
+__host__ __device__ __forceinline__ dd seed_of(dd binomial, int a)
+{
+    const dd r = dd_sqrt(binomial);
+    return {ldexp(r.h, -a), ldexp(r.l, -a)};
+}
+inline dd delta_seed(int a, int b)   // as eight lanes compute it
+{
+    dd c[kSeedParts];
+    for (int i = 0; i < kSeedParts; ++i) c[i] = seed_part(a, b, i);
+    for (int s = kSeedParts / 2; s > 0; s /= 2)
+        for (int i = 0; i < s; ++i) c[i] = dd_mul(c[i], c[i + s]);
+    return seed_of(c[0], a);
 }
 
 }  // namespace pfsoft_dev

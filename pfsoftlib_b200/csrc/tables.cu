@@ -155,40 +155,58 @@ __global__ void trig_kernel(int B, double* trig)
     }
 }
 
-// P[l][a][b] for one pair a >= b per thread, l = a .. B-1, and its mirror image: the recurrence of
+// P[l][a][b] for one pair a >= b per eight lanes, l = a .. B-1, and its mirror image: the recurrence of
 // fn_dwt.hpp:167-199 at cos beta = 0 without its normalisation,
 //   P(l+1) = -((2l+1) a b P(l) + (l+1) sqrt(q(l)) P(l-1)) / (l sqrt(q(l+1))),  q(l) = (l^2-a^2)(l^2-b^2),
-// from delta_seed, in double-double arithmetic (dd.cuh), which keeps the products of two entries within
+// from the seed, in double-double arithmetic (dd.cuh), which keeps the products of two entries within
 // two ulp over any number of steps. The table starts zeroed.
+// What bounds it: the chain over l. A lane takes one of a tile's eight degrees for what does not depend on
+// the chain (the two factors with their roots and quotients, the norm), all eight run the chain, two products
+// and a sum a step. One thread per pair, roots and quotients in the chain, against this, us, cold: B = 8
+// 14.6 / 7.0, 32 43 / 15, 64 80 / 24, 128 150 / 50, 256 294 / 136, 384 466 / 399.
 __global__ void delta_kernel(int B, double* delta)
 {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    const int i = (blockIdx.x * blockDim.x + threadIdx.x) >> 3, lane = threadIdx.x & 7;
     if (i >= num_classes(B)) return;
+    const unsigned group = 0xffu << (threadIdx.x & 24);
+    auto from = [&](dd v, int src) { return dd{__shfl_sync(group, v.h, src, 8), __shfl_sync(group, v.l, src, 8)}; };
     int a, b;
     class_orders(i, a, b);
-    dd cur = delta_seed(a, b), prev = {0.0, 0.0};
+    dd cur = seed_part(a, b, lane), prev = {0.0, 0.0};
+    for (int s = kSeedParts / 2; s > 0; s /= 2)
+        cur = dd_mul(cur, dd{__shfl_xor_sync(group, cur.h, s, 8), __shfl_xor_sync(group, cur.l, s, 8)});
+    cur = seed_of(from(cur, 0), a);
     auto at = [&](int M, int n, int l) {
         const int lb = l >> 3, b0 = M >> 3;
         return delta_offset(B, M) + 64 * (long long)(lb * (lb + 1) / 2 - b0 * (b0 + 1) / 2 + (n >> 3)) + (l & 7) * 8 + (n & 7);
     };
-    dd sq = {0.0, 0.0};   // sqrt(q(l))
-    for (int l = a; l < B; ++l) {
+    auto root = [&](int l) {   // sqrt(q(l)), q an exact integer
+        const double k2 = (double)l * l;
+        return dd_sqrt(dd{(k2 - (double)a * a) * (k2 - (double)b * b), 0.0});
+    };
+    for (int l0 = a & ~7; l0 < B; l0 += 8) {
+        const int l = l0 + lane;
+        dd f1 = {0.0, 0.0}, f2 = {0.0, 0.0}, mine = {0.0, 0.0};
+        if (l >= a && l > 0) {
+            const dd inv = dd_div(dd{1.0, 0.0}, dd_scale(root(l + 1), (double)l));
+            f1 = dd_scale(inv, -(double)(2 * l + 1) * a * b);
+            f2 = dd_mul(dd_scale(root(l), -(double)(l + 1)), inv);
+        }
+#pragma unroll
+        for (int j = 0; j < 8; ++j) {
+            const dd g1 = from(f1, j), g2 = from(f2, j);
+            if (l0 + j < a) continue;
+            if (lane == j) mine = cur;
+            const dd next = dd_add(dd_mul(g1, cur), dd_mul(g2, prev));
+            prev = cur;
+            cur = next;
+        }
+        if (l < a || l >= B) continue;
         // with a fourth root of the rows' squared norm, so that a product of two has its square root
-        const dd x = dd_mul(cur, dd_sqrt(dd_sqrt(dd{l + 0.5, 0.0})));
+        const dd x = dd_mul(mine, dd_sqrt(dd_sqrt(dd{l + 0.5, 0.0})));
         const double v = x.h + x.l;
         delta[at(a, b, l)] = v;
         if (a != b) delta[at(b, a, l)] = ((a - b) & 1) ? -v : v;
-        const double k2 = (double)(l + 1) * (l + 1);
-        const double q1 = (k2 - (double)a * a) * (k2 - (double)b * b);   // an exact integer
-        const dd sn = dd_sqrt(dd{q1, 0.0});
-        dd nx = {0.0, 0.0};
-        if (l > 0) {
-            nx = dd_add(dd_scale(cur, (double)(2 * l + 1) * a * b), dd_scale(dd_mul(sq, prev), (double)(l + 1)));
-            nx = dd_div(nx, dd_scale(sn, -(double)l));
-        }
-        prev = cur;
-        cur = nx;
-        sq = sn;
     }
 }
 
@@ -241,7 +259,7 @@ cudaError_t series_tables_build(int B, void* mem, BandTables* t, cudaStream_t st
     const int threads = 64;
     cudaError_t e = cudaMemsetAsync(delta, 0, dbytes, stream);
     if (e != cudaSuccess) return e;
-    delta_kernel<<<(num_classes(B) + threads - 1) / threads, threads, 0, stream>>>(B, delta);
+    delta_kernel<<<(8 * num_classes(B) + threads - 1) / threads, threads, 0, stream>>>(B, delta);
     e = cudaGetLastError();
     if (e != cudaSuccess) return e;
     trig_kernel<<<(int)std::min<long long>((trig_entries(B) + 255) / 256, 1024), 256, 0, stream>>>(B, trig);
