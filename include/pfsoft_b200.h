@@ -74,8 +74,8 @@ int pfsoft_cuda_idsoft(const double* d_coeffs, int B, double* d_grid, void* d_wo
  * synchronisation): it makes no allocation at all and uses a scratch array that the library
  * holds in device memory from load to exit (5.83 MiB per GPU). Limit: bandwidth B <= 32; a
  * larger B returns PFSOFT_EINVAL. The first call on a device looks up that array's device
- * address: make that first call before any stream capture. The first direct call for a bandwidth builds its
- * tables in the array, where they stay; a recording made before it builds them in every replay.
+ * address: make that first call before any stream capture. The first call for a bandwidth builds its
+ * tables in the array, where they stay, beside the recording if the call is being recorded.
  * All calls on a device share the array, so calls that overlap on the GPU race; nothing in it
  * has to start at zero. Same layouts and results as pfsoft_cuda_dsoft. */
 int pfsoft_cuda_dsoft_noalloc(const double* d_grid, int B, double* d_coeffs, void* stream);

@@ -340,14 +340,6 @@ size_t grid_elems(int B)
     return N * N * N;
 }
 
-// The calling thread's capture mode is relaxed while it lives: a first call may come while a stream is
-// being captured, and allocating would invalidate the capture in the other modes.
-struct RelaxedCapture {
-    cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
-    RelaxedCapture() { cudaThreadExchangeStreamCaptureMode(&mode); }
-    ~RelaxedCapture() { cudaThreadExchangeStreamCaptureMode(&mode); }
-};
-
 // Tables for bandwidth B on the current device, each set built on first use, on a stream of its own: the
 // caller's may be under capture, and the tables belong to no recording.
 int get_tables(int B, BandTables* out, int sets = kSeriesTables)

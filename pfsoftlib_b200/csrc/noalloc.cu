@@ -16,8 +16,9 @@
 // as its first call leaves them whatever runs in between, a replayed graph among it: one place for all
 // costs three small kernels and a clear whenever the bandwidth changes, and once a call has been recorded in
 // every later call and replay (us per call, B = 16 after a recorded call 57 against 14, its replay 47
-// against 12; B = 16 and 32 in turn 144 against 35). Only a recording made before the bandwidth's first
-// direct call holds the kernels that build the tables, since the host does not see whether it is replayed.
+// against 12; B = 16 and 32 in turn 144 against 35). A recording that is the bandwidth's first call has them
+// built beside it, on the thread's own stream, and waits for them; only one made on that stream holds their
+// kernels, since the host does not see whether it is replayed.
 
 #include <cuda_runtime.h>
 
@@ -46,7 +47,7 @@ __device__ __align__(256) unsigned char g_noalloc_scratch[kSpectrumBytes + kTabl
 struct NoAllocDevice {
     bool ready;          // symbol address resolved on this device
     unsigned char* base; // device address of g_noalloc_scratch
-    bool built[kNoAllocMaxB + 1];   // a direct call has queued the bandwidth's table kernels
+    bool built[kNoAllocMaxB + 1];   // the bandwidth's table kernels are queued, and not in a recording
     BandTables tables[kNoAllocMaxB + 1];
 };
 
@@ -92,10 +93,14 @@ int pfsoft_cuda_dsoft_noalloc(const double* d_grid, int B, double* d_coeffs, voi
         size_t at = kSpectrumBytes;
         for (int b = 1; b < B; ++b) at += all_tables_bytes(b);
         if (at + all_tables_bytes(B) > sizeof(g_noalloc_scratch)) return fail(PFSOFT_EINVAL, "pfsoft_cuda_dsoft_noalloc: tables exceed the reserve");
-        if (tables_build(B, d.base + at, &d.tables[B], s) != cudaSuccess ||
-            series_tables_build(B, d.base + at + tables_bytes(B), &d.tables[B], s) != cudaSuccess)
+        RelaxedCapture relaxed;
+        const bool beside = cap != cudaStreamCaptureStatusNone && s != cudaStreamPerThread;
+        const cudaStream_t ts = beside ? cudaStreamPerThread : s;
+        if (tables_build(B, d.base + at, &d.tables[B], ts) != cudaSuccess ||
+            series_tables_build(B, d.base + at + tables_bytes(B), &d.tables[B], ts) != cudaSuccess ||
+            (beside && cudaStreamSynchronize(ts) != cudaSuccess))
             return fail(PFSOFT_ECUDA, "pfsoft_cuda_dsoft_noalloc: table kernels failed to launch");
-        d.built[B] = cap == cudaStreamCaptureStatusNone;
+        d.built[B] = beside || cap == cudaStreamCaptureStatusNone;
     }
     const BandTables& t = d.tables[B];
     const int N = 2 * B;

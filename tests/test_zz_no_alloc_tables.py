@@ -1,6 +1,6 @@
-"""pfsoft_cuda_dsoft_noalloc builds a bandwidth's tables once: a recording made after the bandwidth's first direct call
-holds its three launches and nothing that builds tables, whatever bandwidths ran in between; one made before it
-builds its own, and either gives pfsoft_cuda_dsoft's result in any order of calls and replays."""
+"""pfsoft_cuda_dsoft_noalloc builds a bandwidth's tables once: a recording holds the call's three launches and nothing
+that builds tables, whatever bandwidths ran in between and also where it is the bandwidth's first call, and
+gives pfsoft_cuda_dsoft's result in any order of calls and replays."""
 import ctypes
 
 import numpy as np
@@ -72,3 +72,14 @@ def test_recording_before_the_first_direct_call(lib):
         small.check(small.call)
         a.check(ga.replay)
         b.check(b.call)
+
+
+@pytest.mark.parametrize("B", [11, 29])   # no other test's bandwidths
+def test_first_call_in_a_recording_builds_beside_it(lib, B):
+    small, case = _Case(lib, 2), _Case(lib, B)
+    small.check(small.call)   # the device's first call
+    graph = case.record(torch.cuda.CUDAGraph(keep_graph=True))
+    assert _nodes(graph) <= 3
+    small.check(small.call)
+    case.check(graph.replay)
+    case.check(case.call)
