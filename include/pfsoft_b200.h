@@ -284,8 +284,9 @@ int pfsoft_tune_dwt_case_split(int direction, int case_split);
 int pfsoft_tune_fft_fused(int B, int on);
 /* Tuning knob: whether a plan created with PFSOFT_BATCH_SPLIT runs bandwidth B's DWT on the split
  * kernel (use_split != 0) or on the FP64 kernels (0). B <= 0: every bandwidth, clearing the
- * per-bandwidth choices; use_split != 0 then is the default, the faster form for each bandwidth and
- * number of transforms. Set by the autotuner; read when a plan is created. */
+ * per-bandwidth choices; use_split 2 is the split kernel wherever it is supported, any other value but 0 the
+ * default, the faster form for each bandwidth and number of transforms. Set by the autotuner; read when a
+ * plan is created. */
 int pfsoft_tune_split_bandwidth(int B, int use_split);
 /* Test knob for the split-precision DWT's failure path (no counterpart in the reference): when
  * wait_ns > 0, every later split launch first waits up to wait_ns nanoseconds on a barrier that

@@ -28,10 +28,10 @@ using namespace pfsoft_dev;
 
 namespace {
 
-// The split-precision choice per bandwidth (0 default, 1 split, -1 FP64) and of the rest (default or
-// FP64), read when a PFSOFT_BATCH_SPLIT plan is created.
+// The split-precision choice per bandwidth (0 that of the rest, 1 split, -1 FP64) and of the rest (0 FP64, 1 the
+// faster form, 2 split), read when a PFSOFT_BATCH_SPLIT plan is created.
 signed char g_split_choice[513] = {};
-bool g_split_all = true;
+int g_split_rest = 1;
 
 // Default: the faster DWT for T transforms of bandwidth B. The FP64 kernels' sums over the series take
 // fewer steps than the split kernel's digit products; only without a DFT over beta, whose matrix product
@@ -45,7 +45,7 @@ bool split_faster(int B, int T) { return B <= 16 || (B >= 140 && T >= 2 && !dwt_
 bool split_wanted(int B, int T)
 {
     if (B >= 1 && B <= 512 && g_split_choice[B]) return g_split_choice[B] > 0;
-    return g_split_all && split_faster(B, T);
+    return g_split_rest == 2 || (g_split_rest == 1 && split_faster(B, T));
 }
 
 __global__ void zero_nyquist_batched(double2* const* X, int B)
@@ -375,7 +375,7 @@ int pfsoft_tune_split_bandwidth(int B, int use_split)
 {
     if (B > 512) return fail(PFSOFT_EINVAL, "bandwidth must be at most 512");
     if (B <= 0) {
-        g_split_all = use_split != 0;
+        g_split_rest = use_split == 2 ? 2 : use_split != 0;
         for (auto& v : g_split_choice) v = 0;
     } else {
         g_split_choice[B] = use_split ? 1 : -1;
