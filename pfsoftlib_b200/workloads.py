@@ -4,7 +4,8 @@ example). ``python -m pfsoftlib_b200.workloads <name> [reps]``:
   single-<B>      IDSOFT then DSOFT of one transform at bandwidth B (PCG64-seeded inputs)
   batch-<B>x<T>   a batch plan of T transforms at bandwidth B, IDSOFT then DSOFT
   mixed           256 transforms, B uniform over {32,48,64,96,128} (seed 2), batched
-  <name>-split    a batch or mixed workload through the split-precision tensor-core DWT
+  <name>-split    a batch or mixed workload through the split-precision tensor-core DWT at every bandwidth
+                  (pfsoft_tune_split_bandwidth, restored to the default afterwards)
   <name>-fusedfft any of the above with pfsoft_tune_fft_fused on (without effect in the present
                   passes), restored to the default afterwards
   shard-<B>x<P>   IDSOFT then DSOFT of one transform sharded over P ranks, the ranks run one after
@@ -63,7 +64,11 @@ def run(name: str, reps: int = 1) -> float:
         fs = [torch.empty_like(c) for c in cs]
         plan = ctypes.c_void_p()
         arr = (ctypes.c_int * len(bws))(*bws)
-        assert lib.pfsoft_batch_create(arr, len(bws), 0, 1 | (2 if split else 0), ctypes.byref(plan)) == 0
+        lib.pfsoft_tune_split_bandwidth(0, 2)
+        try:
+            assert lib.pfsoft_batch_create(arr, len(bws), 0, 1 | (2 if split else 0), ctypes.byref(plan)) == 0
+        finally:
+            lib.pfsoft_tune_split_bandwidth(0, 1)
         cp = (ctypes.c_void_p * len(bws))(*[t.data_ptr() for t in cs])
         gp = (ctypes.c_void_p * len(bws))(*[t.data_ptr() for t in gs])
         fp = (ctypes.c_void_p * len(bws))(*[t.data_ptr() for t in fs])
