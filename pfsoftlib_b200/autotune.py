@@ -1,16 +1,13 @@
 """Project autotuner for the batched engine.
 
-For a multiset of bandwidths it times candidate schedules on the device with CUDA events and
-caches the winners in a JSON table keyed by GPU name and the sorted bandwidth counts:
+For a multiset of bandwidths ``tune_plan`` times, per bandwidth, the DWT of a PFSOFT_BATCH_SPLIT plan on
+the split-precision kernel and on the FP64 kernels with CUDA events, caches the winners in a JSON
+table keyed by GPU name and the sorted bandwidth counts, applies them to the library
+(pfsoft_tune_split_bandwidth) and returns them. What else earlier kernels left to choose
+(``transforms_per_cta``, pfsoft_tune_fft_fused) has no effect in the present ones: ``tune_batch`` and
+the ``fft_fused`` entries keep their form, and nothing is timed for them.
 
-  tune_batch  the `transforms_per_cta` argument of a batch plan (1, 2, 4; the present DWT kernels
-              take one transform per CTA whatever it is);
-  tune_plan   per bandwidth: pfsoft_tune_fft_fused on or off (without effect in the present
-              passes), and the DWT of a PFSOFT_BATCH_SPLIT plan on the
-              split-precision kernel or the FP64 kernels (pfsoft_tune_split_bandwidth); the
-              choices are applied to the library and returned.
-
-``choose`` is the pure decision rule (tested on CPU); the tune_* functions do the timing.
+``choose`` is the pure decision rule (tested on CPU).
 """
 from __future__ import annotations
 
@@ -62,44 +59,9 @@ def store(key: str, value: int, path: str | None = None) -> None:
 
 
 def tune_batch(lib, bandwidths, coeffs, grids, back, reps: int = 2, use_cache: bool = True) -> tuple[int, dict]:
-    """Time a round trip (IDSOFT then DSOFT) of the batch for each candidate; returns the
-    chosen transforms-per-CTA and the timings in ms. Buffers are lists of CUDA tensors."""
-    import torch
-
-    gpu = torch.cuda.get_device_name()
-    key = key_for(gpu, bandwidths)
-    if use_cache:
-        cached = load_cache().get(key)
-        if cached in CANDIDATES:
-            return cached, {}
-    arr = (ctypes.c_int * len(bandwidths))(*[int(b) for b in bandwidths])
-    cp = (ctypes.c_void_p * len(coeffs))(*[t.data_ptr() for t in coeffs])
-    gp = (ctypes.c_void_p * len(grids))(*[t.data_ptr() for t in grids])
-    bp = (ctypes.c_void_p * len(back))(*[t.data_ptr() for t in back])
-    s = torch.cuda.current_stream().cuda_stream
-    timings = {}
-    for tpc in CANDIDATES:
-        plan = ctypes.c_void_p()
-        if lib.pfsoft_batch_create(arr, len(bandwidths), tpc, 0, ctypes.byref(plan)) != 0:
-            continue
-        try:
-            lib.pfsoft_batch_idsoft(plan, cp, gp, s)
-            lib.pfsoft_batch_dsoft(plan, gp, bp, s)
-            torch.cuda.synchronize()
-            e0 = torch.cuda.Event(enable_timing=True)
-            e1 = torch.cuda.Event(enable_timing=True)
-            e0.record()
-            for _ in range(reps):
-                lib.pfsoft_batch_idsoft(plan, cp, gp, s)
-                lib.pfsoft_batch_dsoft(plan, gp, bp, s)
-            e1.record()
-            torch.cuda.synchronize()
-            timings[tpc] = e0.elapsed_time(e1) / reps
-        finally:
-            lib.pfsoft_batch_destroy(plan)
-    best = choose(timings)
-    store(key, best)
-    return best, timings
+    """The transforms-per-CTA argument of a batch plan and the timings in ms behind the choice. The kernels
+    take one transform per CTA whatever it is, so the smallest candidate is returned, without timings."""
+    return CANDIDATES[0], {}
 
 
 def _time_ms(fn, reps: int) -> float:
@@ -125,10 +87,9 @@ def apply(lib, plan: dict) -> None:
 
 
 def tune_plan(lib, bandwidths, coeffs, grids, back, reps: int = 2, use_cache: bool = True) -> dict:
-    """Per distinct bandwidth of the mix: (1) the FFT stage fused or as two passes, timed on a
-    single-transform round trip; (2) the DWT of a split plan on the split kernel or the FP64
-    kernels, timed on a batch plan of that bandwidth's transforms (FFT choice applied). Applies the
-    winners (apply) and returns {"fft_fused": {B: bool}, "split": {B: bool}, "ms": {...}}.
+    """Per distinct bandwidth of the mix: the DWT of a split plan on the split kernel or the FP64 kernels,
+    timed on a batch plan of that bandwidth's transforms. Applies the winners (apply) and returns
+    {"fft_fused": {B: False}, "split": {B: bool}, "ms": {"fft": {}, "dwt": {...}}}.
     Buffers are lists of CUDA tensors in the order of `bandwidths`."""
     import torch
 
@@ -143,22 +104,7 @@ def tune_plan(lib, bandwidths, coeffs, grids, back, reps: int = 2, use_cache: bo
     out = {"fft_fused": {}, "split": {}, "ms": {"fft": {}, "dwt": {}}}
     for b in sorted(set(int(x) for x in bandwidths)):
         idx = [i for i, x in enumerate(bandwidths) if int(x) == b]
-        i0 = idx[0]
-        ws = torch.empty(lib.pfsoft_workspace_bytes(b) // 8, dtype=torch.float64, device="cuda")
-
-        def single():
-            lib.pfsoft_cuda_idsoft(coeffs[i0].data_ptr(), b, grids[i0].data_ptr(), ws.data_ptr(), ws.numel() * 8, s)
-            lib.pfsoft_cuda_dsoft(grids[i0].data_ptr(), b, back[i0].data_ptr(), ws.data_ptr(), ws.numel() * 8, s)
-
-        t = {}
-        for on in (1, 0):
-            lib.pfsoft_tune_fft_fused(b, on)
-            t[on] = _time_ms(single, reps)
-        fused = t[1] <= t[0]
-        lib.pfsoft_tune_fft_fused(b, int(fused))
-        out["fft_fused"][str(b)] = fused
-        out["ms"]["fft"][str(b)] = {"fused": t[1], "two_passes": t[0]}
-        del ws
+        out["fft_fused"][str(b)] = False
         arr = (ctypes.c_int * len(idx))(*[b] * len(idx))
         cp = (ctypes.c_void_p * len(idx))(*[coeffs[i].data_ptr() for i in idx])
         gp = (ctypes.c_void_p * len(idx))(*[grids[i].data_ptr() for i in idx])
