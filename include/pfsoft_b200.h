@@ -16,10 +16,11 @@
  *           2l+1+M -- the storage of DSOFTFourierCoefficients
  *           (src/dsoft_fourier_coefficients.cpp:48-57, :80-89), packed contiguously.
  *
- * First use of a bandwidth on a device builds its constant tables (one cudaMalloc and a few
- * small kernels, then a stream synchronisation); make that first call before any stream
- * capture. Later calls for the same bandwidth allocate nothing. The tables stay until exit:
- * about 11 MB at B = 128, 77 MB at B = 256, 575 MB at B = 512 per bandwidth and device.
+ * The first use of a bandwidth on a device builds the constant tables it needs (a few allocations and
+ * small kernels on a stream of the library's own, then a wait for them), also where the call is being
+ * recorded into a CUDA graph: they are built beside the recording. Later calls of the same kind allocate
+ * nothing. The tables stay until exit: about 6 MB at B = 128, 48 MB at B = 256, 371 MB at B = 512 per
+ * bandwidth and device for the FP64 transforms; the split kernel's 11 MB at B = 128, 77 MB at 256.
  */
 #ifndef PFSOFT_B200_H
 #define PFSOFT_B200_H
@@ -287,7 +288,8 @@ long long pfsoft_launch_count(void);
  * values are checked; the present kernels have one form for all symmetry cases. */
 int pfsoft_tune_dwt_case_split(int direction, int case_split);
 /* Tuning knob of an earlier form (both FFT passes of a direction in one launch), for bandwidth B (B <= 0:
- * every bandwidth). The bandwidth is checked; the passes always run as two launches. */
+ * every bandwidth). The bandwidth is checked and the knob has no effect: both passes are one launch for the
+ * small even lengths where that is faster (single transforms up to N = 48, batches up to 32), two for all others. */
 int pfsoft_tune_fft_fused(int B, int on);
 /* Tuning knob: whether a plan created with PFSOFT_BATCH_SPLIT runs bandwidth B's DWT on the split
  * kernel (use_split != 0) or on the FP64 kernels (0). B <= 0: every bandwidth, clearing the

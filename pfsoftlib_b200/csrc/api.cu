@@ -278,6 +278,8 @@ DeviceState* device_state(int dev)
 }
 
 // ---- launch accounting and optional per-stage timing ------------------------------------
+// A small transform's one FFT launch counts as the first pass of its direction; the two fused stages are of an
+// earlier form, kept for the stages' numbers.
 enum Stage { ST_FFT_FWD_ROWS, ST_FFT_FWD_COLS, ST_DWT_FWD, ST_NYQUIST, ST_DWT_INV, ST_FFT_INV_COLS, ST_FFT_INV_ROWS,
              ST_TABLES, ST_FFT_FWD_FUSED, ST_FFT_INV_FUSED, ST_COUNT };
 const char* kStageNames[ST_COUNT] = {"fft_forward_gamma", "fft_forward_alpha", "dwt_forward", "zero_nyquist",
@@ -877,7 +879,7 @@ long long pfsoft_launch_count(void) { return g_launches.load(); }
 int pfsoft_tune_fft_fused(int B, int on)
 {
     if (B > kMaxBandwidth) return fail(PFSOFT_EINVAL, "bandwidth must be at most 512");
-    (void)on;   // both passes in one launch was never the faster form; the knob has no effect any more
+    (void)on;   // of an earlier form of both passes in one launch; fft_plane_supported decides now
     return PFSOFT_OK;
 }
 

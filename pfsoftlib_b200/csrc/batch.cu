@@ -38,8 +38,9 @@ int g_split_rest = 1;
 // grows as B^4, and with pairs of transforms to share the split kernel's Wigner tiles, the split kernel
 // is ahead from about B = 140 on. Whole plans, split over FP64, iDSOFT / DSOFT: B = 32 (T = 4) 2.0 / 2.5, 64 1.4 /
 // 1.6, 128 1.3 / 1.3, 256 1.1 / 1.2; without DFT and T >= 2: 116 1.1, 137 1.0, 166 0.98, 184 0.94, 251
-// 0.92, T = 1: 1.1 and more. Up to B = 16, where calls of a few transforms are bound by their launches, the split kernel
-// stays although FP64 is 5 to 15 us ahead: it is the one whose failure is reported by pfsoft_batch_status.
+// 0.92, T = 1: 1.1 and more. Up to B = 16, where calls of a few transforms are bound by their launches, the rule
+// does not follow the times (FP64 is 5 to 15 us ahead): split plans run there what they always ran, and with
+// it the bounded waits whose failure pfsoft_batch_status reports in plans made without a tuning call.
 bool split_faster(int B, int T) { return B <= 16 || (B >= 140 && T >= 2 && !dwt_has_dft(2 * B)); }
 
 bool split_wanted(int B, int T)

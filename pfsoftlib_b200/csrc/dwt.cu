@@ -36,7 +36,9 @@
 // one barrier. Measured, MMA form against DFT, us forward / inverse: N = 96 17 / 18 against 19 / 19,
 // 98 25 / 26 against 20 / 22, 128 33 / 33 against 29 / 29, 168 70 / 77 against 60 / 64, 224 168 / 168
 // against 126 / 123, 272 428 / 434 against 309 / 300, 360 956 / 1007 against 699 / 664, 480 2699 / 2658
-// against 1602 / 1628; the radices 17 and 19 at N = 114 and 152 break even, 23 spills. Two large
+// against 1602 / 1628; the radices 17 and 19 at N = 114 and 152 break even, 23 spills. The register caps cost some
+// kernels a little too: 8 to 80 bytes of spills in the forward sums at four tile columns per warp (60 at N = 256, 64 at
+// 512, 80 in the MMA form up to B = 256). Two large
 // radices beat three small ones (N = 240 16.15 152 / 152 against 16.3.5 160 / 168).
 //
 // One CTA per item, a class of one transform; longest classes first.
@@ -203,8 +205,8 @@ __device__ __forceinline__ int case_index(int i1, int i2, int l)
     return (int)((unsigned)(l * (4 * l * l - 1)) / 3u) + (i2 < 0 ? i2 + L : i2) * L + (i1 < 0 ? i1 + L : i1);
 }
 
-// The launch's items: every class (of the list) of every transform, a class's transforms side by side,
-// longest classes first; a CTA takes every gridDim.x-th.
+// The launch's items, one per CTA: every class (of the list) of every transform, a class's transforms side by
+// side, longest classes first.
 struct Item {
     int M, Mp, nc, odd, tr;
     int rev;           // bit c: case c is read at pi - beta
@@ -726,10 +728,10 @@ cudaError_t launch(K kernel, In in, Out out, int threads, size_t smem, size_t la
 {
     DwtArgs b = a;
     b.T = T;
-    b.items = (a.classes ? a.n_classes : num_classes(a.B)) * T;
+    const int items = (a.classes ? a.n_classes : num_classes(a.B)) * T;
     const cudaError_t e = allow_shared(kernel, smem, largest);
     if (e != cudaSuccess) return e;
-    kernel<<<b.items, threads, smem, s>>>(in, out, b);
+    kernel<<<items, threads, smem, s>>>(in, out, b);
     return cudaGetLastError();
 }
 
@@ -812,6 +814,13 @@ LaunchFn fixed_launch_for(int N)
 cudaError_t dispatch(int dir, const double2* X, double2* coeffs, const DwtArgs& a, int T, cudaStream_t s)
 {
     if (const LaunchFn fixed = fixed_launch_for(a.N)) return fixed(dir, X, coeffs, a, T, s);
+    // The MMA form: warps, tile columns per warp (NW KP blocks of 8 in all: the bandwidth's), CTAs per SM. Few
+    // warps keep short classes' warps busy, eight hide more where the CTA's shared memory allows two only. Measured, us
+    // forward / inverse, this against the best other: B = 16 8.5 / 8.6 (all shapes), 32 10.6 / 10.6 (4 warps the same), 33
+    // 11.3 / 12.6 (2 warps of 3, 12.6 / 12.6), 40 15.4 / 17.0 (the same, 12.7 / 12.8), 48 16.7 / 16.8 (the same, 14.7 / 16.7), 64
+    // 31 / 31 (4 of 2, 29 / 33), 67 41 / 44 (six CTAs, 39 / 41), 96 93 / 97 (six, 100 / 97), 127 260 / 233 (8 of 2, 242 / 249), 137
+    // 453 / 443 (three CTAs, 387 / 397), 191 1113 / 1127 (three, 1080 / 1058), 193 1457 / 1437 (three, 1477 / 1455), 251
+    // 3183 / 3086 (three, 3327 / 3166). So the lines at 40 and 192 are not the best there are.
     if (a.B <= 16) return launch_mma<2, 1, 12>(dir, X, coeffs, a, T, s);
     if (a.B <= 32) return launch_mma<2, 2, 12>(dir, X, coeffs, a, T, s);
     if (a.B <= 40) return launch_mma<4, 2, 5>(dir, X, coeffs, a, T, s);

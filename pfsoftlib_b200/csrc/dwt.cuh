@@ -88,7 +88,7 @@ struct DwtArgs {
     // Several transforms of one bandwidth: device tables of their spectra and coefficients
     double2* const* Xs;
     double2* const* coefs;
-    int T, items;   // set by the launch
+    int T;   // set by the launch
     // Inverse only: also zero the Nyquist bins (row B or column B of X, which no order class
     // writes) in the kernel's tail, instead of a separate launch.
     int zero_nyquist;

@@ -4,8 +4,11 @@
 //   fft_two.cu         n = ra rb with register butterflies up to 32: one shared-memory exchange
 //   fft_matrix.cu      n = R p, p odd and 17 .. 249: a matrix product on the FP64 MMA
 //   fft_chirp_kernel   n with a larger prime, or one with too many other factors: Bluestein's convolution
-//   fft_pass_kernel    what is left (n below 4, 5, 7, 11 and 13, lengths such as 343, n above 1024):
-//                      mixed-radix Stockham autosort (Govindaraju et al., SC'08 formulation). A stage of
+//   fft_pass_kernel    what is left: n up to 7, 9, 11 and 13; products of 2, 3, 5, 7, 11 and 13 that no two factors
+//                      up to 32 make, such as 243, 343, 486 and 648; odd n of 513 and more with a prime that the
+//                      matrix pass does not take (521: direct O(R^2) stages, no table is kept for odd lengths
+//                      and the chirp pass ends at 512); such n above 1024. Mixed-radix Stockham autosort
+//                      (Govindaraju et al., SC'08 formulation). A stage of
 //     radix R over n points with Ns = product of the earlier radices maps butterfly j to
 //       inputs  x[j + r*n/R] * w_n^(r * (j mod Ns) * n/(Ns R)),   r < R
 //       outputs y[(j/Ns)*Ns*R + (j mod Ns) + q*Ns],              q < R
