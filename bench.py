@@ -395,6 +395,12 @@ def mixed_section(lib, steps: int, warmup: int, tune: bool = False) -> dict:
     split_grid_vs = max(_rel(grids[i], g64[i]) for i in range(len(bws)))
     split_coef_vs = max(_rel(back[i], c64[i]) for i in range(len(bws)))
     split_rt = max(_rel(back[i], coeffs[i]) for i in range(len(bws)))
+    # the split plan's first B = 32 transform against the oracle (long double, all on the host)
+    i32 = bws.index(32)
+    ora = orc.Oracle()
+    g_h = grids[i32].cpu().numpy()
+    oracle_grid = orc.rel_l2(g_h, ora.idsoft(coeffs[i32].cpu().numpy(), 32))
+    oracle_coef = orc.rel_l2(back[i32].cpu().numpy(), ora.dsoft(g_h))
     # the autotuned plan: per bandwidth, the DWT split or FP64
     tuned = autotune.tune_plan(lib, bws, coeffs, grids, back, use_cache=False)
     ptu = _Plan(lib, bws, SPLIT)
@@ -404,13 +410,6 @@ def mixed_section(lib, steps: int, warmup: int, tune: bool = False) -> dict:
     tuned_vs = max(_rel(back[i], c64[i]) for i in range(len(bws)))
     lib.pfsoft_tune_fft_fused(0, 0)        # back to the defaults for what follows
     lib.pfsoft_tune_split_bandwidth(0, 1)
-    # the oracle on the first B = 32 transform (long double, all on the host)
-    i32 = bws.index(32)
-    ora = orc.Oracle()
-    c_h = coeffs[i32].cpu().numpy()
-    g_h = grids[i32].cpu().numpy()
-    oracle_grid = orc.rel_l2(g_h, ora.idsoft(c_h, 32))
-    oracle_coef = orc.rel_l2(back[i32].cpu().numpy(), ora.dsoft(g_h))
     # the split-precision server, saturated: all 512 requests at once, fresh outputs
     out_g = [torch.empty_like(g) for g in grids]
     out_c = [torch.empty_like(c) for c in coeffs]
