@@ -39,6 +39,21 @@ def sources() -> list[str]:
     return sorted(glob.glob(os.path.join(CSRC, "*.cu")) + glob.glob(os.path.join(CSRC, "*.cpp")))
 
 
+# sources compiled several times, once for each part that they define (a module of its own each)
+PARTS = {"dwt_fixed.cu": ("DWT_PART", 13),   # kFixedParts in dwt.cuh
+         "fft_two_kind.cu": ("FFT_KIND", 7)}   # kKinds in fft_two.cuh
+
+
+def units() -> list[tuple[str, str, list[str]]]:
+    """(source, object name, extra flags) of every compilation."""
+    out = []
+    for src in sources():
+        name = os.path.basename(src)
+        macro, n = PARTS.get(name, ("", 1))
+        out += [(src, f"{name}.{i}.o" if macro else f"{name}.o", [f"-D{macro}={i}"] if macro else []) for i in range(n)]
+    return out
+
+
 def up_to_date() -> bool:
     if not os.path.exists(LIB):
         return False
@@ -56,9 +71,9 @@ def build(force: bool = False, verbose: bool = False, extra: list[str] | None = 
     os.makedirs(objdir, exist_ok=True)
     objs = []
     procs = []
-    for src in sources():
-        obj = os.path.join(objdir, os.path.basename(src) + ".o")
-        cmd = [nvcc(), *host_compiler(), *ARCH, *NVCC_FLAGS, *(extra or []), "-I", os.path.join(ROOT, "include"),
+    for src, name, flags in units():
+        obj = os.path.join(objdir, name)
+        cmd = [nvcc(), *host_compiler(), *ARCH, *NVCC_FLAGS, *flags, *(extra or []), "-I", os.path.join(ROOT, "include"),
                "-c", src, "-o", obj]
         if verbose:
             print(" ".join(cmd))

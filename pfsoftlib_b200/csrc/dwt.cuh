@@ -97,6 +97,18 @@ struct DwtArgs {
 // Arguments of the DWT launches over every order class of a bandwidth's tables.
 DwtArgs dwt_args_for(const BandTables& t);
 
+// A launch of direction 0 (forward) or 1: of T transforms of one length.
+typedef cudaError_t (*DwtLaunch)(int dir, const double2* X, double2* coeffs, const DwtArgs& a, int T, cudaStream_t stream);
+
+// The even lengths that may have a compile-time DFT over beta (dwt_fixed.cu), in parts of kFixedSpan that are
+// compiled by themselves, part by part; null for a length without one.
+constexpr int kFixedFirst = 98, kFixedLast = 512, kFixedSpan = 32;
+constexpr int kFixedParts = (kFixedLast - kFixedFirst) / kFixedSpan + 1;
+template <int PART>
+struct DwtFixedPart {
+    static DwtLaunch launch(int N);
+};
+
 // T transforms (T > 1: a.Xs and a.coefs; X and coeffs are then unused).
 // Forward: X (beta-innermost spectrum, N^3) -> packed coefficients, scale pi/(2B^2).
 // Whether the columns of length N have a compile-time DFT over beta (dwt.cu) instead of a matrix product.

@@ -1,6 +1,6 @@
 // Device building blocks of the DFT kernels: register butterflies (radix 2 .. 32), the
 // twiddle table access, and the padded shared-memory position of an element. Shared by the grid's FFT
-// passes (fft.cu) and the beta transforms of the discrete Wigner transform (dwt.cu).
+// passes (fft.cu, fft_two_kind.cu, fft_matrix.cu) and the beta transforms of the discrete Wigner transform (dwt_fixed.cu).
 #pragma once
 
 #include "common.cuh"

@@ -19,144 +19,17 @@
 // CTAs per SM measured faster (N = 320 199 us against 230), from 28 on eight (N = 512 885 against 1000).
 
 #include <algorithm>
-#include <type_traits>
 
 #include "common.cuh"
 #include "fft.cuh"
 #include "fft_core.cuh"
+#include "fft_two.cuh"
 
 namespace pfsoft_dev {
 
 namespace {
 
 using namespace fftk;
-
-// Vectors of a tile are this far apart in shared memory: 8 vectors (or 4 vectors x 2 butterflies) of one
-// access meet distinct 16-byte banks.
-__host__ __device__ __forceinline__ int block_pitch(int ra, int rb, int kb)
-{
-    const int len = rb * (ra | 1);
-    return kb == 8 ? (len | 1) : len + (10 - len % 8) % 8;
-}
-
-// butterfly t of a stage with m butterflies per vector: its vector and index
-__device__ __forceinline__ void place(bool across, int t, int lg, int m, unsigned inv, int& kk, int& j)
-{
-    if (across) {
-        kk = t & ((1 << lg) - 1);
-        j = t >> lg;
-    } else {
-        kk = m == 1 ? t : (int)__umulhi((unsigned)t, inv);   // t / m
-        j = t - kk * m;
-    }
-}
-
-template <int SIGN, int R>
-__device__ __forceinline__ void stage_one(const FftPassArgs& a, const double2* src, double2* smem, int nv, int lg, int vp)
-{
-    const int m = a.n / R, pitch = R | 1;
-    const bool across = a.src.se != 1;
-    const unsigned inv = 0xffffffffu / (unsigned)m + 1u;
-    for (int t = threadIdx.x; t < m << lg; t += blockDim.x) {
-        int kk, j;
-        place(across, t, lg, m, inv, kk, j);
-        if (kk >= nv) continue;
-        const double2* p = src + (long long)kk * a.src.sv + (long long)j * a.src.se;
-        const long long step = (long long)m * a.src.se;
-        double2 v[R];
-#pragma unroll
-        for (int r = 0; r < R; ++r) v[r] = __ldg(p + r * step);
-        butterfly<SIGN, R>(v);
-        double2* o = smem + kk * vp + j * pitch;
-#pragma unroll
-        for (int q = 0; q < R; ++q) o[q] = v[q];
-    }
-}
-
-template <int SIGN, int R>
-__device__ __forceinline__ void stage_two(const FftPassArgs& a, double2* dst, const double2* smem, int nv, int lg, int vp)
-{
-    const int m = a.n / R, pitch = m | 1;
-    const bool across = a.dst.se != 1;
-    const unsigned inv = 0xffffffffu / (unsigned)m + 1u;
-    const double2* tw = a.twiddle + a.n;
-    for (int t = threadIdx.x; t < m << lg; t += blockDim.x) {
-        int kk, j;
-        place(across, t, lg, m, inv, kk, j);
-        if (kk >= nv) continue;
-        const double2* o = smem + kk * vp + j;
-        double2 v[R];
-        v[0] = o[0];
-#pragma unroll
-        for (int r = 1; r < R; ++r) {
-            double2 w = __ldg(tw + (r - 1) * m + j);
-            if (SIGN > 0) w.y = -w.y;
-            v[r] = cmul(o[r * pitch], w);
-        }
-        butterfly<SIGN, R>(v);
-        double2* p = dst + (long long)kk * a.dst.sv + (long long)j * a.dst.se;
-        const long long step = (long long)m * a.dst.se;
-#pragma unroll
-        for (int q = 0; q < R; ++q) __stcs(p + q * step, cscale(v[q], a.scale));   // evict-first: next read from HBM
-    }
-}
-
-// The kernels: 0 for radices up to 16, 1 up to 26, 2 up to 30, 4 and 5 up to 26 and 32 with the primes from
-// 17 on (23 only in 5: its sums would spill in 4), 3 and 6 for 16.32, 32.32 and 16.16 alone, so that no length
-// pays the registers or the code of a radix that it does not need (us per pass: N = 256 in kernel 0 93.2,
-// alone 88.9; 512 with the primes 913, without 885, alone 853). CTAs per SM: up to 16 five are faster than four (N =
-// 128 21.2 against 23.1, 192 44.8 against 47.3, 240 78.2 against 80.7; not for 16.16), up to 30 three
-// faster than two (N = 448 545 against 653), at 32 two (N = 512 885 against 947).
-constexpr int kKinds = 7;
-constexpr int kMaxRadix[kKinds] = {16, 26, 30, 32, 26, 32, 16}, kBlocks[kKinds] = {5, 4, 3, 2, 4, 2, 4};
-constexpr bool is_prime17(int r) { return r == 17 || r == 19 || r == 23 || r == 29 || r == 31; }
-constexpr bool has_radix(int kind, int r)
-{
-    if (kind == 3 || kind == 6) return r == 16 || (kind == 3 && r == 32);
-    return r >= (kind == 1 ? 7 : (kind == 2 ? 14 : 2)) && r <= kMaxRadix[kind] && r != 27 &&
-           (kind == 4 || kind == 5 || !is_prime17(r)) && (kind != 4 || r != 23);
-}
-constexpr int kind_of(int ra, int rb)
-{
-    if (ra == 16 && rb == 16) return 6;
-    for (int kind = 0; kind < kKinds; ++kind)
-        if (has_radix(kind, ra) && has_radix(kind, rb)) return kind;
-    return -1;
-}
-
-// f.template run<R>() for the kernel's radix R == r
-template <int KIND, int R, class Fn>
-__device__ __forceinline__ void with_radix(int r, const Fn& f)
-{
-    if constexpr (R <= kMaxRadix[KIND]) {
-        if constexpr (has_radix(KIND, R)) {
-            if (r == R) {
-                f(std::integral_constant<int, R>());
-                return;
-            }
-        }
-        with_radix<KIND, R + 1>(r, f);
-    }
-}
-
-template <int SIGN, int KIND>
-__global__ void __launch_bounds__(128, kBlocks[KIND])
-    fft_two_kernel(const double2* src, double2* dst, const __grid_constant__ FftPassArgs a)
-{
-    extern __shared__ double2 smem[];
-    if (a.srcs) {
-        src = a.srcs[blockIdx.z];
-        dst = a.dsts[blockIdx.z];
-    }
-    const int v0 = blockIdx.x * a.kb;
-    const int nv = min(a.kb, a.nvec - v0), lg = a.kb == 8 ? 3 : 2;
-    const int vp = block_pitch(a.radix[0], a.radix[1], a.kb);
-    src += (long long)v0 * a.src.sv + (long long)blockIdx.y * a.src.sb;
-    dst += (long long)v0 * a.dst.sv + (long long)blockIdx.y * a.dst.sb;
-    with_radix<KIND, 2>(a.radix[0], [&](auto R) { stage_one<SIGN, decltype(R)::value>(a, src, smem, nv, lg, vp); });
-    __syncthreads();   // in place: every input of the tile has been read
-    with_radix<KIND, 2>(a.radix[1], [&](auto R) { stage_two<SIGN, decltype(R)::value>(a, dst, smem, nv, lg, vp); });
-}
 
 // ---- both passes of small planes ------------------------------------------------------------------
 // One CTA transforms a whole beta layer, N x N points in shared memory: four stages in place between
@@ -305,26 +178,14 @@ int fft_two_vectors(int n)
 
 cudaError_t fft_two_launch(const double2* src, double2* dst, const FftPassArgs& a, int ntiles, int sign, cudaStream_t stream, int nz)
 {
-    const int ra = a.radix[0], rb = a.radix[1];
-    const int kind = kind_of(ra, rb);
-    const size_t smem = (size_t)a.kb * block_pitch(ra, rb, a.kb) * sizeof(double2);
-    const int top = kMaxRadix[kind < 0 ? 0 : kind];
-    const size_t largest = (size_t)8 * block_pitch(top, top, 8) * sizeof(double2);   // the kind's largest radices
-    const int threads = std::min(128, (a.kb * rb + 31) / 32 * 32);
-    auto go = [&](auto k) -> cudaError_t {
-        const cudaError_t e = allow_shared(k, smem, largest);
-        if (e != cudaSuccess) return e;
-        k<<<dim3((a.nvec + a.kb - 1) / a.kb, ntiles, nz), threads, smem, stream>>>(src, dst, a);
-        return cudaGetLastError();
-    };
-    switch (kind) {
-        case 0: return sign < 0 ? go(fft_two_kernel<-1, 0>) : go(fft_two_kernel<1, 0>);
-        case 1: return sign < 0 ? go(fft_two_kernel<-1, 1>) : go(fft_two_kernel<1, 1>);
-        case 2: return sign < 0 ? go(fft_two_kernel<-1, 2>) : go(fft_two_kernel<1, 2>);
-        case 3: return sign < 0 ? go(fft_two_kernel<-1, 3>) : go(fft_two_kernel<1, 3>);
-        case 4: return sign < 0 ? go(fft_two_kernel<-1, 4>) : go(fft_two_kernel<1, 4>);
-        case 5: return sign < 0 ? go(fft_two_kernel<-1, 5>) : go(fft_two_kernel<1, 5>);
-        case 6: return sign < 0 ? go(fft_two_kernel<-1, 6>) : go(fft_two_kernel<1, 6>);
+    switch (kind_of(a.radix[0], a.radix[1])) {
+        case 0: return FftTwoKind<0>::launch(src, dst, a, ntiles, sign, stream, nz);
+        case 1: return FftTwoKind<1>::launch(src, dst, a, ntiles, sign, stream, nz);
+        case 2: return FftTwoKind<2>::launch(src, dst, a, ntiles, sign, stream, nz);
+        case 3: return FftTwoKind<3>::launch(src, dst, a, ntiles, sign, stream, nz);
+        case 4: return FftTwoKind<4>::launch(src, dst, a, ntiles, sign, stream, nz);
+        case 5: return FftTwoKind<5>::launch(src, dst, a, ntiles, sign, stream, nz);
+        case 6: return FftTwoKind<6>::launch(src, dst, a, ntiles, sign, stream, nz);
         default: return cudaErrorInvalidValue;
     }
 }
