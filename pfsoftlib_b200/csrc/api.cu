@@ -67,20 +67,6 @@ struct StagingContext {
     cudaEvent_t bounce_ev[kRing] = {};
 };
 
-// Chunks of a copy through the bounce buffer: the DMA of a chunk overlaps the host threads' copies of its
-// neighbours, and what does not overlap is one chunk at either end; below 1 MB, and above 8 MB, the
-// threads' start costs more than that. Two chunks of 16 MB (up to 16 MB nothing overlapped) against this,
-// us, median, 16 host cores, 27 GB/s to the device: DSOFT of B = 24 194 / 142, 32 767 / 251, 48 1750 / 750,
-// 64 2260 / 1890, iDSOFT 24 199 / 134, 32 870 / 237, 48 1400 / 585, 64 1850 / 1150; equal from B = 100 on.
-struct Chunks {
-    size_t bytes, count;   // of a chunk; of the ring
-    explicit Chunks(size_t total)
-    {
-        bytes = std::min((size_t)8 << 20, std::max((size_t)1 << 20, (total / 16 + 0x3ffff) & ~(size_t)0x3ffff));
-        count = std::min((size_t)kRing, kBounceBytes / bytes);
-    }
-};
-
 // Host threads that copy the slices of one large memcpy in parallel (the pageable side of a
 // bounce-buffer transfer is a host memory copy, which one thread does at a fraction of the
 // host's memory bandwidth). The calling thread takes a slice too.
@@ -157,6 +143,31 @@ class CopyPool {
     unsigned long long gen_ = 0;
 };
 
+// Chunks of a copy through the bounce buffer: the DMA of a chunk overlaps the host threads' copies of its
+// neighbours, and what does not overlap is one chunk at either end; below 1 MB, and above 8 MB, the
+// threads' start costs more than that. Below 2 MB in all the calling thread copies alone: between calls the other
+// threads' cores fall asleep, and waking them takes 100 us, as long as the copy. Two chunks of 16 MB (up to 16 MB nothing
+// overlapped; a thread per MB) against this, us, median, 16 host cores, 27 GB/s to the device, back to back (2 ms
+// apart): DSOFT of B = 16 71 / 70 (87 / 85; threads from 128 KB on 72 (159)), 20 126 / 121 (152 / 148; 96 (199)), 24 194 / 180 (250 / 235;
+// 146 (217)), 32 770 / 250 (790 / 440), 48 1680 / 740 (1720 / 890), 64 2160 / 1840 (2190 / 1930), iDSOFT 20 124 / 115 (137 / 125; 95 ..
+// 243 (229)), 24 207 / 192 (225 / 213; 147 .. 339 (340)), 32 980 / 240 (990 / 600), 48 1820 / 630 (1720 / 870), 64 1640 / 1100
+// (2250 / 1290); equal from B = 100 on.
+struct Chunks {
+    size_t bytes, count;   // of a chunk; of the ring
+    bool shared;           // the host threads share a chunk's copy
+    explicit Chunks(size_t total)
+    {
+        bytes = std::min((size_t)8 << 20, std::max((size_t)1 << 20, (total / 16 + 0x3ffff) & ~(size_t)0x3ffff));
+        count = std::min((size_t)kRing, kBounceBytes / bytes);
+        shared = total >= (size_t)2 << 20;
+    }
+    void copy(void* dst, const void* src, size_t n) const
+    {
+        if (shared) CopyPool::get().copy(dst, src, n);
+        else std::memcpy(dst, src, n);
+    }
+};
+
 bool is_pinned(const void* p)
 {
     cudaPointerAttributes a;
@@ -195,7 +206,7 @@ cudaError_t copy_in(StagingContext* st, void* dev, const void* host, size_t byte
         if (i >= c.count) e = cudaEventSynchronize(st->bounce_ev[b]);   // its last DMA has read it
         if (e != cudaSuccess) break;
         char* chunk = st->bounce + b * c.bytes;
-        CopyPool::get().copy(chunk, static_cast<const char*>(host) + off, n);
+        c.copy(chunk, static_cast<const char*>(host) + off, n);
         e = cudaMemcpyAsync(static_cast<char*>(dev) + off, chunk, n, cudaMemcpyHostToDevice, s);
         if (e == cudaSuccess) e = cudaEventRecord(st->bounce_ev[b], s);
     }
@@ -224,8 +235,7 @@ cudaError_t copy_out(StagingContext* st, void* host, const void* dev, size_t byt
         } else {
             const size_t off = done * c.bytes, b = done % c.count;
             e = cudaEventSynchronize(st->bounce_ev[b]);
-            if (e == cudaSuccess)
-                CopyPool::get().copy(static_cast<char*>(host) + off, st->bounce + b * c.bytes, std::min(c.bytes, bytes - off));
+            if (e == cudaSuccess) c.copy(static_cast<char*>(host) + off, st->bounce + b * c.bytes, std::min(c.bytes, bytes - off));
             ++done;
         }
     }
