@@ -748,14 +748,15 @@ static int layer_wise(int cols, int rows, int lays, double* d_arr, double scale,
             blu = t.bluestein;
         } else {
             // odd length: a private table (rare); freed after the stream drains
-            std::vector<double2> h(fft_twiddle_elems(n));
+            int ra, rb;
+            const bool two = fft_two_radices(n, &ra, &rb);
+            std::vector<double2> h(two ? fft_twiddle_elems(n) : n);
             for (int i = 0; i < n; ++i) {
                 const long double a = 6.283185307179586476925286766559005768L * (long double)i / (long double)n;
                 h[i] = make_double2((double)cosl(a), -(double)sinl(a));
             }
-            int ra, rb;
-            if (fft_two_radices(n, &ra, &rb))
-                for (int i = 0; i < n; ++i) h[n + i] = h[(size_t)(i / ra + 1) * (i % ra) % n];
+            for (int r = 1, i = n; two && r <= rb; ++r)
+                for (int j = 0, e = 0; j < ra; ++j, e = e + r < n ? e + r : e + r - n) h[i++] = h[e];   // e = r j mod n
             PF_CUDA(cudaMalloc(&tmp, h.size() * sizeof(double2)));
             PF_CUDA(cudaMemcpyAsync(tmp, h.data(), h.size() * sizeof(double2), cudaMemcpyHostToDevice, s));
             PF_CUDA(cudaStreamSynchronize(s));

@@ -154,20 +154,35 @@ __global__ void __launch_bounds__(512, 1)
 
 }  // namespace
 
+namespace {
+
+// The two radices of every length up to 32 x 32, zero for those without: a pass asks several times.
+struct TwoPlans {
+    static constexpr int kLast = 32 * 32;
+    unsigned char ra[kLast + 1] = {}, rb[kLast + 1] = {};
+    TwoPlans()
+    {
+        // of a length's pairs the one with the smallest larger factor, the larger one last
+        for (int hi = 32; hi >= 4; --hi)
+            for (int lo = 2; lo <= hi; ++lo) {
+                const int kind = kind_of(lo, hi);
+                // 2 x 17 .. 2 x 31 fill too few threads (n = 58, us per pass: 19, the chirp pass 13)
+                if (kind < 0 || ((kind == 4 || kind == 5) && lo < (is_prime17(lo) || is_prime17(hi) ? 3 : 14))) continue;
+                ra[lo * hi] = (unsigned char)lo;
+                rb[lo * hi] = (unsigned char)hi;
+            }
+    }
+};
+
+}  // namespace
+
 bool fft_two_radices(int n, int* ra, int* rb)
 {
-    // the pair with the smallest larger factor, the larger one last
-    for (int hi = 4; hi <= 32; ++hi) {
-        const int lo = n / hi;
-        if (n % hi || lo > hi || lo < 2) continue;
-        const int kind = kind_of(lo, hi);
-        // 2 x 17 .. 2 x 31 fill too few threads (n = 58, us per pass: 19, the chirp pass 13)
-        if (kind < 0 || ((kind == 4 || kind == 5) && lo < (is_prime17(lo) || is_prime17(hi) ? 3 : 14))) continue;
-        *ra = lo;
-        *rb = hi;
-        return true;
-    }
-    return false;
+    static const TwoPlans plans;
+    if (n < 0 || n > TwoPlans::kLast || plans.ra[n] == 0) return false;
+    *ra = plans.ra[n];
+    *rb = plans.rb[n];
+    return true;
 }
 
 int fft_two_vectors(int n)
