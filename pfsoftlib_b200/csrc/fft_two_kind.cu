@@ -100,9 +100,15 @@ __global__ void __launch_bounds__(128, kBlocks[KIND])
 }  // namespace
 
 template <int KIND>
-cudaError_t FftTwoKind<KIND>::launch(const double2* src, double2* dst, const FftPassArgs& a, int ntiles, int sign, cudaStream_t stream, int nz)
+cudaError_t FftTwoKind<KIND>::launch(const double2* src, double2* dst, const FftPassArgs& a0, int ntiles, int sign, cudaStream_t stream, int nz)
 {
+    FftPassArgs a = a0;
     const int ra = a.radix[0], rb = a.radix[1], top = kMaxRadix[KIND];
+    // Where tiles of eight vectors leave SMs idle, tiles of four: a thread then has one butterfly of a stage, not two
+    // or more. Us per layer-wise call of two passes, the kernels before these / eight / four: 640 x 24 x 9 14.4 / 17.5 /
+    // 15.4, 768 16.4 / 17.6 / 16.1, 960 18.5 / 20.5 / 18.5, 512 14.4 / 11.3 / 10.6, 1024 16.4 / 15.4 / 12.4, with 24 layers
+    // (72 tiles) 640 17.5 / 18.5 / 17.5, 1024 21.6 / 18.5 / 16.4.
+    if (a.kb == 8 && 8 * rb > 128 && (long long)((a.nvec + 7) / 8) * ntiles * nz <= 148) a.kb = 4;
     const size_t smem = (size_t)a.kb * block_pitch(ra, rb, a.kb) * sizeof(double2);
     const size_t largest = (size_t)8 * block_pitch(top, top, 8) * sizeof(double2);   // the kind's largest radices
     const int threads = std::min(128, (a.kb * rb + 31) / 32 * 32);
