@@ -145,8 +145,8 @@ class CopyPool {
 
 // Chunks of a copy through the bounce buffer: the DMA of a chunk overlaps the host threads' copies of its
 // neighbours, and what does not overlap is one chunk at either end; below 1 MB, and above 8 MB, the
-// threads' start costs more than that. Below 2 MB in all the calling thread copies alone: between calls the other
-// threads' cores fall asleep, and waking them takes 100 us, as long as the copy. Two chunks of 16 MB (up to 16 MB nothing
+// threads' start costs more than that. For grids below 2 MB the calling thread copies alone: between calls the other
+// threads' cores fall asleep, and waking them takes 100 us, as long as the copies. Two chunks of 16 MB (up to 16 MB nothing
 // overlapped; a thread per MB) against this, us, median, 16 host cores, 27 GB/s to the device, back to back (2 ms
 // apart): DSOFT of B = 16 71 / 70 (87 / 85; threads from 128 KB on 72 (159)), 20 126 / 121 (152 / 148; 96 (199)), 24 194 / 180 (250 / 235;
 // 146 (217)), 32 770 / 250 (790 / 440), 48 1680 / 740 (1720 / 890), 64 2160 / 1840 (2190 / 1930), iDSOFT 20 124 / 115 (137 / 125; 95 ..
@@ -155,11 +155,10 @@ class CopyPool {
 struct Chunks {
     size_t bytes, count;   // of a chunk; of the ring
     bool shared;           // the host threads share a chunk's copy
-    explicit Chunks(size_t total)
+    Chunks(size_t total, size_t grid_bytes) : shared(grid_bytes >= (size_t)2 << 20)
     {
         bytes = std::min((size_t)8 << 20, std::max((size_t)1 << 20, (total / 16 + 0x3ffff) & ~(size_t)0x3ffff));
         count = std::min((size_t)kRing, kBounceBytes / bytes);
-        shared = total >= (size_t)2 << 20;
     }
     void copy(void* dst, const void* src, size_t n) const
     {
@@ -196,11 +195,11 @@ cudaError_t bounce_ready(StagingContext* st)
 
 // Host-to-device copy, stream ordered: pinned sources go straight to DMA; pageable ones are
 // copied by the host threads into the ring's chunks while the DMAs of earlier chunks run.
-cudaError_t copy_in(StagingContext* st, void* dev, const void* host, size_t bytes, cudaStream_t s)
+cudaError_t copy_in(StagingContext* st, void* dev, const void* host, size_t bytes, size_t grid_bytes, cudaStream_t s)
 {
     if (is_pinned(host)) return cudaMemcpyAsync(dev, host, bytes, cudaMemcpyHostToDevice, s);
     cudaError_t e = bounce_ready(st);
-    const Chunks c(bytes);
+    const Chunks c(bytes, grid_bytes);
     for (size_t off = 0, i = 0; e == cudaSuccess && off < bytes; off += c.bytes, ++i) {
         const size_t b = i % c.count, n = std::min(c.bytes, bytes - off);
         if (i >= c.count) e = cudaEventSynchronize(st->bounce_ev[b]);   // its last DMA has read it
@@ -216,14 +215,14 @@ cudaError_t copy_in(StagingContext* st, void* dev, const void* host, size_t byte
 // Device-to-host copy after the work queued on s (copy_in's included: its chunks are free then); returns
 // when the host buffer holds the data. Pageable destinations: the DMAs of the ring's next chunks overlap
 // the host threads' copy out of the oldest.
-cudaError_t copy_out(StagingContext* st, void* host, const void* dev, size_t bytes, cudaStream_t s)
+cudaError_t copy_out(StagingContext* st, void* host, const void* dev, size_t bytes, size_t grid_bytes, cudaStream_t s)
 {
     if (is_pinned(host)) {
         cudaError_t e = cudaMemcpyAsync(host, dev, bytes, cudaMemcpyDeviceToHost, s);
         return e == cudaSuccess ? cudaStreamSynchronize(s) : e;
     }
     cudaError_t e = bounce_ready(st);
-    const Chunks c(bytes);
+    const Chunks c(bytes, grid_bytes);
     const size_t chunks = (bytes + c.bytes - 1) / c.bytes;
     for (size_t i = 0, done = 0; e == cudaSuccess && done < chunks;) {
         if (i < chunks && i < done + c.count) {
@@ -704,15 +703,15 @@ static int host_staged(int B, bool forward, const double* in, double* out)
     cudaStream_t s = st->h_stream;
     int rc;
     if (forward) {
-        PF_CUDA(copy_in(st, st->h_grid, in, gb, s));
+        PF_CUDA(copy_in(st, st->h_grid, in, gb, gb, s));
         rc = run_dsoft(static_cast<const double*>(st->h_grid), B, static_cast<double*>(st->h_coef), st->h_ws, s);
         if (rc) return rc;
-        PF_CUDA(copy_out(st, out, st->h_coef, cb, s));
+        PF_CUDA(copy_out(st, out, st->h_coef, cb, gb, s));
     } else {
-        PF_CUDA(copy_in(st, st->h_coef, in, cb, s));
+        PF_CUDA(copy_in(st, st->h_coef, in, cb, gb, s));
         rc = run_idsoft(static_cast<const double*>(st->h_coef), B, static_cast<double*>(st->h_grid), st->h_ws, s);
         if (rc) return rc;
-        PF_CUDA(copy_out(st, out, st->h_grid, gb, s));
+        PF_CUDA(copy_out(st, out, st->h_grid, gb, gb, s));
     }
     PF_CUDA(cudaStreamSynchronize(s));
     return PFSOFT_OK;
