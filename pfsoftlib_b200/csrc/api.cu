@@ -144,20 +144,20 @@ class CopyPool {
 };
 
 // Chunks of a copy through the bounce buffer: the DMA of a chunk overlaps the host threads' copies of its
-// neighbours, and what does not overlap is one chunk at either end; below 1 MB, and above 8 MB, the
-// threads' start costs more than that. For grids below 2 MB the calling thread copies alone: between calls the other
-// threads' cores fall asleep, and waking them takes 100 us, as long as the copies. Two chunks of 16 MB (up to 16 MB nothing
-// overlapped; a thread per MB) against this, us, median, 16 host cores, 27 GB/s to the device, back to back (2 ms
-// apart): DSOFT of B = 16 71 / 70 (87 / 85; threads from 128 KB on 72 (159)), 20 126 / 121 (152 / 148; 96 (199)), 24 194 / 180 (250 / 235;
-// 146 (217)), 32 770 / 250 (790 / 440), 48 1680 / 740 (1720 / 890), 64 2160 / 1840 (2190 / 1930), iDSOFT 20 124 / 115 (137 / 125; 95 ..
-// 243 (229)), 24 207 / 192 (225 / 213; 147 .. 339 (340)), 32 980 / 240 (990 / 600), 48 1820 / 630 (1720 / 870), 64 1640 / 1100
-// (2250 / 1290); equal from B = 100 on.
+// neighbours, and what does not overlap is one chunk at either end; below 1 MB (512 KB where the calling thread copies
+// alone), and above 8 MB, the threads' start or the calls cost more than that. For grids below 2 MB the calling thread
+// copies alone: between calls the other threads' cores fall asleep, and waking them takes 100 us, as long as the copies.
+// Measured, us, median, 16 host cores, 27 GB/s to the device, calls back to back (2 ms apart), two chunks of 16 MB and a
+// thread per MB / these chunks, threads from 128 KB on at every size / this: DSOFT of B = 16 73 / 74 / 75 (74 / 167 / 71), 20 128 / 95 /
+// 110 (138 / 268 / 123), 24 182 / 140 / 159 (190 / 257 / 179), iDSOFT 16 72 / 72 / 77 (76 / 164 / 72), 20 130 / 252 / 106 (139 / 269 / 115), 24 201 /
+// 267 / 176 (212 / 358 / 186); with the threads, DSOFT 32 770 / 250 (790 / 440), 48 1680 / 740 (1720 / 890), 64 2160 / 1840 (2190 / 1930),
+// iDSOFT 32 980 / 240 (990 / 600), 48 1820 / 630 (1720 / 870), 64 1640 / 1100 (2250 / 1290); equal from B = 100 on.
 struct Chunks {
     size_t bytes, count;   // of a chunk; of the ring
     bool shared;           // the host threads share a chunk's copy
     Chunks(size_t total, size_t grid_bytes) : shared(grid_bytes >= (size_t)2 << 20)
     {
-        bytes = std::min((size_t)8 << 20, std::max((size_t)1 << 20, (total / 16 + 0x3ffff) & ~(size_t)0x3ffff));
+        bytes = std::min((size_t)8 << 20, std::max((size_t)(shared ? 2 : 1) << 19, (total / 16 + 0x3ffff) & ~(size_t)0x3ffff));
         count = std::min((size_t)kRing, kBounceBytes / bytes);
     }
     void copy(void* dst, const void* src, size_t n) const
